@@ -152,6 +152,24 @@ def test_gemm_bf16_tcgen05_with_swiglu_epilogue(m, inter, k, pair):
     assert (y.double() - want).abs().max() / want.abs().max() < 2 * BF16_EPS
 
 
+@pytest.mark.parametrize("m,inter", [(257, 1100), (2290, 1256), (4336, 640)])
+@pytest.mark.parametrize("limit", [0.0, 2.0])
+def test_gemm_bf16_tcgen05_several_tiles_per_pair_with_a_ragged_last_row_block(m, inter, limit):
+    """More tiles than pairs of blocks, rows and columns that end inside a tile, biases, both gated activations."""
+    o = ops()
+    k = 200
+    x, w, b = rnd((m, k), torch.bfloat16, 94), rnd((2 * inter, k), torch.bfloat16, 95, 0.1), rnd((2 * inter,), torch.float32, 96)
+    y = torch.full((m + 1, inter), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.gemm_bf16_tcgen05(x, w, y, m, swiglu=True, bias=b, glu=(limit, 1.702, 1.0) if limit else None)
+    assert int(o.gemm_tc_status(x.device)[0]) == 0
+    g, u = (x.double() @ w.double().T + b.double()).split(inter, dim=1)
+    if limit:
+        g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+    want = g * torch.sigmoid(1.702 * g) * (u + 1.0) if limit else g * torch.sigmoid(g) * u
+    assert (y[:m].double() - want).abs().max() / want.abs().max() < 2 * BF16_EPS          # (one rounding of the result; float32 sums of 200 terms)
+    assert bool((y[m] == 7.0).all())
+
+
 # ------------------------------------------------------------------------------------------ rope + cache write
 def make_cache(kv_heads, head_dim, n_pages, n_slots, dtype, pages_per_slot):
     """A one-entry paged cache with a page table that scatters each slot's pages."""

@@ -184,20 +184,19 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
             const uint32_t trow = tmem + ab * 256 + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
             for (int c = 0; c < 128 / 32 * (SWIGLU ? 1 : 2); ++c) {
-                float v[32];
+                float v[32], u[SWIGLU ? 32 : 1];
                 tc_ld32(trow + c * 32, v);
-                if (SWIGLU) {
-                    float u[32];
-                    tc_ld32(trow + 128 + c * 32, u);
-                    if (glu.bias != nullptr) tc_add_bias(v, u, &sh->bias[quarter][c * 32]);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = glu_act(v[i], u[i], glu);
-                } else if (glu.out_act != X0NE_OUT_AS_IT_IS) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = out_act(v[i], glu);
-                }
+                if constexpr (SWIGLU) tc_ld32(trow + 128 + c * 32, u);
                 const int n = n0 + c * 32;
                 if (m < M) {
+                    if constexpr (SWIGLU) {
+                        if (glu.bias != nullptr) tc_add_bias(v, u, &sh->bias[quarter][c * 32]);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = glu_act(v[i], u[i], glu);
+                    } else if (glu.out_act != X0NE_OUT_AS_IT_IS) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = out_act(v[i], glu);
+                    }
                     OutT* dst = Y + (int64_t)m * ldy + n;
                     if (n + 32 <= N && (((uintptr_t)dst) & 31) == 0) {
 #pragma unroll
@@ -233,8 +232,17 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
 //   * the epilogue threads of both blocks arrive on the first block's "accumulator drained" barrier.
 // With SwiGLU the first block's W rows are the gate rows and the second block's the up rows, so the
 // accumulator's columns 0-127 are gate and 128-255 up, in both blocks.
+//
+// A tile's products take 13 us per 2,048 of K (256 x 256, sustained); what its epilogue takes has to stay below that, or it
+// bounds the kernel.  With one warp per quarter of the rows the gated epilogue took 15.5 us, so two warps share a quarter,
+// half of the columns each: gate|up 12288 x 2048 at 2,048 / 4,096 / 8,192 rows 99 / 171 / 329 -> 82 / 151 / 287 us (the same
+// product without the activation: 80 / 147 / 281).  Rows past the last one are not activated: their gates are zeros, and the
+// division of a zero takes the slow path of the correctly rounded division, which made the tiles of a ragged last row block
+// twice as long (9,456 rows, 240 of the last 256 real: 762-815 us -> 340-353; 9,472 rows took 375-390 -> 352).
 // ----------------------------------------------------------------------------------------
 #define TC2_STAGES 6
+#define TC2_EPILOGUE_WARPS 8          // two per quarter of a block's rows, each with half of a tile's columns
+#define TC2_THREADS (64 + 32 * TC2_EPILOGUE_WARPS)
 
 struct Tc2Shared {
     uint64_t full[TC2_STAGES];
@@ -243,7 +251,7 @@ struct Tc2Shared {
     uint64_t accum_empty[2];
     uint32_t tmem_base;
     int failed;
-    __align__(16) float bias[4][256];       // as in TcShared
+    __align__(16) float bias[TC2_EPILOGUE_WARPS][256];       // as in TcShared
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -282,7 +290,7 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
 }
 
 template <bool SWIGLU, typename OutT>
-__global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(TC2_THREADS) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                   const __grid_constant__ CUtensorMap map_w,
                                                                   OutT* __restrict__ Y, int M, int N, int K, int ldy,
                                                                   int m_tiles, int n_tiles, int* status, GluParams glu) {
@@ -305,7 +313,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(const __grid_c
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sh->accum_full[b], 1);
-            mbar_init(&sh->accum_empty[b], 256);     // the epilogue threads of both blocks
+            mbar_init(&sh->accum_empty[b], 2 * 32 * TC2_EPILOGUE_WARPS);     // the epilogue threads of both blocks
         }
         sh->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -375,13 +383,14 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(const __grid_c
             }
         }
     } else {
-        const int quarter = warp & 3;
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        constexpr int CHUNKS = 128 / 32 * (SWIGLU ? 1 : 2) / 2;         // pieces of 32 columns of a warp's half
         int t = 0;
         for (int tile = pair; tile < tiles; tile += pairs, ++t) {
             const int ab = t & 1;
             const int m0 = (tile % m_tiles) * 256 + 128 * (int)rank, n0 = (tile / m_tiles) * BN;
             const int m = m0 + quarter * 32 + lane;
-            if (SWIGLU && glu.bias != nullptr) tc_stage_bias(sh->bias[quarter], glu.bias, n0, N, lane);
+            if (SWIGLU && glu.bias != nullptr) tc_stage_bias(sh->bias[warp - 2], glu.bias, n0, N, lane);
             if (!mbar_wait(&sh->accum_full[ab], (t >> 1) & 1, status, 3) || sh->failed) {
                 sh->failed = 1;
                 break;
@@ -389,21 +398,20 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_pair_kernel(const __grid_c
             tc_fence_after();
             const uint32_t trow = tmem + ab * 256 + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-            for (int c = 0; c < 128 / 32 * (SWIGLU ? 1 : 2); ++c) {
-                float v[32];
+            for (int c = half * CHUNKS; c < (half + 1) * CHUNKS; ++c) {
+                float v[32], u[SWIGLU ? 32 : 1];
                 tc_ld32(trow + c * 32, v);
-                if (SWIGLU) {
-                    float u[32];
-                    tc_ld32(trow + 128 + c * 32, u);
-                    if (glu.bias != nullptr) tc_add_bias(v, u, &sh->bias[quarter][c * 32]);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = glu_act(v[i], u[i], glu);
-                } else if (glu.out_act != X0NE_OUT_AS_IT_IS) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = out_act(v[i], glu);
-                }
+                if constexpr (SWIGLU) tc_ld32(trow + 128 + c * 32, u);
                 const int n = n0 + c * 32;
                 if (m < M) {
+                    if constexpr (SWIGLU) {
+                        if (glu.bias != nullptr) tc_add_bias(v, u, &sh->bias[warp - 2][c * 32]);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = glu_act(v[i], u[i], glu);
+                    } else if (glu.out_act != X0NE_OUT_AS_IT_IS) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) v[i] = out_act(v[i], glu);
+                    }
                     OutT* dst = Y + (int64_t)m * ldy + n;
                     if (n + 32 <= N && (((uintptr_t)dst) & 31) == 0) {
 #pragma unroll
@@ -516,7 +524,7 @@ static int launch_tc_pair(const void* W, const void* X, OutT* Y, int M, int N, i
     if (tiles < pairs) pairs = tiles;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(TC_THREADS);
+    cfg.blockDim = dim3(TC2_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

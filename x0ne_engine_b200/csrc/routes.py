@@ -92,15 +92,15 @@ RULES: List[Rule] = [
     Rule("skinny", (17, 48), False, lambda s: s.weight_bytes >= 64 * MB,
          "10240 x 5120 at 32 rows: skinny 20.1 us, library 21.1; 5120 x 8192: 17.0 / 19.4; at 64 rows the library is ahead on both"),
     # ---- many rows
-    Rule("library", (768, 2048), True, lambda s: s.k <= 2048,
-         "gate|up 12288 x 2048 at 2,048 rows: library 89.8 us with the activation's launch, tc_pair 99.9 (113.1 with biases in the "
-         "epilogue: a tile of 32 steps over K does not cover it)"),
+    Rule("library", (768, 2048), True, lambda s: s.k <= 1024,
+         "gate|up 6144 x 1024 at 1,024 / 1,536 / 2,048 rows: library 23.1 / 26.7 / 36.9 us with the activation's launch, tc_pair 28.0 / 29.4 / 38.1 "
+         "(a tile of 16 steps over K does not cover its epilogue); at 4,096 rows 64.1 against 63.7"),
     Rule("tc_pair", (1536, 1 << 30), False, lambda s: s.k <= 2048 and s.n >= 2 * s.k,
          "squared ReLU behind 9216 x 2048 at 2,048 rows: 56.6 us in the epilogue, library 59.8 with the launch; 6144 x 2048: 56.5 / 60.7 "
          "(at 4,096: 82.5 / 114.9); 18432 x 4096 stays with the library, 213.7 against 220.6", act=True),
     Rule("tc_pair", (768, 1 << 30), True, _always,
-         "gate|up 24576 x 4096 at 2,048 rows: 1.62 PFLOP/s with the activation in the epilogue; at 512 rows the library "
-         "(74.9 us + 8.5 for SwiGLU) is ahead of it (84.6)"),
+         "gate|up 24576 x 4096 at 2,048 rows: tc_pair 288 us, library 310 with the activation's launch, 12288 x 2048: 86.0 against 95.7 "
+         "(at 768 rows 117.0 / 118.2 and 38.6 / 38.5); at 384 rows 83.5 / 82.1 and 36.1 / 24.7"),
     Rule("library", (1, 1 << 30), None, _always,
          "elsewhere cuBLAS is the fastest product measured: 6144 x 4096 at 128 rows 11.9 us (tcgen05 product here: 27.7), "
          "at 512 rows 21.0 (29.0)"),
