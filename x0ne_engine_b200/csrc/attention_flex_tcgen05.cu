@@ -1,0 +1,510 @@
+// The general attention of attention_flex.cu for passes with many rows, on the 5th-generation tensor cores: keys and values of
+// different widths, values out of the key rows, chunks, windows, kept first keys, a sink, slopes, gates, sigmoid weights, float32
+// results, rows inside wider buffers.  Scores, maxima, sums, weights and the accumulated output are float32; a weight p goes into
+// the product with the values as bfloat16(p) and bfloat16(p - bfloat16(p)), as in the mma.sync kernel.
+//
+// A block takes up to 128 rows of one sequence and one q head and walks the pages (64 keys) that the tile can see.  Ten warps:
+//   * copies (warp 9): TMA loads of Q (once), and of each page's key and value tiles into two stages each (64-value wide boxes, 128-byte
+//     swizzle; a tensor map per operand [pages, rows of a page, width] reads zeros past a head's width, so widths that are
+//     no multiple of 64 need nothing else);
+//   * products (warp 8): S(i + 1) = Q K^T into the other of two score buffers, then, when the softmax threads are done with page i,
+//     O += P(i) V(i).  P is read from tensor memory: its high and low halves lie over the scores it was made from, so no
+//     shared memory is written and the block fits twice on an SM;
+//   * softmax (warps 0-7): two threads per row, each with half of a page's keys; they meet at a named barrier of their 64 threads
+//     (the row's maximum goes through shared memory, and neither writes P over scores that the other has not read).  The
+//     accumulator is rescaled in tensor memory only when a row's maximum has grown by more than 2^8.
+// Every mbarrier wait is bounded; where one runs out the block says so in `status` and goes on without waiting, so that it ends.
+//
+// What bounds it: per page of 128 x 128 heads the tensor pipe has 900 cycles of work (scores 64 keys wide are bound by shared memory,
+// the split weights take two products), the softmax threads' instructions and exponentials 600 each; two blocks share an SM.
+// A layer of 32 q heads over 8 kv heads of 128 with its projections, one sequence of 128 / 1,024 / 8,192 rows: 61.6 / 209 / 4,385 us
+// with the mma.sync kernel, 37.7 / 105 / 1,188 with this one; latent attention (32 heads over rows of 256 + 64) of 100 / 2,048 rows:
+// 81.7 / 729 -> 53.6 / 351.  It is ahead from 16 rows on, so it takes every pass whose widths and rows TMA can copy.
+#include "tcgen05.cuh"
+
+struct FlexTcArgs {
+    void* out;
+    const int32_t* tile_seq;       // [tiles]
+    const int32_t* tile_row0;      // [tiles] first row of the tile within the pass
+    const int32_t* seq_first_row;  // [seqs + 1]
+    const int32_t* seq_slot;       // [seqs]
+    const int32_t* seq_pos0;       // [seqs]
+    int32_t q_heads, window;
+    int32_t vd;                    // value width
+    int32_t nbk, nbv;              // 64-wide blocks of a key row and of a value row
+    int32_t tmem_cols;
+    float scale_log2;
+};
+
+struct FlexTcShared {
+    uint64_t q_full;
+    uint64_t k_full[2], v_full[2];
+    uint64_t s_ready[2];           // S of a page is complete (and its key tile has been read)
+    uint64_t p_ready[2];           // the weights of a page are in tensor memory
+    uint64_t pv_done[2];           // the product with a page's values is complete
+    uint32_t tmem_base;
+    int failed;
+    int page_ok[4];                // whether the sequence has the page (ring over the walk)
+    float xmax[2][2][128];         // [page parity][half][row]: the halves' maxima; at the end their sums
+};
+
+#define FT_THREADS 320
+#define FT_LOG2E 1.4426950408889634f
+#define FT_RESCALE_LOG2 8.0f
+
+__device__ __forceinline__ float ft_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void ft_tma_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(tc_smem(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(tc_smem(bar)) : "memory");
+}
+// A from tensor memory (bfloat16 pairs along K, one 32-bit column per pair), B from shared memory
+__device__ __forceinline__ void ft_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void ft_st8(uint32_t taddr, const uint32_t* v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+}
+__device__ __forceinline__ void ft_st32(uint32_t taddr, const float* v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ft_st8(taddr + 8 * i, reinterpret_cast<const uint32_t*>(v) + 8 * i);
+}
+__device__ __forceinline__ void ft_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// N-major (the matrix's N runs along the 128-byte rows) shared-memory descriptor, 128-byte swizzle: 8-row groups 1024 bytes apart,
+// 64-wide column blocks `block_bytes` apart.
+__device__ __forceinline__ uint64_t ft_desc_nmajor(uint32_t smem_addr, uint32_t block_bytes) {
+    const uint32_t lo = ((smem_addr >> 4) & 0x3FFFu) | (((block_bytes >> 4) & 0x3FFFu) << 16);
+    const uint32_t hi = 64u | (1u << 14) | (2u << 29);
+    return ((uint64_t)hi << 32) | lo;
+}
+__device__ __forceinline__ void ft_pair_sync(int rows32) { asm volatile("bar.sync %0, 64;" ::"r"(1 + rows32) : "memory"); }
+__device__ __forceinline__ int ft_first_key(int pos, int window, int chunk) {
+    int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    if (chunk > 0) lo = max(lo, pos - pos % chunk);
+    return lo;
+}
+
+// SIG: weights sigmoid(score + bias) in the place of the softmax.
+template <bool SIG>
+__global__ void __launch_bounds__(FT_THREADS, 2) flex_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                                                                        const __grid_constant__ CUtensorMap map_v, FlexTcArgs a, PagedCache cache,
+                                                                        AttnExtra ex, int* status) {
+    extern __shared__ __align__(1024) unsigned char ft_raw[];
+    const int kt_bytes = a.nbk * 64 * 128, vt_bytes = a.nbv * 64 * 128;       // a page's key and value tile: [block][64 keys][128 bytes]
+    const bool own_v = ex.v_from_k <= 0;
+    unsigned char* qs = ft_raw;                                               // [block][128 rows][128 bytes]
+    unsigned char* ks = qs + a.nbk * 128 * 128;
+    unsigned char* vs = own_v ? ks + 2 * kt_bytes : ks;
+    const int v_stage = own_v ? vt_bytes : kt_bytes;
+    FlexTcShared* sh = reinterpret_cast<FlexTcShared*>(ks + 2 * kt_bytes + (own_v ? 2 * vt_bytes : 0));
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+
+    const int head = blockIdx.x, tile = gridDim.y - 1 - blockIdx.y;
+    const int kh = head / (a.q_heads / cache.kv_heads);
+    const int seq = a.tile_seq[tile], row0 = a.tile_row0[tile];
+    const int n_rows = min(128, a.seq_first_row[seq + 1] - row0);
+    const int slot = a.seq_slot[seq];
+    const int pos_first = a.seq_pos0[seq] + (row0 - a.seq_first_row[seq]);
+    const int pos_last = pos_first + n_rows - 1;
+    const int pg_first = ft_first_key(pos_first, a.window, ex.chunk) / 64, pg_last = pos_last / 64;
+    // pages of kept first keys that lie wholly before the first page of the window come first in the walk
+    const int n_kept = min((ex.keep_first + 63) / 64, pg_first);
+    const int n_walk = slot < 0 || n_rows <= 0 ? 0 : n_kept + pg_last - pg_first + 1;
+    auto page_at = [&](int i) { return i < n_kept ? i : pg_first + i - n_kept; };
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        mbar_init(&sh->q_full, 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&sh->k_full[b], 1);
+            mbar_init(&sh->v_full[b], 1);
+            mbar_init(&sh->s_ready[b], 1);
+            mbar_init(&sh->p_ready[b], 256);
+            mbar_init(&sh->pv_done[b], 1);
+        }
+        sh->failed = (tc_smem(ft_raw) & 1023u) != 0 ? 1 : 0;      // the swizzle needs 1024-byte aligned tiles
+        if (sh->failed) atomicOr(status, 1 << 9);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 8) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&sh->tmem_base)), "r"(a.tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_s = sh->tmem_base, tmem_o = tmem_s + 128;       // S / P: two buffers of 64 columns; O: 64 nbv columns
+    bool ok = !sh->failed;
+
+    if (warp >= 8) {
+        // The two control warps run their loops with all lanes; one elected lane issues.
+        uint32_t leader = 0;
+        asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+        auto wait = [&](uint64_t* bar, int parity, int code) {
+            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
+        };
+        if (warp == 9) {
+            auto page_of = [&](int i) -> int {
+                if (i >= n_walk) return -1;
+                const int pg = cache.page_table[(int64_t)slot * cache.table_stride + page_at(i) % cache.ring_pages];
+                return pg < 0 || pg >= cache.n_pages ? -1 : pg;
+            };
+            int pages[3] = {page_of(0), page_of(1), page_of(2)};        // looked up well ahead of the copies that need them
+            int k_issued = 0, v_issued = 0;
+            auto load_k = [&](int i, int page) {
+                const int st = i & 1;
+                if (leader) {
+                    sh->page_ok[i & 3] = page >= 0;
+                    mbar_expect_tx(&sh->k_full[st], kt_bytes);
+                    for (int nb = 0; nb < a.nbk; ++nb)
+                        ft_tma_3d(ks + st * kt_bytes + nb * 64 * 128, &map_k, nb * 64, kh * 64, max(page, 0), &sh->k_full[st]);
+                }
+                __syncwarp();
+                ++k_issued;
+            };
+            pdl_wait();      // q and the newest cache rows were written by the kernel before this one
+            asm volatile("fence.proxy.async.global;" ::: "memory");
+            if (ok && n_walk > 0) {
+                if (leader) {
+                    mbar_expect_tx(&sh->q_full, a.nbk * 128 * 128);
+                    for (int nb = 0; nb < a.nbk; ++nb) ft_tma_3d(qs + nb * 128 * 128, &map_q, nb * 64, head, row0, &sh->q_full);
+                }
+                __syncwarp();
+                load_k(0, pages[0]);
+            }
+            for (int i = 0; i < n_walk && ok; ++i) {
+                // a key tile's stage is free when its scores are complete (values out of the keys: when the product with them is),
+                // a value tile's when the product with it is
+                if (i + 1 < n_walk) {
+                    if (i >= 1) {
+                        if (own_v) wait(&sh->s_ready[(i - 1) & 1], ((i - 1) >> 1) & 1, 17);
+                        else wait(&sh->pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, 8);
+                    }
+                    if (ok) load_k(i + 1, pages[1]);
+                }
+                if (own_v) {
+                    if (i >= 2) wait(&sh->pv_done[i & 1], ((i - 2) >> 1) & 1, 8);
+                    if (ok) {
+                        if (leader) {
+                            mbar_expect_tx(&sh->v_full[i & 1], vt_bytes);
+                            for (int nb = 0; nb < a.nbv; ++nb)
+                                ft_tma_3d(vs + (i & 1) * vt_bytes + nb * 64 * 128, &map_v, nb * 64, kh * 64, max(pages[0], 0), &sh->v_full[i & 1]);
+                        }
+                        __syncwarp();
+                        ++v_issued;
+                    }
+                }
+                pages[0] = pages[1];
+                pages[1] = pages[2];
+                pages[2] = page_of(i + 3);
+            }
+            if (!ok) {       // copies that nobody waited for must land before the block's memory is given back
+                if (k_issued > 0) mbar_wait(&sh->q_full, 0, status, 5);
+                for (int back = 1; back <= 2; ++back) {
+                    if (k_issued >= back) mbar_wait(&sh->k_full[(k_issued - back) & 1], ((k_issued - back) >> 1) & 1, status, 6);
+                    if (v_issued >= back) mbar_wait(&sh->v_full[(v_issued - back) & 1], ((v_issued - back) >> 1) & 1, status, 13);
+                }
+            }
+        } else {
+            // instruction descriptors: f32 accumulate, bf16 operands, M = 128; scores N = 64; output N = 64 nbv with an N-major B
+            const uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+            const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(a.nbv * 8) << 17) | ((128u >> 4) << 24);
+            const uint32_t qb = tc_smem(qs);
+            auto scores = [&](int i) {
+                wait(&sh->k_full[i & 1], (i >> 1) & 1, 6);
+                if (ok) {
+                    tc_fence_after();
+                    if (leader) {
+                        const uint32_t kb = tc_smem(ks + (i & 1) * kt_bytes);
+                        for (int nb = 0; nb < a.nbk; ++nb) {
+#pragma unroll
+                            for (int kk = 0; kk < 4; ++kk)
+                                tc_mma(tmem_s + (i & 1) * 64, tc_desc(qb + nb * 128 * 128 + kk * 32), tc_desc(kb + nb * 64 * 128 + kk * 32), idesc_qk,
+                                       nb + kk > 0 ? 1u : 0u);
+                        }
+                        tc_commit(&sh->s_ready[i & 1]);
+                    }
+                    __syncwarp();
+                }
+            };
+            if (n_walk > 0) {
+                wait(&sh->q_full, 0, 5);
+                scores(0);
+            }
+            for (int i = 0; i < n_walk && ok; ++i) {
+                if (i + 1 < n_walk) {
+                    if (i >= 1) wait(&sh->pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, 8);      // the weights in this score buffer have been used
+                    scores(i + 1);
+                }
+                if (own_v) wait(&sh->v_full[i & 1], (i >> 1) & 1, 13);
+                wait(&sh->p_ready[i & 1], (i >> 1) & 1, 7);
+                if (ok) {
+                    tc_fence_after();
+                    if (leader) {
+                        const uint32_t vb = tc_smem(vs + (i & 1) * v_stage), pb = tmem_s + (i & 1) * 64;
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            const uint64_t vdesc = ft_desc_nmajor(vb + kk * 16 * 128, 64 * 128);
+                            ft_mma_ts(tmem_o, pb + kk * 8, vdesc, idesc_pv, i + kk > 0 ? 1u : 0u);
+                            ft_mma_ts(tmem_o, pb + 32 + kk * 8, vdesc, idesc_pv, 1u);
+                        }
+                        tc_commit(&sh->pv_done[i & 1]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+        if (!ok) sh->failed = 1;
+    } else {
+        const int sw = warp & 3, half = warp >> 2;
+        const int r = sw * 32 + lane, p = pos_first + r;
+        const uint32_t lane_base = (uint32_t)(sw * 32) << 16;
+        const int lo = ft_first_key(p, a.window, ex.chunk);
+        const int warp_pos = pos_first + sw * 32, warp_lo = ft_first_key(warp_pos + 31, a.window, ex.chunk);     // (first keys only grow along the rows)
+        const bool sloped = ex.slope != nullptr;
+        const float sl2 = sloped ? ex.slope[head] * FT_LOG2E : 0.f, sb2 = SIG ? ex.sig_bias[head] * FT_LOG2E : 0.f;
+        const float sink2 = !SIG && ex.sink != nullptr ? ex.sink[head] * FT_LOG2E : -INFINITY;
+        const float sc = sloped ? 1.f : a.scale_log2;            // what a score (with its slope) is multiplied by in the exponent
+        float m_ref = -INFINITY, l = 0.f;                        // reference maximum, and this half's sum of weights
+        auto wait = [&](uint64_t* bar, int parity, int code) {
+            if (ok) ok = mbar_wait(bar, parity, status, code);
+            __syncwarp();
+        };
+        for (int i = 0; i < n_walk; ++i) {
+            const int pg0 = page_at(i) * 64, j0 = pg0 + half * 32;
+            wait(&sh->s_ready[i & 1], (i >> 1) & 1, 10);
+            tc_fence_after();
+            float s[32];
+            tc_ld32(tmem_s + (i & 1) * 64 + half * 32 + lane_base, s);
+            const bool have = sh->page_ok[i & 3] != 0;
+            if (sloped) {
+                const float at = sl2 * (float)(p - j0);
+#pragma unroll
+                for (int c = 0; c < 32; ++c) s[c] = fmaf(s[c], a.scale_log2, fmaf(sl2, (float)c, -at));
+            }
+            if (!have || !(pg0 + 63 <= warp_pos && (pg0 >= warp_lo || pg0 + 64 <= ex.keep_first))) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    const int j = j0 + c;
+                    if (!have || j > p || (j < lo && j >= ex.keep_first)) s[c] = -INFINITY;
+                }
+            }
+            float neg = 0.f;
+            tc_fence_before();
+            if (SIG) {
+                ft_pair_sync(sw);                 // the other half has read its scores
+            } else {
+                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains instead of one
+#pragma unroll
+                for (int c = 0; c < 32; c += 4) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) mx4[e] = fmaxf(mx4[e], s[c + e]);
+                }
+                const float mine = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+                sh->xmax[i & 1][half][r] = mine;
+                ft_pair_sync(sw);
+                const float mx = fmaxf(mine, sh->xmax[i & 1][half ^ 1][r]);
+                // raise the reference only when it is first set or falls too far behind
+                const bool raise = mx > m_ref && (m_ref == -INFINITY || (mx - m_ref) * sc > FT_RESCALE_LOG2);
+                const bool shrink = raise && m_ref != -INFINITY;          // what this row has accumulated must be rescaled
+                const float alpha = shrink ? ft_ex2((m_ref - mx) * sc) : 1.f;
+                if (raise) m_ref = mx;
+                neg = m_ref == -INFINITY ? 0.f : -m_ref * sc;
+                l *= alpha;
+                if (i > 0 && __any_sync(0xffffffffu, shrink)) {
+                    wait(&sh->pv_done[(i - 1) & 1], ((i - 1) >> 1) & 1, 14);
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = half * a.nbv; c < (half + 1) * a.nbv; ++c) {
+                        float ov[32];
+                        tc_ld32(tmem_o + lane_base + c * 32, ov);
+#pragma unroll
+                        for (int d = 0; d < 32; ++d) ov[d] *= alpha;
+                        ft_st32(tmem_o + lane_base + c * 32, ov);
+                    }
+                    ft_st_wait();
+                }
+            }
+            tc_fence_after();
+            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint32_t pcol = tmem_s + (i & 1) * 64 + half * 16 + lane_base;
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                uint32_t hi[8], lw[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int c = 16 * g + 2 * e;
+                    float p0, p1;
+                    if (SIG) {
+                        p0 = __fdividef(1.0f, 1.0f + ft_ex2(-fmaf(s[c], sc, sb2)));
+                        p1 = __fdividef(1.0f, 1.0f + ft_ex2(-fmaf(s[c + 1], sc, sb2)));
+                    } else {
+                        p0 = ft_ex2(fmaf(s[c], sc, neg));
+                        p1 = ft_ex2(fmaf(s[c + 1], sc, neg));
+                        sum4[e & 3] += p0 + p1;
+                    }
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
+                    hi[e] = *reinterpret_cast<const uint32_t*>(&h2);
+                    const __nv_bfloat162 l2 = __floats2bfloat162_rn(p0 - __uint_as_float(hi[e] << 16), p1 - __uint_as_float(hi[e] & 0xffff0000u));
+                    lw[e] = *reinterpret_cast<const uint32_t*>(&l2);
+                }
+                ft_st8(pcol + 8 * g, hi);
+                ft_st8(pcol + 32 + 8 * g, lw);
+            }
+            l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+            // Rows of the page past the tile's last position may hold anything (an earlier sequence's values): zero them, so that
+            // 0 * value stays 0.  (Values out of the keys: the page's scores are complete, nobody reads its keys any more.)
+            if (pg0 + 63 > pos_last) {
+                if (own_v) wait(&sh->v_full[i & 1], (i >> 1) & 1, 15);
+                if (half == 0 && r < 64 && pg0 + r > pos_last) {
+                    unsigned char* vrow = vs + (i & 1) * v_stage + r * 128;
+                    for (int nb = 0; nb < a.nbv; ++nb)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(vrow + nb * 64 * 128 + c * 16) = make_uint4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+            }
+            ft_st_wait();
+            tc_fence_before();
+            mbar_arrive(&sh->p_ready[i & 1]);
+        }
+        pdl_wait();                                               // (long over: for the gates and the results below)
+        if (n_walk > 0) wait(&sh->pv_done[(n_walk - 1) & 1], ((n_walk - 1) >> 1) & 1, 11);
+        tc_fence_after();
+        float* xl = &sh->xmax[n_walk & 1][0][0];                  // (the last page's maxima, in the other one, may still be read)
+        float f = 1.f;
+        if (!SIG) {
+            xl[half * 128 + r] = l;
+            ft_pair_sync(sw);
+            l += xl[(half ^ 1) * 128 + r];
+            const float m2 = m_ref * sc;
+            if (ex.sink != nullptr) {
+                const float mf = fmaxf(m2, sink2);
+                f = ft_ex2(m2 - mf);
+                l = l * f + ft_ex2(sink2 - mf);
+            }
+            f = l > 0.f ? f / l : 0.f;
+        }
+        if (ex.out_scale != 0.f) f *= ex.out_scale;
+        const int64_t row = row0 + r;
+        const bool wide = ex.gate != nullptr && ex.gate_wide > 0, live = r < n_rows;
+        if (ex.gate != nullptr && !wide && live) f *= 1.0f / (1.0f + expf(-__bfloat162float(((const bf16*)ex.gate)[row * ex.gate_ld + head])));
+        const bf16* gates = (const bf16*)ex.gate + row * ex.gate_ld + (int64_t)head * a.vd;
+        const int64_t at = row * (ex.out_ld > 0 ? ex.out_ld : (int64_t)a.q_heads * a.vd) + ex.out_col + (int64_t)head * a.vd;
+        if (!ok) sh->failed = 1;
+#pragma unroll 1
+        for (int c = half * a.nbv; c < (half + 1) * a.nbv; ++c) {
+            if (c * 32 >= a.vd) break;
+            float ov[32];
+            if (n_walk > 0) tc_ld32(tmem_o + lane_base + c * 32, ov);      // every lane takes part in the load
+            else
+#pragma unroll
+                for (int d = 0; d < 32; ++d) ov[d] = 0.f;
+            if (live) {
+                const int n = min(32, a.vd - c * 32);
+#pragma unroll
+                for (int d = 0; d < 32; ++d) ov[d] *= f;
+                if (wide) {
+#pragma unroll
+                    for (int d = 0; d < 32; ++d)
+                        if (d < n) ov[d] *= 1.0f / (1.0f + expf(-__bfloat162float(gates[c * 32 + d])));
+                }
+                if (ex.out_f32 > 0) {
+                    float* dst = (float*)a.out + at + c * 32;
+                    if (n == 32 && (((uintptr_t)dst) & 15) == 0) {
+#pragma unroll
+                        for (int d = 0; d < 32; d += 4) *reinterpret_cast<float4*>(dst + d) = make_float4(ov[d], ov[d + 1], ov[d + 2], ov[d + 3]);
+                    } else {
+#pragma unroll
+                        for (int d = 0; d < 32; ++d)
+                            if (d < n) dst[d] = ov[d];
+                    }
+                } else {
+                    bf16* dst = (bf16*)a.out + at + c * 32;
+                    if (n == 32 && (((uintptr_t)dst) & 15) == 0) {
+#pragma unroll
+                        for (int d = 0; d < 32; d += 8) tc_store8(dst + d, ov + d);
+                    } else {
+#pragma unroll
+                        for (int d = 0; d < 32; ++d)
+                            if (d < n) dst[d] = __float2bfloat16_rn(ov[d]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh->tmem_base), "r"(a.tmem_cols) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// host
+// ------------------------------------------------------------------------------------------------
+static size_t ft_smem(int dk, int vd, int v_from_k) {
+    const size_t nbk = (dk + 63) / 64, nbv = v_from_k > 0 ? 0 : (vd + 63) / 64;
+    const size_t need = nbk * 128 * 128 + 2 * (nbk + nbv) * 64 * 128 + sizeof(FlexTcShared);
+    // never more blocks on an SM than its tensor memory serves: two, or one whose values are wider than 128
+    const size_t least = ((v_from_k > 0 ? v_from_k : vd) > 128 ? 120 : 80) * 1024;
+    return need > least ? need : least;
+}
+
+// Whether the kernel takes these widths (0: no).
+X0NE_API int x0ne_attention_flex_tc_takes(int dk, int vd, int v_from_k) {
+    if (v_from_k > 0) vd = v_from_k;
+    return dk > 0 && vd > 0 && dk % 8 == 0 && vd % 8 == 0 && vd <= 256 && (v_from_k <= 0 || v_from_k <= dk) && ft_smem(dk, vd, v_from_k) <= 226 * 1024;
+}
+
+// q: bfloat16 rows (`q_rows` of them may be read), ex.q_ld values apart (0: the heads' width).  `status` as for the other tcgen05 kernels.
+X0NE_API int x0ne_attention_flex_prefill_tc(const void* q, void* out, int q_rows, PagedCache cache, const int32_t* tile_seq, const int32_t* tile_row0,
+                                            int n_tiles, const int32_t* seq_first_row, const int32_t* seq_slot, const int32_t* seq_pos0, int q_heads,
+                                            float scale, int window, AttnExtra ex, int* status, cudaStream_t stream) {
+    const int dk = cache.head_dim, vd = ex.v_from_k > 0 ? ex.v_from_k : cache_v_dim(cache);
+    X0NE_REQUIRE(q_heads > 0 && cache.kv_heads > 0 && q_heads % cache.kv_heads == 0, "attention_flex_tc: %d q heads over %d kv heads", q_heads, cache.kv_heads);
+    X0NE_REQUIRE(n_tiles >= 0 && n_tiles <= 65535 && window >= 0 && ex.chunk >= 0 && ex.keep_first >= 0 && q_rows > 0 && status != nullptr && scale > 0.f,
+                 "attention_flex_tc: bad sizes");
+    X0NE_REQUIRE(cache.page_size == 64 && (ex.v_from_k > 0 || cache.v_dim >= 0) && x0ne_attention_flex_tc_takes(dk, vd, ex.v_from_k),
+                 "attention_flex_tc: keys of %d, values of %d, pages of %d are not taken", dk, vd, cache.page_size);
+    const int64_t q_ld = ex.q_ld > 0 ? ex.q_ld : (int64_t)q_heads * dk;
+    X0NE_REQUIRE(((((uintptr_t)q) | ((uintptr_t)cache.base)) & 15) == 0 && q_ld % 8 == 0 && cache.page_stride % 8 == 0 && q_ld >= (int64_t)q_heads * dk,
+                 "attention_flex_tc: rows or pages are not 16-byte aligned");
+    if (n_tiles == 0) return 0;
+    CUtensorMap map_q, map_k, map_v;
+    if (int e = x0ne_tc_make_map_3d(&map_q, q, dk, q_heads, q_rows, dk, q_ld, 1, 128)) return e;
+    if (int e = x0ne_tc_make_map_3d(&map_k, cache.base, dk, (int64_t)cache.kv_heads * 64, cache.n_pages, dk, cache.page_stride, 64, 1)) return e;
+    if (ex.v_from_k > 0) map_v = map_k;
+    else if (int e = x0ne_tc_make_map_3d(&map_v, (const bf16*)cache.base + (int64_t)cache.kv_heads * 64 * dk, vd, (int64_t)cache.kv_heads * 64, cache.n_pages,
+                                         vd, cache.page_stride, 64, 1))
+        return e;
+    const int nbv = (vd + 63) / 64;
+    FlexTcArgs a{out, tile_seq, tile_row0, seq_first_row, seq_slot, seq_pos0, q_heads, window, vd, (dk + 63) / 64, nbv, nbv <= 2 ? 256 : 512, scale * FT_LOG2E};
+    const size_t smem = ft_smem(dk, vd, ex.v_from_k);
+    static OncePerDevice configured;
+    if (configured.need()) {
+        for (auto* k : {flex_prefill_tc_kernel<false>, flex_prefill_tc_kernel<true>}) {
+            cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+            X0NE_REQUIRE(e == cudaSuccess, "attention_flex_tc: shared memory: %s", cudaGetErrorString(e));
+        }
+        configured.done();
+    }
+    if (ex.sig_bias != nullptr)
+        x0ne_launch(flex_prefill_tc_kernel<true>, dim3(q_heads, n_tiles), dim3(FT_THREADS), smem, stream, map_q, map_k, map_v, a, cache, ex, status);
+    else
+        x0ne_launch(flex_prefill_tc_kernel<false>, dim3(q_heads, n_tiles), dim3(FT_THREADS), smem, stream, map_q, map_k, map_v, a, cache, ex, status);
+    X0NE_LAUNCH_CHECK();
+}

@@ -93,3 +93,6 @@ __device__ __forceinline__ void tc_store8(bf16* p, const float* v) {
 // A [rows, cols] row-major bfloat16 matrix as a TMA tensor map: boxes of box_rows x 64 values,
 // 128-byte swizzle, zeros outside the matrix (defined in gemm_tcgen05.cu).
 int x0ne_tc_make_map(CUtensorMap* map, const void* ptr, int64_t rows, int64_t cols, int box_rows);
+// A [n2][n1][n0] array of bfloat16 whose rows along n0 are `s1` values apart along n1 and `s2` along n2 as a TMA tensor map: boxes of
+// 64 x box1 x box2, 128-byte swizzle, zeros outside (defined in gemm_tcgen05.cu).
+int x0ne_tc_make_map_3d(CUtensorMap* map, const void* ptr, int64_t n0, int64_t n1, int64_t n2, int64_t s1, int64_t s2, int box1, int box2);
