@@ -513,3 +513,33 @@ def test_short_prompt_passes_replayed_from_graphs_give_the_same_bits():
             got.append((first, nxt))
         assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1]), lengths
     assert eng.pass_graph_replays - before >= 4
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 8, 13, 16, 17, 32])
+@pytest.mark.parametrize("inner,taps", [(40, 4), (264, 2)])
+def test_staged_scan_and_register_convolution_at_the_edges_of_their_stages(inner, n, taps):
+    """bfloat16 runs: sequences of 1, 15, 16, 17, 31, 32, 33, 64, 65 and 100 rows in one launch (rows that begin anywhere in a
+    stretch of the convolution, channels that end inside a block), a padding sequence, then a second launch from the kept state."""
+    from x0ne_engine_b200.csrc import ops
+    g = torch.Generator().manual_seed(n + inner)
+    lens = [1, 15, 16, 17, 31, 32, 33, 64, 65, 100]
+    rows = 2 * sum(lens)
+    xz, w, b, dt_raw, dt_bias, A, bc, D = scan_inputs(g, rows, inner, n, taps, torch.bfloat16)
+    state = torch.zeros((len(lens) + 1, inner * (n + taps - 1)), device=DEV)
+    first = [0]
+    for k in lens:
+        first.append(first[-1] + k)
+    slots = list(range(len(lens), 0, -1))
+    ys = []
+    for half in range(2):
+        at = half * sum(lens)
+        ys.append(run_mixer(ops, xz, w, b, dt_raw, dt_bias, A, bc, D, state, slice(at, at + sum(lens)), sum(([s] * k for s, k in zip(slots, lens)), []),
+                            sum((list(range(half * k, half * k + k)) for k in lens), []), first + first[-1:], slots + [-1], len(lens) + 1, inner, n, taps))
+    for s, k in enumerate(lens):
+        idx = list(range(first[s], first[s] + k)) + list(range(sum(lens) + first[s], sum(lens) + first[s] + k))
+        u_want, want, st = plain_mixer_rows(xz, w, b, dt_raw, dt_bias, A, bc, D, idx, n, inner, torch.bfloat16)
+        u, y = (torch.cat([ys[h][i][first[s]:first[s] + k] for h in range(2)]).double().cpu() for i in range(2))
+        assert (u - u_want).abs().max() <= 2 ** -8 * u_want.abs().max(), f"convolution, sequence {s}"
+        assert (y - want).abs().max() <= 2 ** -7 * want.abs().max(), f"scan, sequence {s}"
+        # (a token's hardware exponential is off by up to 2^-21 of its argument's size; states forget)
+        assert (state[slots[s], :inner * n].double().cpu().view(inner, n) - st["S"]).abs().max() <= 2e-4 * st["S"].abs().max()

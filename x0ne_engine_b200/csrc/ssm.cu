@@ -18,6 +18,10 @@
 
 #define SSM_THREADS 128    // per block of the scan: channels x the threads that share a channel's states
 #define SSM_TC 32          // tokens staged at a time
+#define SSM_STAGERS 256    // staging threads of the bfloat16 scan
+#define SSM_MANY_ROWS 0    // what a scan is told of the rows its sequences bring: nothing, one each, at most 16 each
+#define SSM_ONE_ROW 1
+#define SSM_FEW_ROWS 2
 #define SSM_MAX_TAPS 16
 
 // exp(a * b) for a * b <= 0, closer than the library's exponential (whose error of up to two units in the last place, met
@@ -44,6 +48,9 @@ __device__ __forceinline__ float ssm_exp_prod(float a, float b) {
 }
 
 __device__ __forceinline__ float ssm_silu(float v) { return v / (1.0f + expf(-v)); }
+// the same for results that are stored as bfloat16: the hardware's exponential and reciprocal, errors near 2^-21
+template <typename T> __device__ __forceinline__ float ssm_silu_for(float v) { return ssm_silu(v); }
+template <> __device__ __forceinline__ float ssm_silu_for<bf16>(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 __device__ __forceinline__ float ssm_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 // ----------------------------------------------------------------------------------------
@@ -82,7 +89,7 @@ __global__ void causal_conv_silu_kernel(const T* __restrict__ x, int64_t ld, con
         else if (slot >= 0) v = state[(int64_t)slot * state_stride + conv_off + (int64_t)(taps - 1 + above - back) * channels + c];
         acc = fmaf(wk[k], v, acc);
     }
-    out[(int64_t)row * channels + c] = from_f32<T>(ssm_silu(acc));
+    out[(int64_t)row * channels + c] = from_f32<T>(ssm_silu_for<T>(acc));
 }
 
 // The same for 8 consecutive channels per thread (channels and row pitch multiples of 8, 16-byte aligned rows): 16-byte
@@ -101,6 +108,10 @@ __device__ __forceinline__ void ssm_load8(const bf16* p, float* v) {
         v[2 * i + 1] = f.y;
     }
 }
+// 8 values as they lie in memory
+template <typename T> struct Raw8;
+template <> struct __align__(16) Raw8<bf16> { uint4 a = {0, 0, 0, 0}; };
+template <> struct __align__(16) Raw8<float> { float4 a = {0.f, 0.f, 0.f, 0.f}, b = {0.f, 0.f, 0.f, 0.f}; };
 __device__ __forceinline__ void ssm_store8(float* p, const float* v) {
     reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
     reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
@@ -111,6 +122,104 @@ __device__ __forceinline__ void ssm_store8(bf16* p, const float* v) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
     *reinterpret_cast<uint4*>(p) = r;
+}
+
+#define SSM_CONV_RUN 8          // rows a thread of the register convolution walks
+#define SSM_CONV_TAPS 4         // most taps it keeps
+
+// The same with a thread's taps and its stretch of rows in registers: all rows are asked for at once, each is read by one thread of a
+// column (and by the next stretch's for its first taps).  2,048 rows of 4,096 channels, 4 taps, bfloat16: 48 -> 27 us, with the
+// hardware's exponential and reciprocal behind it 16 (33.5 MB: 5.1 us at the copy rate; what is left is the activation).
+template <typename T>
+__global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
+        const T* x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias, const float* state, int64_t state_stride,
+        int64_t conv_off, T* __restrict__ out, const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int n_rows,
+        int channels, int taps) {
+    constexpr int BEFORE = SSM_CONV_TAPS - 1;
+    pdl_launch_dependents();
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 8, first = blockIdx.y * SSM_CONV_RUN;
+    if (c >= channels) {
+        pdl_wait();
+        return;
+    }
+    float wk[SSM_CONV_TAPS][8], b8[8];          // wk[k]: the tap that meets the input k tokens ago
+#pragma unroll
+    for (int i = 0; i < 8; ++i) b8[i] = 0.f;
+    if (bias != nullptr) ssm_load8(bias + c, b8);
+    if (taps == SSM_CONV_TAPS && (((uintptr_t)w) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 t = reinterpret_cast<const float4*>(w)[c + i];
+            wk[3][i] = t.x; wk[2][i] = t.y; wk[1][i] = t.z; wk[0][i] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int k = 0; k < SSM_CONV_TAPS; ++k) wk[k][i] = k < taps ? w[(int64_t)(c + i) * taps + taps - 1 - k] : 0.f;
+    }
+    pdl_wait();             // (x and the state are not __restrict__: reads that nothing may alias could be moved ahead of the wait)
+    // rows first - BEFORE .. first + RUN - 1, as they are stored
+    Raw8<T> raw[BEFORE + SSM_CONV_RUN];
+#pragma unroll
+    for (int r = 0; r < BEFORE + SSM_CONV_RUN; ++r) {
+        const int row = first - BEFORE + r;
+        raw[r] = row >= 0 && row < n_rows ? *reinterpret_cast<const Raw8<T>*>(x + (int64_t)row * ld + c) : Raw8<T>();
+    }
+    // a row whose `taps` - 1 rows above continue its sequence takes its inputs from them alone; where that holds for the whole stretch
+    // (for every thread of the block alike) nothing else is looked at
+    bool inner = first >= taps - 1 && first + SSM_CONV_RUN <= n_rows;
+    if (inner) {
+        const int slot = row_slot[first], pos = row_pos[first];
+#pragma unroll
+        for (int r = 1 - SSM_CONV_TAPS; r < SSM_CONV_RUN; ++r)
+            if (r > -taps) inner = inner && row_slot[first + r] == slot && row_pos[first + r] == pos + r;
+    }
+    if (inner) {
+#pragma unroll
+        for (int r = 0; r < SSM_CONV_RUN; ++r) {
+            float acc[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = b8[i];
+#pragma unroll
+            for (int back = BEFORE; back >= 0; --back) {
+                if (back < taps) {
+                    float v[8];
+                    ssm_load8(reinterpret_cast<const T*>(&raw[BEFORE + r - back]), v);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk[back][i], v[i], acc[i]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
+            ssm_store8(out + (int64_t)(first + r) * channels + c, acc);
+        }
+        return;
+    }
+#pragma unroll 1
+    for (int row = first; row < min(n_rows, first + SSM_CONV_RUN); ++row) {
+        const int slot = row_slot[row], pos = row_pos[row];
+        int above = 0;          // how many rows right above this one continue its sequence (at most taps - 1 are looked at)
+        while (above < taps - 1 && row - above - 1 >= 0 && row_slot[row - above - 1] == slot && row_pos[row - above - 1] == pos - above - 1) ++above;
+        float acc[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = b8[i];
+#pragma unroll
+        for (int back = BEFORE; back >= 0; --back) {
+            if (back >= taps) continue;
+            float v[8];
+            if (back <= above) ssm_load8(x + (int64_t)(row - back) * ld + c, v);
+            else if (slot >= 0) ssm_load8(state + (int64_t)slot * state_stride + conv_off + (int64_t)(taps - 1 + above - back) * channels + c, v);
+            else
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk[back][i], v[i], acc[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
+        ssm_store8(out + (int64_t)row * channels + c, acc);
+    }
 }
 
 #define SSM_CONV_ROWS 16        // rows a block of the vectorised convolution walks with its taps staged once (one row in short passes)
@@ -159,7 +268,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(
             for (int i = 0; i < 8; ++i) acc[i] = fmaf(w_s[(k * 8 + i) * 128 + tid], v[i], acc[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu(acc[i]);
+        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
         ssm_store8(out + (int64_t)row * channels + c, acc);
     }
 }
@@ -172,8 +281,20 @@ X0NE_API int x0ne_causal_conv_silu(const void* x, int64_t ld, int dt, const floa
     X0NE_REQUIRE(conv_off >= 0 && state_stride >= conv_off + (int64_t)(taps - 1) * channels, "causal_conv: the state row is too short");
     if (n_rows == 0) return 0;
     if (channels % 8 == 0 && ld % 8 == 0 && conv_off % 4 == 0 && state_stride % 4 == 0 && (dt == X0NE_F32 || dt == X0NE_BF16) &&
-        taps <= SSM_CONV_VEC_TAPS && n_rows <= 65535 * SSM_CONV_ROWS &&
+        taps <= SSM_CONV_VEC_TAPS && n_rows <= 65535 * SSM_CONV_RUN &&
         ((((uintptr_t)x | (uintptr_t)out | (uintptr_t)state | (uintptr_t)bias) & 15) == 0)) {
+        // (below 256 rows, a decoding batch among them, whose rows continue nobody's, a block per row is ahead: 55.6 us for a layer at
+        // 64 sequences against 59.8)
+        if (taps <= SSM_CONV_TAPS && n_rows >= 256) {
+            const dim3 rgrid((unsigned)((channels + 1023) / 1024), (unsigned)((n_rows + SSM_CONV_RUN - 1) / SSM_CONV_RUN));
+            if (dt == X0NE_F32)
+                x0ne_launch(causal_conv_silu_run_kernel<float>, rgrid, dim3(128), 0, stream, (const float*)x, ld, w, bias, state, state_stride, conv_off,
+                            (float*)out, row_slot, row_pos, n_rows, channels, taps);
+            else
+                x0ne_launch(causal_conv_silu_run_kernel<bf16>, rgrid, dim3(128), 0, stream, (const bf16*)x, ld, w, bias, state, state_stride, conv_off,
+                            (bf16*)out, row_slot, row_pos, n_rows, channels, taps);
+            X0NE_LAUNCH_CHECK();
+        }
         const int rpb = n_rows >= 256 ? SSM_CONV_ROWS : 1;
         const dim3 vgrid((unsigned)((channels + 1023) / 1024), (unsigned)((n_rows + rpb - 1) / rpb));
         if (dt == X0NE_F32)
@@ -259,11 +380,26 @@ __device__ __forceinline__ void ssm_keep_inputs(const SsmArgs& a, float* st, con
     }
 }
 
+__device__ __forceinline__ float ssm_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+template <int N> struct SsmVec;
+template <> struct SsmVec<4> { typedef float4 T; };
+template <> struct SsmVec<2> { typedef float2 T; };
+template <int NS> __device__ __forceinline__ void ssm_load_states(float (&v)[NS], const float* p) {
+    if constexpr (NS == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+    else if constexpr (NS == 2) *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(p);
+    else v[0] = p[0];
+}
+
 // A pass in which every sequence brings one row (or few): a thread reads its token's values itself, nothing is staged and
 // no thread waits for another.  The operations of a token and their order are the staged kernel's, so the bits are.
 template <typename T, int NS, int SSM_SPLIT>
 __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArgs a) {
     constexpr int SSM_CH = SSM_THREADS / SSM_SPLIT;
+    constexpr bool STAGED = sizeof(T) == 2 && NS * SSM_SPLIT <= 32;     // whether the scan of many rows is the staged kernel below
     pdl_launch_dependents();
     const int tid = threadIdx.x;
     const int cl = tid / SSM_SPLIT, part = tid % SSM_SPLIT;
@@ -275,7 +411,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArg
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
         const int n = part * NS + i;
-        An[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] : 0.f;
+        An[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] * (STAGED ? 1.4426950408889634f : 1.f) : 0.f;
     }
     if (live) {
         Dc = a.D != nullptr ? a.D[c] : 0.f;
@@ -304,11 +440,11 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArg
         for (int i = 0; i < NS; ++i) {
             const int n = part * NS + i;
             const float bn = n < a.N ? a.bc[r * a.bc_ld + a.b_col + n] : 0.f, cn = n < a.N ? a.bc[r * a.bc_ld + a.c_col + n] : 0.f;
-            S[i] = fmaf(SsmMath<T>::decay(dt, An[i]), S[i], dtu * bn);
+            S[i] = fmaf(STAGED ? ssm_ex2(dt * An[i]) : SsmMath<T>::decay(dt, An[i]), S[i], dtu * bn);
             acc = fmaf(S[i], cn, acc);
         }
 #pragma unroll
-        for (int w = 1; w < SSM_SPLIT; w <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
+        for (int w = 1; w < SSM_SPLIT; w <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, STAGED ? SSM_SPLIT / 2 / w : w);
         if (part == 0 && live)
             out[r * a.channels + c] = from_f32<T>(fmaf(Dc, uv, acc) * SsmMath<T>::silu(to_f32(xz[r * a.xz_ld + a.z_col + c])));
     }
@@ -464,17 +600,223 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_kernel(SsmArgs a) 
     if (part == 0) ssm_keep_inputs<T>(a, st, xz, row0, n_tok, c);
 }
 
-// How many threads share a channel: 4, 8 or 16 (more threads per channel are more warps to hide the latency of a token's
+// The scan of bfloat16 runs (up to 32 states per channel).  128 working threads carry the states, SPLIT (4 or 8) per channel with NS
+// states each in registers, 2 SPLIT tokens at a time: their exponentials first, then the states' chains, then the channel's threads
+// exchange partial sums so that each ends up with the sums of two tokens.  256 more threads stage: they fetch two stages of SSM_TC
+// tokens ahead, work out step sizes and gates on the way to shared memory (laid out [channel][token]: a working thread reads 4
+// tokens at once), and write the results of the stage before out, a row of the block's channels per warp.  One barrier per stage.
+// A token's exponentials, 16 per channel at 16 a clock and multiprocessor, are 30 us for 2,048 tokens of 4,096 channels, its shared
+// memory traffic and the staging's arithmetic about 40 each; the kernel takes 103 us (one state per thread, 16 threads per
+// channel, no staging threads: 296-327), 288 for 8,000 tokens of 9 sequences.  128 staging threads: 137; one group of SPLIT tokens at a time: 147.
+template <int NS, int SPLIT>
+__global__ void __launch_bounds__(SSM_THREADS + SSM_STAGERS, 2) selective_scan_staged_kernel(SsmArgs a) {
+    constexpr int CH = SSM_THREADS / SPLIT, U = SPLIT, NP = NS * SPLIT, PITCH = SSM_TC + 4, G = 2;
+    constexpr int TP = CH * SSM_TC / SSM_STAGERS;                  // tokens of one channel a staging thread brings per stage
+    constexpr int PER_N = (SSM_TC * NP + SSM_STAGERS - 1) / SSM_STAGERS;
+    static_assert(TP == 4 || TP == 2, "a staging thread's tokens are stored at once");
+    typedef typename SsmVec<TP>::T Vec;
+    __shared__ __align__(16) float s_dt[2][CH][PITCH], s_in[2][CH][PITCH], s_u[2][CH][PITCH], s_z[2][CH][PITCH];   // s_z: the gate, then the result
+    __shared__ __align__(16) float s_b[2][SSM_TC][NP], s_c[2][SSM_TC][NP];
+    pdl_launch_dependents();
+    const int seq = blockIdx.y;
+    const bool works = threadIdx.x < SSM_THREADS;
+    const int tid = works ? threadIdx.x : threadIdx.x - SSM_THREADS;
+    const int cl = tid / SPLIT, part = tid % SPLIT;
+    const int c = blockIdx.x * CH + cl;
+    const bool live = works && c < a.channels;
+    float A2[NS], S[NS];
+    float Dc = 0.f;
+    const int ch = tid % CH, t_own = tid / CH * TP, c_own = blockIdx.x * CH + ch;          // a staging thread's channel and tokens
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        const int n = part * NS + i;
+        A2[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] * 1.4426950408889634f : 0.f;
+    }
+    if (live && a.D != nullptr) Dc = a.D[c];
+    const bool owns = !works && c_own < a.channels;
+    const float dtb = owns && a.dt_bias != nullptr ? a.dt_bias[c_own] : 0.f;
+    pdl_wait();
+    const int slot = a.seq_slot[seq];
+    const int row0 = a.seq_first_row[seq], n_tok = a.seq_first_row[seq + 1] - row0;
+    if (slot < 0 || n_tok <= 0) return;
+    float* st = a.state + (int64_t)slot * a.state_stride;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        const int n = part * NS + i;
+        S[i] = live && n < a.N ? st[(int64_t)c * a.N + n] : 0.f;
+    }
+    const bf16* u = (const bf16*)a.u;
+    const bf16* xz = (const bf16*)a.xz;
+    bf16* out = (bf16*)a.out;
+
+    float f_dt[TP], f_b[PER_N], f_c[PER_N];
+    bf16 f_u[TP], f_z[TP];
+    const float* p_dt = a.dt_raw + (owns ? (int64_t)(row0 + t_own) * a.channels + c_own : 0);
+    const bf16* p_u = u + (owns ? (int64_t)(row0 + t_own) * a.channels + c_own : 0);
+    const bf16* p_z = xz + (owns ? (int64_t)(row0 + t_own) * a.xz_ld + a.z_col + c_own : 0);
+    bf16* p_out = out + (owns ? (int64_t)(row0 + t_own) * a.channels + c_own : 0);
+    auto fetch = [&](int t0) {
+        const int64_t at = (int64_t)t0 * a.channels, at_z = (int64_t)t0 * a.xz_ld;
+#pragma unroll
+        for (int k = 0; k < TP; ++k) {
+            const bool ok = owns && t0 + t_own + k < n_tok;
+            f_dt[k] = ok ? p_dt[at + (int64_t)k * a.channels] : 0.f;
+            f_u[k] = ok ? p_u[at + (int64_t)k * a.channels] : __ushort_as_bfloat16(0);
+            f_z[k] = ok ? p_z[at_z + k * a.xz_ld] : __ushort_as_bfloat16(0);
+        }
+#pragma unroll
+        for (int j = 0; j < PER_N; ++j) {
+            const int e = tid + j * SSM_STAGERS, t = t0 + e / NP, n = e % NP;
+            const bool ok = e < SSM_TC * NP && t < n_tok && n < a.N;
+            const int64_t r = row0 + (ok ? t : 0);
+            f_b[j] = ok ? a.bc[r * a.bc_ld + a.b_col + n] : 0.f;      // (a state past N, and a token past the last, must read as zero)
+            f_c[j] = ok ? a.bc[r * a.bc_ld + a.c_col + n] : 0.f;
+        }
+    };
+    auto stage = [&](int t0, int b) {
+        __align__(16) float dt[TP], in[TP], uv[TP], z[TP];
+#pragma unroll
+        for (int k = 0; k < TP; ++k) {
+            // a place past the sequence's last row gets a step of zero: it leaves the state as it is, bit for bit
+            const bool ok = t0 + t_own + k < n_tok;
+            dt[k] = ok ? SsmMath<bf16>::softplus(f_dt[k] + dtb) : 0.f;
+            uv[k] = ok ? to_f32(f_u[k]) : 0.f;
+            in[k] = dt[k] * uv[k];
+            z[k] = SsmMath<bf16>::silu(to_f32(f_z[k]));
+        }
+        *reinterpret_cast<Vec*>(&s_dt[b][ch][t_own]) = *reinterpret_cast<const Vec*>(dt);
+        *reinterpret_cast<Vec*>(&s_in[b][ch][t_own]) = *reinterpret_cast<const Vec*>(in);
+        *reinterpret_cast<Vec*>(&s_u[b][ch][t_own]) = *reinterpret_cast<const Vec*>(uv);
+        *reinterpret_cast<Vec*>(&s_z[b][ch][t_own]) = *reinterpret_cast<const Vec*>(z);
+#pragma unroll
+        for (int j = 0; j < PER_N; ++j) {
+            const int e = tid + j * SSM_STAGERS;
+            if (e < SSM_TC * NP) {
+                s_b[b][e / NP][e % NP] = f_b[j];
+                s_c[b][e / NP][e % NP] = f_c[j];
+            }
+        }
+    };
+    auto write_out = [&](int t0, int b) {
+        __align__(16) float y[TP];
+        *reinterpret_cast<Vec*>(y) = *reinterpret_cast<const Vec*>(&s_z[b][ch][t_own]);
+        const int64_t at = (int64_t)t0 * a.channels;
+#pragma unroll
+        for (int k = 0; k < TP; ++k)
+            if (owns && t0 + t_own + k < n_tok) p_out[at + (int64_t)k * a.channels] = __float2bfloat16_rn(y[k]);
+    };
+    if (!works) {
+        fetch(0);
+        stage(0, 0);
+        if (SSM_TC < n_tok) fetch(SSM_TC);
+    }
+    __syncthreads();
+    int b = 0;
+    for (int t0 = 0; t0 < n_tok; t0 += SSM_TC, b ^= 1) {
+        if (works) {
+#pragma unroll 2
+            for (int tl0 = 0; tl0 < SSM_TC && t0 + tl0 < n_tok; tl0 += G * U) {
+                __align__(16) float dt[G * U], in[G * U];
+                float dec[G * U][NS], put[G * U][NS], acc[G * U];
+#pragma unroll
+                for (int k = 0; k < G * U; k += 4) {
+                    *reinterpret_cast<float4*>(&dt[k]) = *reinterpret_cast<const float4*>(&s_dt[b][cl][tl0 + k]);
+                    *reinterpret_cast<float4*>(&in[k]) = *reinterpret_cast<const float4*>(&s_in[b][cl][tl0 + k]);
+                }
+#pragma unroll
+                for (int k = 0; k < G * U; ++k) {
+                    __align__(16) float B[NS];
+                    ssm_load_states<NS>(B, &s_b[b][tl0 + k][part * NS]);
+#pragma unroll
+                    for (int i = 0; i < NS; ++i) {
+                        dec[k][i] = ssm_ex2(dt[k] * A2[i]);
+                        put[k][i] = in[k] * B[i];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < G * U; ++k) {
+                    __align__(16) float C[NS];
+                    ssm_load_states<NS>(C, &s_c[b][tl0 + k][part * NS]);
+                    acc[k] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < NS; ++i) {
+                        S[i] = fmaf(dec[k][i], S[i], put[k][i]);
+                        acc[k] = fmaf(S[i], C[i], acc[k]);
+                    }
+                }
+                // the channel's threads share the tokens out: thread `part` ends up with the sums of tokens part and U + part
+#pragma unroll
+                for (int m = U / 2; m >= 1; m >>= 1) {
+                    const bool up = (part & m) != 0;
+#pragma unroll
+                    for (int g = 0; g < G; ++g) {
+#pragma unroll
+                        for (int k = 0; k < m; ++k) {
+                            const float send = up ? acc[g * U + k] : acc[g * U + k + m], keep = up ? acc[g * U + k + m] : acc[g * U + k];
+                            acc[g * U + k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+                        }
+                    }
+                }
+                float y[G];
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const int t = tl0 + g * U + part;
+                    y[g] = fmaf(Dc, s_u[b][cl][t], acc[g * U]) * s_z[b][cl][t];
+                }
+#pragma unroll
+                for (int g = 0; g < G; ++g) s_z[b][cl][tl0 + g * U + part] = y[g];
+            }
+        } else {
+            if (t0 > 0) write_out(t0 - SSM_TC, b ^ 1);
+            if (t0 + SSM_TC < n_tok) stage(t0 + SSM_TC, b ^ 1);
+            if (t0 + 2 * SSM_TC < n_tok) fetch(t0 + 2 * SSM_TC);
+        }
+        __syncthreads();
+    }
+    if (!works) {
+        write_out((n_tok - 1) / SSM_TC * SSM_TC, b ^ 1);
+        return;
+    }
+    if (!live) return;
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+        const int n = part * NS + i;
+        if (n < a.N) st[(int64_t)c * a.N + n] = S[i];
+    }
+    if (part == 0) ssm_keep_inputs<bf16>(a, st, xz, row0, n_tok, c);
+}
+
+// How many threads share a channel in the other kernels: 4, 8 or 16 (more threads per channel are more warps to hide the latency of a token's
 // dependent steps with, at more instructions in all; a single prompt's scan is bound by that latency, many sequences'
 // by the instructions).
 // A float32 run's choice depends on N alone, so that a token has the same bits in every pass; a bfloat16 run takes the
 // fewest threads per channel that still give every scheduler of the GPU a few warps.
 template <typename T>
-static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int one_token, cudaStream_t stream) {
+static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int rows, cudaStream_t stream) {
+    const bool one_token = rows == SSM_ONE_ROW;
+    // sequences of a few rows stay with the kernel of 128 threads a block, of which many fit on a multiprocessor: 16 sequences of 9 /
+    // 13 / 20 rows, a layer of 4,096 channels, 64.0 / 74.4 / 93.0 us with it, 74.3 / 82.3 / 80.1 staged; one sequence of 9: 39.4 and 39.7
+    if (sizeof(T) == 2 && rows == SSM_MANY_ROWS && a.N <= 32) {
+        // 8 threads per channel where 4 would leave more than a quarter of the multiprocessors without a block
+        const bool eight = a.N > 16 || (a.N > 4 && (int64_t)n_seqs * ((a.channels + 31) / 32) * 4 < (int64_t)sm_count * 3);
+        const int per = eight ? 16 : 32;
+        const dim3 sgrid((unsigned)((a.channels + per - 1) / per), (unsigned)n_seqs), sblock(SSM_THREADS + SSM_STAGERS);
+        if (eight) {
+            if (a.N <= 8) x0ne_launch(selective_scan_staged_kernel<1, 8>, sgrid, sblock, 0, stream, a);
+            else if (a.N <= 16) x0ne_launch(selective_scan_staged_kernel<2, 8>, sgrid, sblock, 0, stream, a);
+            else x0ne_launch(selective_scan_staged_kernel<4, 8>, sgrid, sblock, 0, stream, a);
+        } else {
+            if (a.N <= 4) x0ne_launch(selective_scan_staged_kernel<1, 4>, sgrid, sblock, 0, stream, a);
+            else if (a.N <= 8) x0ne_launch(selective_scan_staged_kernel<2, 4>, sgrid, sblock, 0, stream, a);
+            else x0ne_launch(selective_scan_staged_kernel<4, 4>, sgrid, sblock, 0, stream, a);
+        }
+        X0NE_LAUNCH_CHECK();
+    }
     int split = a.N > 32 ? 16 : 4;
     if (sizeof(T) == 2) {
         const int64_t want_warps = (int64_t)sm_count * 4 * 3;
-        while (split < 16 && split < a.N && (int64_t)n_seqs * a.channels * split / 32 < want_warps) split *= 2;
+        const int most = a.N > 32 || !one_token ? 16 : 8;         // (one token's bits are the staged scan's where both take 8)
+        while (split < most && split < a.N && (int64_t)n_seqs * a.channels * split / 32 < want_warps) split *= 2;
     }
     const int ns = (a.N + split - 1) / split;
     const dim3 grid((unsigned)((a.channels + SSM_THREADS / split - 1) / (SSM_THREADS / split)), (unsigned)n_seqs), block(SSM_THREADS);
@@ -506,7 +848,8 @@ static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int
     X0NE_LAUNCH_CHECK();
 }
 
-X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int one_token, cudaStream_t stream) {
+// `rows`: what is known of the sequences' rows (SSM_*_ROW*).
+X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int rows, cudaStream_t stream) {
     X0NE_REQUIRE(n_seqs >= 0 && n_seqs <= 65535 && a.channels > 0 && a.N > 0 && a.N <= 128 && a.taps >= 1 && a.taps <= SSM_MAX_TAPS,
                  "selective_scan: %d sequences, %d channels of %d states (at most %d), %d taps", n_seqs, a.channels, a.N, 128, a.taps);
     X0NE_REQUIRE(a.conv_off >= (int64_t)a.channels * a.N && a.state_stride >= a.conv_off + (int64_t)(a.taps - 1) * a.channels,
@@ -521,7 +864,7 @@ X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int one_token, c
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev >= 0 ? dev : 0) != cudaSuccess || sms <= 0) sms = 148;
         if (dev >= 0) sm_count[dev] = sms;
     }
-    if (dt == X0NE_F32) return selective_scan_launch<float>(a, n_seqs, sms, one_token, stream);
-    if (dt == X0NE_BF16) return selective_scan_launch<bf16>(a, n_seqs, sms, one_token, stream);
+    if (dt == X0NE_F32) return selective_scan_launch<float>(a, n_seqs, sms, rows, stream);
+    if (dt == X0NE_BF16) return selective_scan_launch<bf16>(a, n_seqs, sms, rows, stream);
     X0NE_REQUIRE(false, "selective_scan: unknown dtype tag %d", dt);
 }
