@@ -97,6 +97,28 @@ def test_gemm_f32_matches_and_rows_do_not_depend_on_the_batch(m, n, k):
 
 
 # ------------------------------------------------------------------------------------------ small-M bf16 product
+@pytest.mark.parametrize("n,k", [(4, 4), (33, 20), (130, 68), (65, 132), (2080, 64)])
+def test_gemm_f32_gives_a_row_the_same_bits_in_every_kernel_it_has(n, k):
+    """Row counts on both sides of every change of kernel (ragged tiles, ragged k, the scalar kernel for rows of another pitch)."""
+    o = ops()
+    rows = 300
+    x, w = rnd((rows, k), torch.float32, 21), rnd((n, k), torch.float32, 22)
+    want = torch.zeros((rows, n), dtype=torch.float32, device=DEV)
+    o.gemm_f32_nt(x, w, want, rows)
+    ref = x.double() @ w.double().T
+    assert (want.double() - ref).abs().max() <= k * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T).max()
+    for m in (1, 7, 8, 9, 16, 17, 32, 33, 64, 65, 66, 128, 129, 299):
+        for first in (0, rows - m):
+            y = torch.full((m + 1, n), 3.0, device=DEV)
+            o.gemm_f32_nt(x[first:first + m].contiguous(), w, y, m)
+            assert torch.equal(y[:m], want[first:first + m]) and bool((y[m] == 3.0).all()), (m, first)
+    odd = torch.zeros((rows * k + 1,), device=DEV)[1:].view(rows, k)        # rows that do not start on 16 bytes
+    odd.copy_(x)
+    y = torch.zeros_like(want)
+    o.gemm_f32_nt(odd, w, y, rows)
+    assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("n,k", [(16, 32), (100, 120), (333, 200), (4096, 1024)])
 def test_gemm_bf16_smallm(m, n, k):
