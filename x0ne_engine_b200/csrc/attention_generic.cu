@@ -129,6 +129,229 @@ __global__ void attention_rows_kernel(const T* __restrict__ q, T* __restrict__ o
     }
 }
 
+// The same in 32-bit for passes whose sequences bring several rows: up to 16 (row, q head) items that share a kv head walk their keys
+// together.  The plain kernel gives every item a warp whose lanes read a key row each straight from memory (32 rows apart, a
+// value at a time) and reads every row once per item; here a block of 4 warps copies a tile's rows to shared memory, 16 bytes at a
+// time, and a warp takes 4 items.  Tiles still begin at each row's first visible key, lanes own the same keys and every sum runs in
+// the plain kernel's order, so the bits are its bits: with a window the rows of a block begin up to 15 keys apart, and a tile
+// in shared memory holds that many more.  Rows of one sequence at consecutive positions go together; others in turn.
+// 700 rows of two sequences, 16 heads over 8 of 128: 1,561 -> 399 us.
+#define AP_ITEMS 4                         // of a warp
+#define AP_ROWS (32 + 4 * AP_ITEMS - 1)    // of a tile
+template <int NV>
+__global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos,
+                                                               int n_rows, int q_heads, float scale, int window, AttnExtra ex, int block_rows,
+                                                               int block_heads) {
+    extern __shared__ __align__(16) float ap_smem[];
+    const int hd = cache.head_dim, vd = ex.v_from_k > 0 ? ex.v_from_k : cache_v_dim(cache);
+    const int kp = hd + 4, vp = ex.v_from_k > 0 ? kp : vd;                    // (a warp's 16-byte reads of 32 key rows meet no bank twice)
+    float* qs = ap_smem;                                                    // [item][hd]
+    float* ks = qs + 4 * AP_ITEMS * hd;                                     // [key][kp]
+    float* vs = ex.v_from_k > 0 ? ks : ks + AP_ROWS * kp;                   // [key][vp]
+    __shared__ int key_ok[AP_ROWS];
+    pdl_prologue();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rep = q_heads / cache.kv_heads, chunks = (rep + block_heads - 1) / block_heads;
+    const int kh = blockIdx.y / chunks, head0 = kh * rep + blockIdx.y % chunks * block_heads;
+    const int heads = min(block_heads, (kh + 1) * rep - head0);
+    const int group = (gridDim.x - 1 - blockIdx.x) * block_rows, group_end = min(n_rows, group + block_rows);      // long rows first
+    const int64_t v_plane = (int64_t)cache.kv_heads * cache.page_size * hd;
+    const int64_t q_ld = ex.q_ld > 0 ? ex.q_ld : (int64_t)q_heads * hd;
+    const float* base = (const float*)cache.base;
+    auto first_key = [&](int pos) {
+        int lo = window > 0 ? max(0, pos - window + 1) : 0;
+        if (ex.chunk > 0) lo = max(lo, pos - pos % ex.chunk);
+        return lo;
+    };
+    for (int first = group; first < group_end;) {
+        // rows first .. first + n - 1: one sequence, consecutive positions, first keys close enough for one tile
+        const int slot = row_slot[first], pos0 = row_pos[first], lo0 = first_key(pos0);
+        int n = 1, tiles = (pos0 - lo0) / 32 + 1;
+        while (first + n < group_end && row_slot[first + n] == slot && row_pos[first + n] == pos0 + n && first_key(pos0 + n) - lo0 < 4 * AP_ITEMS) {
+            tiles = max(tiles, (pos0 + n - first_key(pos0 + n)) / 32 + 1);
+            ++n;
+        }
+        const int spread = first_key(pos0 + n - 1) - lo0, last = pos0 + n - 1;
+        __syncthreads();                    // the rows before are done with the tiles and the queries
+        for (int e = tid; e < n * heads * (hd / 4); e += 128) {
+            const int it = e / (hd / 4), d = e % (hd / 4) * 4;
+            const float4 v = *reinterpret_cast<const float4*>(q + (int64_t)(first + it / heads) * q_ld + (int64_t)(head0 + it % heads) * hd + d);
+            *reinterpret_cast<float4*>(qs + it * hd + d) = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
+        }
+        int pos[AP_ITEMS], lo[AP_ITEMS], head[AP_ITEMS];
+        float m[AP_ITEMS], l[AP_ITEMS], acc[AP_ITEMS][NV];
+#pragma unroll
+        for (int i = 0; i < AP_ITEMS; ++i) {
+            const int it = warp * AP_ITEMS + i;
+            const bool live = it < n * heads;
+            pos[i] = live ? pos0 + it / heads : -1;
+            lo[i] = live ? first_key(pos[i]) : lo0;
+            head[i] = live ? head0 + it % heads : head0;
+            m[i] = -INFINITY;
+            l[i] = 0.f;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[i][v] = 0.f;
+        }
+        for (int t = 0; t < tiles; ++t) {
+            const int j0 = lo0 + 32 * t, n_keys = min(32 + spread, last - j0 + 1);
+            __syncthreads();                // everybody is done with the tile before
+            for (int r = warp; r < n_keys; r += 4) {
+                const int64_t off = cache_row_offset(cache, slot, j0 + r, kh, 0);
+                if (lane == 0) key_ok[r] = off >= 0;
+                if (off >= 0) {
+                    for (int d = lane * 4; d < hd; d += 128) *reinterpret_cast<float4*>(ks + r * kp + d) = *reinterpret_cast<const float4*>(base + off + d);
+                    if (ex.v_from_k <= 0) {
+                        const float* vr = base + (off - off % cache.page_stride) + v_plane + ((off % cache.page_stride) / hd) * vd;
+                        for (int d = lane * 4; d < vd; d += 128) *reinterpret_cast<float4*>(vs + r * vp + d) = *reinterpret_cast<const float4*>(vr + d);
+                    }
+                }
+            }
+            __syncthreads();
+            float s[AP_ITEMS];
+#pragma unroll
+            for (int i = 0; i < AP_ITEMS; ++i) s[i] = 0.f;
+            const float* qw = qs + warp * AP_ITEMS * hd;
+            if (spread == 0) {
+                const float* kr = ks + min(lane, n_keys - 1) * kp;
+                for (int d = 0; d < hd; d += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+                    for (int i = 0; i < AP_ITEMS; ++i) {
+                        const float4 q4 = *reinterpret_cast<const float4*>(qw + i * hd + d);
+                        s[i] = fmaf(q4.x, k4.x, s[i]);
+                        s[i] = fmaf(q4.y, k4.y, s[i]);
+                        s[i] = fmaf(q4.z, k4.z, s[i]);
+                        s[i] = fmaf(q4.w, k4.w, s[i]);
+                    }
+                }
+            } else {
+                const float* kr[AP_ITEMS];
+#pragma unroll
+                for (int i = 0; i < AP_ITEMS; ++i) kr[i] = ks + min(lane + lo[i] - lo0, n_keys - 1) * kp;
+                for (int d = 0; d < hd; d += 4) {
+#pragma unroll
+                    for (int i = 0; i < AP_ITEMS; ++i) {
+                        const float4 k4 = *reinterpret_cast<const float4*>(kr[i] + d), q4 = *reinterpret_cast<const float4*>(qw + i * hd + d);
+                        s[i] = fmaf(q4.x, k4.x, s[i]);
+                        s[i] = fmaf(q4.y, k4.y, s[i]);
+                        s[i] = fmaf(q4.z, k4.z, s[i]);
+                        s[i] = fmaf(q4.w, k4.w, s[i]);
+                    }
+                }
+            }
+            float p[AP_ITEMS];
+            int nt[AP_ITEMS], most = 0;                 // keys of this tile that an item takes
+#pragma unroll
+            for (int i = 0; i < AP_ITEMS; ++i) {
+                const int j = lo[i] + 32 * t + lane;
+                const bool ok = j <= pos[i] && key_ok[min(lane + lo[i] - lo0, AP_ROWS - 1)] != 0;
+                nt[i] = min(32, pos[i] - (lo[i] + 32 * t) + 1);
+                if (nt[i] <= 0) {
+                    p[i] = 0.f;
+                    continue;
+                }
+                float a = s[i];
+                a = !ok ? -INFINITY : ex.slope != nullptr ? a - ex.slope[head[i]] * (float)(pos[i] - j) : a;
+                float m_new = m[i];
+                if (ex.sig_bias != nullptr) {
+                    p[i] = ok ? 1.0f / (1.0f + expf(-(a + ex.sig_bias[head[i]]))) : 0.f;
+                } else {
+                    m_new = fmaxf(m[i], warp_max(a));
+                    if (m_new == -INFINITY) {           // no readable key in this tile
+                        nt[i] = 0;
+                        p[i] = 0.f;
+                        continue;
+                    }
+                    p[i] = ok ? expf(a - m_new) : 0.f;
+                    const float alpha = expf(m[i] - m_new);
+                    l[i] = l[i] * alpha + warp_sum(p[i]);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) acc[i][v] *= alpha;
+                }
+                m[i] = m_new;
+                most = max(most, nt[i]);
+            }
+            for (int k = 0; k < most; ++k) {
+                float val[NV];
+                if (spread == 0 && key_ok[k]) {
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) val[v] = lane + 32 * v < vd ? vs[k * vp + lane + 32 * v] : 0.f;
+                }
+#pragma unroll
+                for (int i = 0; i < AP_ITEMS; ++i) {
+                    const float pk = __shfl_sync(0xffffffffu, p[i], k);
+                    const int r = k + lo[i] - lo0;
+                    if (k >= nt[i] || !key_ok[r]) continue;
+                    if (spread != 0) {
+#pragma unroll
+                        for (int v = 0; v < NV; ++v) val[v] = lane + 32 * v < vd ? vs[r * vp + lane + 32 * v] : 0.f;
+                    }
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) acc[i][v] = fmaf(pk, val[v], acc[i][v]);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < AP_ITEMS; ++i) {
+            if (pos[i] < 0) continue;
+            const int row = first + pos[i] - pos0;
+            if (ex.sink != nullptr && slot >= 0 && ex.sig_bias == nullptr) {
+                const float sk = ex.sink[head[i]];
+                const float m_new = fmaxf(m[i], sk);
+                const float alpha = expf(m[i] - m_new);
+                l[i] = l[i] * alpha + expf(sk - m_new);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) acc[i][v] *= alpha;
+            }
+            float* o = out + (int64_t)row * (ex.out_ld > 0 ? ex.out_ld : (int64_t)q_heads * vd) + ex.out_col + (int64_t)head[i] * vd;
+            float inv = ex.sig_bias != nullptr ? 1.f : l[i] > 0.f ? 1.0f / l[i] : 0.f;
+            if (ex.out_scale != 0.f) inv *= ex.out_scale;
+            const float* gate = (const float*)ex.gate + (int64_t)row * ex.gate_ld;
+            if (ex.gate != nullptr && ex.gate_wide <= 0) inv *= 1.0f / (1.0f + expf(-gate[head[i]]));
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int d = lane + 32 * v;
+                if (d < vd) o[d] = ex.gate != nullptr && ex.gate_wide > 0 ? acc[i][v] * inv * (1.0f / (1.0f + expf(-gate[(int64_t)head[i] * vd + d]))) : acc[i][v] * inv;
+            }
+        }
+        first += n;
+    }
+}
+
+static size_t ap_smem_bytes(int hd, int vd, bool v_from_k) {
+    return ((size_t)4 * AP_ITEMS * hd + (size_t)AP_ROWS * (hd + 4) + (v_from_k ? 0 : (size_t)AP_ROWS * vd)) * sizeof(float);
+}
+
+// float32 queries, cache and results; keys of up to 512 and values of up to 256 values, both multiples of four; no kept first keys.
+X0NE_API int x0ne_attention_prompt_f32(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos, int n_rows,
+                                       int q_heads, float scale, int window, AttnExtra ex, cudaStream_t stream) {
+    X0NE_REQUIRE(n_rows >= 0 && q_heads > 0 && cache.kv_heads > 0 && q_heads % cache.kv_heads == 0,
+                 "attention: %d q heads over %d kv heads", q_heads, cache.kv_heads);
+    const int hd = cache.head_dim, vd = ex.v_from_k > 0 ? ex.v_from_k : cache_v_dim(cache), rep = q_heads / cache.kv_heads;
+    const int64_t q_ld = ex.q_ld > 0 ? ex.q_ld : (int64_t)q_heads * hd;
+    X0NE_REQUIRE(hd > 0 && hd <= 512 && hd % 4 == 0 && vd > 0 && vd <= 256 && vd % 4 == 0 && ex.v_from_k <= hd && window >= 0 && ex.chunk >= 0 && ex.keep_first == 0 &&
+                     q_ld % 4 == 0 && cache.page_stride % 4 == 0 && ((((uintptr_t)q) | ((uintptr_t)cache.base)) & 15) == 0,
+                 "attention: keys of %d and values of %d, or what is asked of them, are not for the kernel of several rows", hd, vd);
+    if (n_rows == 0) return 0;
+    const int block_heads = rep < 4 * AP_ITEMS ? rep : 4 * AP_ITEMS, block_rows = 4 * AP_ITEMS / block_heads;
+    const int64_t chunks = (rep + block_heads - 1) / block_heads;
+    X0NE_REQUIRE(chunks * cache.kv_heads <= 65535, "attention: too many heads");
+    const dim3 grid((unsigned)((n_rows + block_rows - 1) / block_rows), (unsigned)(chunks * cache.kv_heads));
+    const size_t smem = ap_smem_bytes(hd, vd, ex.v_from_k > 0);
+    static OncePerDevice configured;
+    if (configured.need()) {
+        for (auto* k : {attention_prompt_kernel<2>, attention_prompt_kernel<4>, attention_prompt_kernel<8>}) {
+            cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            X0NE_REQUIRE(e == cudaSuccess, "attention: shared memory: %s", cudaGetErrorString(e));
+        }
+        configured.done();
+    }
+    if (vd <= 64) x0ne_launch(attention_prompt_kernel<2>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
+    else if (vd <= 128) x0ne_launch(attention_prompt_kernel<4>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
+    else x0ne_launch(attention_prompt_kernel<8>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
+    X0NE_LAUNCH_CHECK();
+}
+
 X0NE_API int x0ne_attention_rows_ex(const void* q, void* out, int dt, PagedCache cache, const int32_t* row_slot,
                                     const int32_t* row_pos, int n_rows, int q_heads, float scale, int window,
                                     AttnExtra ex, cudaStream_t stream) {

@@ -17,7 +17,7 @@ def run_attention(ctx, q, out, view, n_rows, q_heads, scale, window):
     """Chooses the attention kernel for this step: the tensor-core kernels where they take the
     shape, else the plain kernel (which is also the whole 32-bit path)."""
     if not ops.fast_attention_takes(view, q.dtype):
-        ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window)
+        ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window, prompt=not ctx.decode)
     elif ctx.decode:
         # up to 8 splits merge inside a thread-block cluster and need no scratch; several clusters
         # per (sequence, kv head) leave one partial result each in a scratch of the workspace
@@ -71,7 +71,7 @@ def run_attention_ex(ctx, q, out, view, n_rows, q_heads, scale, window, extra):
     sink, gate, queries inside a wider buffer): the general bfloat16 kernels where they take the
     shape, else the plain kernel (which is also the whole 32-bit path)."""
     if not ops.attention_flex_takes(view, q.dtype, extra.v_from_k, ctx.decode):
-        ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window, extra)
+        ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window, extra, prompt=not ctx.decode)
     elif ctx.decode:
         visible = min(v for v in (ctx.max_context, extra.chunk, window + extra.keep_first if window else 0) if v)
         splits = flex_decode_splits(ctx, n_rows, view.kv_heads, q_heads, visible)
