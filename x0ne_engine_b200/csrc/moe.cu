@@ -167,6 +167,7 @@ __global__ void moe_route_kernel(const float* __restrict__ z, int ldz, const flo
 //   tiles   [max_tiles][3]  expert, first place, count (count 0: the tile does not exist); tiles of tile_m pairs
 //   n_tiles_out             how many tiles exist (optional)
 // ----------------------------------------------------------------------------------------
+#define GP_OWN 8        // choices of a thread that stay in registers
 __global__ void moe_group_kernel(const int32_t* __restrict__ chosen, int pairs, int experts, int32_t* __restrict__ offsets,
                                  int32_t* __restrict__ listed, int32_t* __restrict__ tiles, int max_tiles, int tile_m,
                                  int32_t* __restrict__ n_tiles_out) {
@@ -175,9 +176,19 @@ __global__ void moe_group_kernel(const int32_t* __restrict__ chosen, int pairs, 
     int* start = count + experts;         // [experts + 1]
     int* tile0 = start + experts + 1;     // [experts + 1]
     pdl_prologue();
+    // a thread's first choices stay in registers for both walks, asked for together (8,192 pairs: 15 -> 6 us)
+    int own[GP_OWN];
+#pragma unroll
+    for (int i = 0; i < GP_OWN; ++i) {
+        const int p = threadIdx.x + i * blockDim.x;
+        own[i] = p < pairs ? chosen[p] : -1;
+    }
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+#pragma unroll
+    for (int i = 0; i < GP_OWN; ++i)
+        if (own[i] >= 0 && own[i] < experts) atomicAdd(&count[own[i]], 1);
+    for (int p = threadIdx.x + GP_OWN * blockDim.x; p < pairs; p += blockDim.x) {
         const int e = chosen[p];
         if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
     }
@@ -208,7 +219,10 @@ __global__ void moe_group_kernel(const int32_t* __restrict__ chosen, int pairs, 
     __syncthreads();
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+#pragma unroll
+    for (int i = 0; i < GP_OWN; ++i)
+        if (own[i] >= 0 && own[i] < experts) listed[start[own[i]] + atomicAdd(&count[own[i]], 1)] = threadIdx.x + i * blockDim.x;
+    for (int p = threadIdx.x + GP_OWN * blockDim.x; p < pairs; p += blockDim.x) {
         const int e = chosen[p];
         if (e >= 0 && e < experts) listed[start[e] + atomicAdd(&count[e], 1)] = p;
     }
@@ -353,21 +367,23 @@ __device__ __forceinline__ void cmb_store4(bf16* p, const float* v) {
     *reinterpret_cast<uint2*>(p) = u;
 }
 #define CMB_MAX_TOP 16
-template <typename T>
-__global__ void moe_combine_vec_kernel(const float* __restrict__ y, const T* __restrict__ x, const int32_t* __restrict__ chosen,
-                                       const float* __restrict__ weights, int top, int experts, const T* __restrict__ shared,
-                                       const float* __restrict__ sgate, T* __restrict__ out, int hidden) {
+// TOP: the most choices a row may have (registers for 16 leave a third of the threads on a multiprocessor: 2,048 rows of 2,048 with 4
+// choices 31 us, with registers for 4 14).
+template <typename T, int TOP>
+__global__ void moe_combine_vec_kernel(const float* y, const T* x, const int32_t* chosen,
+                                       const float* weights, int top, int experts, const T* shared,
+                                       const float* sgate, T* out, int hidden) {
     pdl_prologue();
     const int row = blockIdx.y;
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (c >= hidden) return;
     const int32_t* ch = chosen + (int64_t)row * top;
     const float* wt = weights + (int64_t)row * top;
-    float v[CMB_MAX_TOP][4], g[CMB_MAX_TOP];
+    float v[TOP][4], g[TOP];
     float xs[4], sv[4] = {0.f, 0.f, 0.f, 0.f};
     cmb_load4(x + (int64_t)row * hidden + c, xs);
 #pragma unroll
-    for (int j = 0; j < CMB_MAX_TOP; ++j) {
+    for (int j = 0; j < TOP; ++j) {
         if (j < top) {
             g[j] = wt[j];
             if (ch[j] < experts) cmb_load4(y + ((int64_t)row * top + j) * hidden + c, v[j]);      // (all the loads are in flight together)
@@ -378,7 +394,7 @@ __global__ void moe_combine_vec_kernel(const float* __restrict__ y, const T* __r
     if (shared != nullptr) cmb_load4(shared + (int64_t)row * hidden + c, sv);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < CMB_MAX_TOP; ++j)
+    for (int j = 0; j < TOP; ++j)
         if (j < top) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) acc[k] = fmaf(g[j], v[j][k], acc[k]);
@@ -461,10 +477,17 @@ X0NE_API int x0ne_moe_combine(const float* y, const void* x, int dt, const int32
         ((((uintptr_t)y | (uintptr_t)x | (uintptr_t)shared | (uintptr_t)out) & 15) == 0)) {
         const int threads = hidden / 4 >= 256 ? 256 : (hidden / 4 + 31) / 32 * 32;
         const dim3 grid((hidden / 4 + threads - 1) / threads, n_rows);
-        if (dt == X0NE_F32)
-            x0ne_launch(moe_combine_vec_kernel<float>, grid, dim3(threads), 0, stream, y, (const float*)x, chosen, weights, top, experts, (const float*)shared, sgate, (float*)out, hidden);
-        else
-            x0ne_launch(moe_combine_vec_kernel<bf16>, grid, dim3(threads), 0, stream, y, (const bf16*)x, chosen, weights, top, experts, (const bf16*)shared, sgate, (bf16*)out, hidden);
+#define CMB_GO(T, TOP)                                                                                                                        \
+    x0ne_launch(moe_combine_vec_kernel<T, TOP>, grid, dim3(threads), 0, stream, y, (const T*)x, chosen, weights, top, experts, (const T*)shared, \
+                sgate, (T*)out, hidden)
+        if (dt == X0NE_F32) {
+            if (top <= 4) CMB_GO(float, 4);
+            else CMB_GO(float, CMB_MAX_TOP);
+        } else {
+            if (top <= 4) CMB_GO(bf16, 4);
+            else CMB_GO(bf16, CMB_MAX_TOP);
+        }
+#undef CMB_GO
         X0NE_LAUNCH_CHECK();
     }
     if (dt == X0NE_F32)
