@@ -13,6 +13,7 @@ sequences of unequal length share a pass and padding never exists.
 """
 from __future__ import annotations
 
+from array import array
 from collections import OrderedDict
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
@@ -47,6 +48,17 @@ def padded_rows(n: int) -> int:
         return n
     step = 16 if n <= 64 else 64
     return -(-n // step) * step
+
+
+def _token_ids(tokens) -> np.ndarray:
+    """A sequence's token ids as int64.  Lists of Python ints, what callers hold, go through `array`: 9,456 ids in 0.15 ms against
+    0.45 through NumPy's own reading of lists; anything else is NumPy's to read."""
+    if type(tokens) is list:
+        try:
+            return np.frombuffer(array("q", tokens), dtype=np.int64)
+        except (TypeError, OverflowError):
+            pass
+    return np.asarray(tokens, dtype=np.int64)
 
 
 class StepError(ValueError):
@@ -201,7 +213,7 @@ class Engine:
             if start + n > self.max_seq_len:
                 raise StepError(f"slot {s}: {start} + {n} tokens exceed the longest sequence, {self.max_seq_len}")
             starts.append(start)
-        flat = np.concatenate([np.asarray(t, dtype=np.int64) for t in tokens])
+        flat = np.concatenate([_token_ids(t) for t in tokens])
         if flat.min() < 0 or flat.max() >= self.vocab_size:
             raise StepError(f"a token id lies outside the vocabulary of {self.vocab_size}")
         if want is None:
