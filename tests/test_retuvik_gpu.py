@@ -367,6 +367,33 @@ def test_attention_kernels_with_distance_bias_and_a_gate_per_value(case):
             assert (out.double().cpu().view(T, H_, Dv) - want).abs().max() <= tol * want.abs().max(), ("decode", splits)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [32, 50, 64])
+def test_scan_of_a_few_blocks_gives_the_bits_of_the_scan_of_many(dtype, n):
+    """Sequences of 1 to 35 tokens alone (a block to a multiprocessor: the form of four tokens at a time, with remainders) and 40 at once."""
+    from x0ne_engine_b200.csrc import ops
+    heads, width, lens = 2, 2 * n, [1, 3, 4, 5, 7, 15, 16, 17, 33, 35] * 4
+    g = torch.Generator().manual_seed(n)
+    rows = sum(lens)
+    mk = lambda *s: torch.randn(*s, generator=g)
+    r, k, v = (mk(rows, heads * n).to(dtype).to(DEV) for _ in range(3))
+    h = mk(rows, width).to(dtype).to(DEV)
+    z, w0, u = mk(rows, heads * n).to(DEV), (mk(heads * n) - 2.0).to(DEV), mk(heads * n).to(DEV)
+    start = mk(len(lens), heads * n * n + width).to(DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    first = [0]
+    for c in lens:
+        first.append(first[-1] + c)
+    whole, o = start.clone(), torch.zeros(rows, heads * n, device=DEV)
+    ops.wkv_scan(r, k, v, z, w0, u, h, o, whole, i32(first), i32(list(range(len(lens)))), len(lens), heads, n)
+    for s in range(10):
+        a, b = first[s], first[s + 1]
+        alone, oa = start.clone(), torch.zeros(b - a, heads * n, device=DEV)
+        cut = lambda t: t[a:b].contiguous()      # noqa: E731
+        ops.wkv_scan(cut(r), cut(k), cut(v), cut(z), w0, u, cut(h), oa, alone, i32([0, b - a]), i32([s]), 1, heads, n)
+        assert torch.equal(oa, o[a:b]) and torch.equal(alone[s], whole[s]), lens[s]
+
+
 # ------------------------------------------------------------------------------------------ the recurrence's kernels
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_token_shift_blends(dtype):

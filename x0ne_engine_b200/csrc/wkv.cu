@@ -15,6 +15,8 @@
 // and every sum are float32; r, k, v, the gate and h come in the activation type.  A sequence's result depends
 // on its own rows and state only, and every sum runs in one fixed order, so it is the same bits however the
 // sequence's tokens are cut into passes and whatever else is in a pass.
+#include <type_traits>
+
 #include "common.cuh"
 
 // ----------------------------------------------------------------------------------------
@@ -106,7 +108,7 @@ __global__ void token_shift_mix_vec_kernel(const T* __restrict__ h, const float*
 //     channels, v of its two columns), 8 steps of the recurrence, one exchange with its neighbour in g (the first
 //     level of the tree: one of the two goes on with the first column, the other with the second) and one store of
 //     that sum to shared memory.  Only S is carried from token to token.
-//   * WKV_PRODUCERS staging threads: they fetch r, k, v and the decay exponents two stages ahead into registers, work
+//   * the staging threads: they fetch r, k, v and the decay exponents two stages ahead into registers, work
 //     out w = exp(-exp(z + w0)) and put all of it into the other half of a double buffer while the current half is
 //     used; then they add the partial sums of the stage before (the tree's other levels) and write out.
 // wkv_step_kernel (one token per sequence): one block per (sequence, head); thread (j, y) reads, uses and writes back
@@ -114,7 +116,12 @@ __global__ void token_shift_mix_vec_kernel(const T* __restrict__ h, const float*
 // ----------------------------------------------------------------------------------------
 #define WKV_CB 16             // value columns of a block of the scan over many tokens
 #define WKV_GI 4              // key channels of a group
-#define WKV_PRODUCERS 128     // staging threads of a block
+// A launch whose blocks each have a multiprocessor to themselves waits for latencies: it gets twice the staging threads and its working
+// threads take four tokens at a time (one sequence of 2,048 tokens, 32 heads of 64: 225 -> 152 us, of 1,000, 16 heads: 97 -> 76).  Where
+// blocks share one, or take turns, fewer threads are ahead (64 heads 266 us, with the wide form 311; 16 sequences of 10 tokens 29 and 43).
+// The operations of a token and their order are the same.
+#define WKV_PRODUCERS 128
+#define WKV_WIDE_PRODUCERS 256
 
 template <int G>
 __device__ __forceinline__ float wkv_tree_sum(float (&q)[G]) {
@@ -125,8 +132,8 @@ __device__ __forceinline__ float wkv_tree_sum(float (&q)[G]) {
     return q[0];
 }
 
-template <typename T, int NB>
-__global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
+template <typename T, int NB, int PRODUCERS, int U_>
+__global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
                                                                          const float* __restrict__ z, const float* __restrict__ w0,
                                                                          const float* __restrict__ u, const T* __restrict__ h,
                                                                          float* __restrict__ o, float* __restrict__ state, int64_t state_stride,
@@ -136,10 +143,10 @@ __global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const 
     constexpr int H = G / 2;                        // partial sums of a column that reach shared memory
     constexpr int NC = G * (WKV_CB / 2);            // working threads: 2 NB
     constexpr int TB = NB <= 64 ? 16 : 8;           // tokens staged at a time
-    constexpr int PER = TB * NB / WKV_PRODUCERS;    // values of r, k, z a staging thread fetches per stage
-    constexpr int PV = TB * WKV_CB / WKV_PRODUCERS; // values of v, and results it adds up
-    constexpr int TSTEP = WKV_PRODUCERS / NB;
-    static_assert(H >= 4 && (G & (G - 1)) == 0 && G <= 32 && WKV_PRODUCERS % NB == 0 && PER >= 1 && PV >= 1 && NC == 2 * NB, "tile shape");
+    constexpr int PER = TB * NB / PRODUCERS;    // values of r, k, z a staging thread fetches per stage
+    constexpr int PV = TB * WKV_CB / PRODUCERS; // values of v, and results it adds up
+    constexpr int TSTEP = PRODUCERS / NB;
+    static_assert(H >= 4 && (G & (G - 1)) == 0 && G <= 32 && PRODUCERS % NB == 0 && PER >= 1 && PV >= 1 && NC == 2 * NB, "tile shape");
     __shared__ __align__(16) float rs[2][TB][NB], ks[2][TB][NB], ws[2][TB][NB], vs[2][TB][WKV_CB];
     __shared__ __align__(16) float part[2][TB][WKV_CB][H];
     pdl_launch_dependents();
@@ -165,7 +172,8 @@ __global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const 
     float* S = state + (int64_t)slot * state_stride + (int64_t)head * N * N;
     const int n_stages = (row1 - row0 + TB - 1) / TB;
 
-    float fr[PER], fk[PER], fz[PER], fv[PV];            // a staging thread's share of one stage, on its way
+    T fr[PER], fk[PER], fv[PV];          // a staging thread's share of one stage, on its way (as it was read: a conversion would wait for it)
+    float fz[PER];
     auto fetch = [&](int at_stage) {
         const int t0 = row0 + at_stage * TB;
 #pragma unroll
@@ -173,35 +181,35 @@ __global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const 
             // every fetch is made, from an address inside the sequence's rows, so that none waits for another;
             // rows past the sequence's last are not used, channels past the head's last are zeroed in `put`
             const int64_t at = (int64_t)min(t0 + ptb + x * TSTEP, row1 - 1) * ld + (int64_t)head * N + min(pi, N - 1);
-            fr[x] = to_f32(r[at]);
-            fk[x] = to_f32(k[at]);
+            fr[x] = r[at];
+            fk[x] = k[at];
             fz[x] = z[at];
         }
 #pragma unroll
         for (int x = 0; x < PV; ++x) {
-            const int e = pt + x * WKV_PRODUCERS, t = e / WKV_CB, c = e % WKV_CB;
-            fv[x] = to_f32(v[(int64_t)min(t0 + t, row1 - 1) * ld + (int64_t)head * N + min(j0 + c, N - 1)]);
+            const int e = pt + x * PRODUCERS, t = e / WKV_CB, c = e % WKV_CB;
+            fv[x] = v[(int64_t)min(t0 + t, row1 - 1) * ld + (int64_t)head * N + min(j0 + c, N - 1)];
         }
     };
     auto put = [&](int buf) {
 #pragma unroll
         for (int x = 0; x < PER; ++x) {
             const int t = ptb + x * TSTEP;
-            rs[buf][t][pi] = pi < N ? fr[x] : 0.f;
-            ks[buf][t][pi] = pi < N ? fk[x] : 0.f;
+            rs[buf][t][pi] = pi < N ? to_f32(fr[x]) : 0.f;
+            ks[buf][t][pi] = pi < N ? to_f32(fk[x]) : 0.f;
             ws[buf][t][pi] = pi < N ? expf(-expf(fz[x] + w0r)) : 0.f;
         }
 #pragma unroll
         for (int x = 0; x < PV; ++x) {
-            const int e = pt + x * WKV_PRODUCERS, c = e % WKV_CB;
-            vs[buf][e / WKV_CB][c] = j0 + c < N ? fv[x] : 0.f;
+            const int e = pt + x * PRODUCERS, c = e % WKV_CB;
+            vs[buf][e / WKV_CB][c] = j0 + c < N ? to_f32(fv[x]) : 0.f;
         }
     };
     auto write_out = [&](int at_stage, int buf) {       // the results of a stage the working threads are done with
         const int t0 = row0 + at_stage * TB;
 #pragma unroll
         for (int x = 0; x < PV; ++x) {
-            const int e = pt + x * WKV_PRODUCERS, t = e / WKV_CB, c = e % WKV_CB;
+            const int e = pt + x * PRODUCERS, t = e / WKV_CB, c = e % WKV_CB;
             if (t0 + t >= row1 || j0 + c >= N) continue;
             float q[H];
 #pragma unroll
@@ -236,27 +244,47 @@ __global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const 
             const int nt = min(TB, row1 - (row0 + it * TB));
             const bool odd = (g & 1) != 0;
             float* mine = &part[buf][0][jc + (odd ? 1 : 0)][g >> 1];
-#pragma unroll 4
-            for (int t = 0; t < nt; ++t) {
-                const float4 r4 = *reinterpret_cast<const float4*>(&rs[buf][t][i0]);
-                const float4 k4 = *reinterpret_cast<const float4*>(&ks[buf][t][i0]);
-                const float4 w4 = *reinterpret_cast<const float4*>(&ws[buf][t][i0]);
-                const float2 v2 = *reinterpret_cast<const float2*>(&vs[buf][t][jc]);
-                const float rr[4] = {r4.x, r4.y, r4.z, r4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w};
-                const float ww[4] = {w4.x, w4.y, w4.z, w4.w}, vv[2] = {v2.x, v2.y};
-                float acc[2] = {0.f, 0.f};
+            // U tokens at a time: all they read is asked for first and their sums are exchanged together
+            auto walk = [&](int t0, auto tokens) {
+                constexpr int U = decltype(tokens)::value;
+                float4 r4[U], k4[U], w4[U];
+                float2 v2[U];
+                float acc[U][2];
 #pragma unroll
-                for (int a = 0; a < WKV_GI; ++a)
+                for (int t = 0; t < U; ++t) {
+                    r4[t] = *reinterpret_cast<const float4*>(&rs[buf][t0 + t][i0]);
+                    k4[t] = *reinterpret_cast<const float4*>(&ks[buf][t0 + t][i0]);
+                    w4[t] = *reinterpret_cast<const float4*>(&ws[buf][t0 + t][i0]);
+                    v2[t] = *reinterpret_cast<const float2*>(&vs[buf][t0 + t][jc]);
+                }
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        const float kv = kk[a] * vv[b];
-                        acc[b] = fmaf(rr[a], fmaf(ur[a], kv, s[a][b]), acc[b]);
-                        s[a][b] = fmaf(ww[a], s[a][b], kv);
-                    }
+                for (int t = 0; t < U; ++t) {
+                    const float rr[4] = {r4[t].x, r4[t].y, r4[t].z, r4[t].w}, kk[4] = {k4[t].x, k4[t].y, k4[t].z, k4[t].w};
+                    const float ww[4] = {w4[t].x, w4[t].y, w4[t].z, w4[t].w}, vv[2] = {v2[t].x, v2[t].y};
+                    acc[t][0] = acc[t][1] = 0.f;
+#pragma unroll
+                    for (int a = 0; a < WKV_GI; ++a)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            const float kv = kk[a] * vv[b];
+                            acc[t][b] = fmaf(rr[a], fmaf(ur[a], kv, s[a][b]), acc[t][b]);
+                            s[a][b] = fmaf(ww[a], s[a][b], kv);
+                        }
+                }
                 // groups g and g ^ 1: the even one goes on with the first column's sum, the odd one with the second's
-                const float sum = (odd ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, odd ? acc[0] : acc[1], 1);
-                mine[t * (WKV_CB * H)] = sum;
+                float sum[U];
+#pragma unroll
+                for (int t = 0; t < U; ++t) sum[t] = (odd ? acc[t][1] : acc[t][0]) + __shfl_xor_sync(0xffffffffu, odd ? acc[t][0] : acc[t][1], 1);
+#pragma unroll
+                for (int t = 0; t < U; ++t) mine[(t0 + t) * (WKV_CB * H)] = sum[t];
+            };
+            int t = 0;
+            if constexpr (U_ > 1) {
+#pragma unroll 2
+                for (; t + U_ <= nt; t += U_) walk(t, std::integral_constant<int, U_>());
             }
+#pragma unroll 4
+            for (; t < nt; ++t) walk(t, std::integral_constant<int, 1>());
         }
         __syncthreads();
     }
@@ -272,7 +300,7 @@ __global__ void __launch_bounds__(2 * NB + WKV_PRODUCERS) wkv_scan_kernel(const 
     if (head == 0 && blockIdx.z == 0) {        // the last row's h, for the token shift of the sequence's next token
         float* last = state + (int64_t)slot * state_stride + (int64_t)heads * N * N;
         const T* hr = h + (int64_t)(row1 - 1) * width;
-        for (int c = tid; c < width; c += NC + WKV_PRODUCERS) last[c] = to_f32(hr[c]);
+        for (int c = tid; c < width; c += NC + PRODUCERS) last[c] = to_f32(hr[c]);
     }
 }
 
@@ -477,17 +505,25 @@ static int wkv_scan_launch(const T* r, const T* k, const T* v, const float* z, c
                            float* state, int64_t state_stride, const int32_t* seq_first_row, const int32_t* seq_slot, int n_seqs,
                            int heads, int N, int width, int one_token, cudaStream_t stream) {
     const dim3 grid(n_seqs, heads);
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
 #define WKV_ARGS r, k, v, z, w0, u, h, o, state, state_stride, seq_first_row, seq_slot, heads, N, width
-#define WKV_SCAN(NB) x0ne_launch(wkv_scan_kernel<T, NB>, dim3(n_seqs, heads, NB / WKV_CB), dim3(2 * NB + WKV_PRODUCERS), 0, stream, WKV_ARGS)
+#define WKV_SCAN_AS(NB, P, U) x0ne_launch(wkv_scan_kernel<T, NB, P, U>, dim3(n_seqs, heads, NB / WKV_CB), dim3(2 * NB + P), 0, stream, WKV_ARGS)
+#define WKV_SCAN(NB)                                                                                     \
+    do {                                                                                                 \
+        if ((int64_t)n_seqs * heads * (NB / WKV_CB) <= sms) WKV_SCAN_AS(NB, WKV_WIDE_PRODUCERS, 4);      \
+        else WKV_SCAN_AS(NB, WKV_PRODUCERS, 1);                                                          \
+    } while (0)
 #define WKV_STEP(NB, GY) x0ne_launch(wkv_step_kernel<T, NB, GY>, grid, dim3(NB, GY), 0, stream, WKV_ARGS)
     if (N <= 32) { if (one_token) WKV_STEP(32, 4); else WKV_SCAN(32); }
     else if (N <= 64) { if (one_token) WKV_STEP(64, 8); else WKV_SCAN(64); }
-    else if (N <= 128) { if (one_token) WKV_STEP(128, 4); else WKV_SCAN(128); }
+    else if (N <= 128) { if (one_token) WKV_STEP(128, 4); else WKV_SCAN_AS(128, WKV_PRODUCERS, 1); }
     else {
         const int threads = N >= 256 ? 256 : (N + 31) / 32 * 32;
         x0ne_launch(wkv_scan_any_kernel<T>, grid, dim3(threads), (size_t)3 * N * sizeof(float), stream, WKV_ARGS);
     }
 #undef WKV_SCAN
+#undef WKV_SCAN_AS
 #undef WKV_STEP
 #undef WKV_ARGS
     X0NE_LAUNCH_CHECK();
