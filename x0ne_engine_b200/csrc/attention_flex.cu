@@ -205,7 +205,7 @@ __device__ __forceinline__ void fx_accumulate(float (*o)[4], const float (*p)[4]
 // ------------------------------------------------------------------------------------------------
 template <int DVT, bool SIG>
 __global__ void __launch_bounds__(256, DVT > 16 ? 1 : 2)
-flex_prefill_kernel(const bf16* __restrict__ q, bf16* __restrict__ out, PagedCache cache, const int32_t* __restrict__ tile_seq,
+flex_prefill_kernel(const bf16* q, bf16* __restrict__ out, PagedCache cache, const int32_t* __restrict__ tile_seq,
                     const int32_t* __restrict__ tile_row0, const int32_t* __restrict__ seq_first_row,
                     const int32_t* __restrict__ seq_slot, const int32_t* __restrict__ seq_pos0, int q_heads, float scale,
                     int window, AttnExtra ex, FxShape sh) {
@@ -410,9 +410,9 @@ flex_prefill_kernel(const bf16* __restrict__ q, bf16* __restrict__ out, PagedCac
 // (in the exp2 domain), the sum and vdp accumulated values: 16 x (vdp + 2) floats.
 template <int DVT>
 __global__ void __launch_bounds__(128)
-flex_decode_kernel(const bf16* __restrict__ q, bf16* __restrict__ out, PagedCache cache, const int32_t* __restrict__ row_slot,
+flex_decode_kernel(const bf16* q, bf16* __restrict__ out, PagedCache cache, const int32_t* __restrict__ row_slot,
                    const int32_t* __restrict__ row_pos, int q_heads, float scale, int window, AttnExtra ex, FxShape sh,
-                   int chunks, int splits, float* __restrict__ scratch) {
+                   int chunks, int splits, float* scratch) {
     extern __shared__ __align__(16) unsigned char fx_smem[];
     bf16* qs = reinterpret_cast<bf16*>(fx_smem);
     bf16* ks0 = qs + 16 * sh.ks;
@@ -614,7 +614,7 @@ flex_decode_kernel(const bf16* __restrict__ q, bf16* __restrict__ out, PagedCach
 // the threads share the (item, column) pairs and add the splits up in split order.
 #define FX_MAX_SPLITS 64
 __global__ void __launch_bounds__(256)
-flex_decode_merge_kernel(const float* __restrict__ scratch, bf16* __restrict__ out, int q_heads, int kv_heads,
+flex_decode_merge_kernel(const float* scratch, bf16* __restrict__ out, int q_heads, int kv_heads,
                          AttnExtra ex, int vd, int vdp, int chunks, int splits) {
     __shared__ float wgt[16][FX_MAX_SPLITS];
     __shared__ float fin_s[16];

@@ -28,7 +28,7 @@
 #define ATT_MAX_I 16  // value width <= 32 * ATT_MAX_I
 
 template <typename T>
-__global__ void attention_rows_kernel(const T* __restrict__ q, T* __restrict__ out, PagedCache cache,
+__global__ void attention_rows_kernel(const T* q, T* __restrict__ out, PagedCache cache,
                                       const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos,
                                       int n_rows, int q_heads, float scale, int window, AttnExtra ex) {
     extern __shared__ float smem[];

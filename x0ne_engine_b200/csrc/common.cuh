@@ -48,7 +48,14 @@ void x0ne_set_error(const char* fmt, ...);
 // their prologue early); `pdl_wait` then blocks until that kernel has finished and its writes
 // are visible.  A kernel calls `pdl_launch_dependents` at once, to let its own successor start
 // early in turn, and `pdl_wait` before it touches anything an earlier kernel may have written,
-// and before its own first write.  Only reads of weights may come before the wait.
+// and before its own first write.  Only reads of weights may come before the wait, and of the pass's
+// tables (rows, slots, positions, tiles, pages), which copies brought before the pass's first kernel.
+// What the wait orders has to look ordered to the compiler too.  Through a `const __restrict__` pointer
+// memory counts as unchanged for the whole kernel, so a read written behind the wait may be made ahead
+// of it; the same holds for reads through any `__restrict__` pointer, which nothing else can alias.  So
+// `__restrict__` stands on weights, on those tables and on results that the kernel only writes, never on
+// what an earlier kernel may have written (tests/test_kernel_sources.py has the list of names).  Where
+// that costs overlap because a store might alias a later load, the loads are written ahead of the stores.
 // Set X0NE_PDL=0 in the environment to launch everything fully serialized.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

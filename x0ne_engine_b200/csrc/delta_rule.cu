@@ -748,7 +748,7 @@ constexpr int dr_chunk_parts() { return 2 * DR_CHUNK_WARPS * 4 * 32 * 2; }
 // accumulators.  A chunk: the warps' shares of p and r meet in shared memory, every warp goes on with the sums, and adds the chunk's
 // writes to its own channels.  A warp without channels makes the results from the sums, another copies the inputs ahead.
 template <int NT>
-__global__ void __launch_bounds__(DR_CHUNK_WARPS * 32 + 64) delta_chunk_scan_kernel(DeltaArgs a, const float* __restrict__ coef, int* status) {
+__global__ void __launch_bounds__(DR_CHUNK_WARPS * 32 + 64) delta_chunk_scan_kernel(DeltaArgs a, const float* coef, int* status) {
     using Feed = DrChunkFeed<NT>;
     constexpr int C = DR_CHUNK, WARPS = DR_CHUNK_WARPS, ROW = dr_chunk_row<NT>(), COLS = DR_COLS, NS = DR_CHUNK_STAGES;
     static_assert(C == 8 && COLS == 16 && WARPS == 4, "a chunk is one tile of 8 tokens; four warps exchange their parts");

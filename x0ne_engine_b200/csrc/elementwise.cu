@@ -40,7 +40,7 @@ bool x0ne_pdl_enabled() {
 // parked in shared memory between the two sweeps when it fits there (`keep` floats of dynamic
 // shared memory, 0 if it does not), so the residual is read once.
 template <typename T>
-__global__ void add_rmsnorm_any_kernel(float* __restrict__ resid, const T* __restrict__ delta, const T* __restrict__ delta2,
+__global__ void add_rmsnorm_any_kernel(float* resid, const T* delta, const T* delta2,
                                        const float* __restrict__ w, T* __restrict__ out,
                                        const int32_t* __restrict__ rows, int hidden, float eps, int keep, int ld) {
     extern __shared__ float parked[];
@@ -122,7 +122,7 @@ __device__ __forceinline__ void copy2(bf16* d, const bf16* s) { *reinterpret_cas
 
 // ITS: how many sweeps of the block cover a row (1, 2 or VEC_IT).
 template <typename T, int ITS>
-__global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __restrict__ delta, const T* __restrict__ delta2,
+__global__ void add_rmsnorm_vec_kernel(float* resid, const T* delta, const T* delta2,
                                        const float* __restrict__ w, T* __restrict__ out,
                                        const int32_t* __restrict__ rows, int hidden, float eps, int ld) {
     __shared__ float sh[32];
@@ -166,10 +166,16 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __res
                 }
 #pragma unroll
                 for (int k = 0; k < 8; ++k) v[it][k] = v[it][k] + dv[k];
-                store8(r + i, v[it]);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) ss += v[it][k] * v[it][k];
+        }
+    }
+    if (d) {                // (behind all the loads: a store ahead of the next sweep's loads would hold them up)
+#pragma unroll
+        for (int it = 0; it < ITS; ++it) {
+            const int i = (it * blockDim.x + threadIdx.x) * 8;
+            if (i < hidden) store8(r + i, v[it]);
         }
     }
     const float total = block_sum(ss, sh);
@@ -252,7 +258,7 @@ X0NE_API int x0ne_add_rmsnorm(float* resid, const void* delta, const float* w, v
 // Same rows / block conventions as above; both sums of squares are fixed-order block sums.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void add_normed_rmsnorm_any_kernel(float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ bias_d,
+__global__ void add_normed_rmsnorm_any_kernel(float* resid, const T* delta, const float* __restrict__ bias_d,
                                               const float* __restrict__ w_d,
                                               float eps_d, const float* __restrict__ w, T* __restrict__ out,
                                               const int32_t* __restrict__ rows, int hidden, float eps, int keep) {
@@ -285,7 +291,7 @@ __global__ void add_normed_rmsnorm_any_kernel(float* __restrict__ resid, const T
 
 // hidden % 8 == 0 and hidden <= 8 * 1024 * 2: 16-byte accesses, the row and the delta stay in registers.
 template <typename T, int ITS>
-__global__ void __launch_bounds__(1024) add_normed_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ bias_d,
+__global__ void __launch_bounds__(1024) add_normed_rmsnorm_vec_kernel(float* resid, const T* delta, const float* __restrict__ bias_d,
                                               const float* __restrict__ w_d,
                                               float eps_d, const float* __restrict__ w, T* __restrict__ out,
                                               const int32_t* __restrict__ rows, int hidden, float eps) {
@@ -490,7 +496,7 @@ __device__ __forceinline__ void rope_one_head(const T* __restrict__ qkv, const f
 
 
 template <typename T>
-__global__ void qk_norm_rope_kv_write_kernel(const T* __restrict__ qkv, const float* __restrict__ norm_q,
+__global__ void qk_norm_rope_kv_write_kernel(const T* qkv, const float* __restrict__ norm_q,
                                              const float* __restrict__ norm_k,
                                              const float* __restrict__ inv_freq, int rot, T* __restrict__ q_out,
                                              PagedCache cache, const int32_t* __restrict__ row_slot,
@@ -528,7 +534,7 @@ __global__ void qk_norm_rope_kv_write_kernel(const T* __restrict__ qkv, const fl
 // row's position): head_dim / 16 lanes per head, each owning 8 consecutive values of the first half
 // and the 8 they pair with, moved 16 bytes at a time; a warp serves 512 / head_dim heads at once.
 template <typename T, int HD>
-__global__ void qk_norm_rope_kv_write_vec_kernel(const T* __restrict__ qkv, const float* __restrict__ norm_q,
+__global__ void qk_norm_rope_kv_write_vec_kernel(const T* qkv, const float* __restrict__ norm_q,
                                                  const float* __restrict__ norm_k, T* __restrict__ q_out,
                                                  PagedCache cache, const int32_t* __restrict__ row_slot,
                                                  const int32_t* __restrict__ row_pos, int n_rows, int q_heads, float eps,
@@ -577,8 +583,13 @@ __global__ void qk_norm_rope_kv_write_vec_kernel(const T* __restrict__ qkv, cons
     }
     pdl_wait();
     float a[8], b[8];
+    __align__(16) T va[8], vb[8];       // the v head that a k head's lanes copy along, asked for with the rest
     load8(src + c, a);
     load8(src + HALF + c, b);
+    if (!is_q && dst != nullptr) {
+        copy16(va, src + kv_dim + c);
+        copy16(vb, src + kv_dim + HALF + c);
+    }
     float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) ss += a[k] * a[k] + b[k] * b[k];
@@ -602,10 +613,9 @@ __global__ void qk_norm_rope_kv_write_vec_kernel(const T* __restrict__ qkv, cons
     store8(dst + c, ra);
     store8(dst + HALF + c, rb);
     if (!is_q) {
-        const T* vs = src + kv_dim;
         T* vd = dst + (int64_t)cache.kv_heads * cache.page_size * HD;
-        copy16(vd + c, vs + c);
-        copy16(vd + HALF + c, vs + HALF + c);
+        copy16(vd + c, va);
+        copy16(vd + HALF + c, vb);
     }
 }
 
@@ -675,7 +685,7 @@ X0NE_API int x0ne_qk_norm_rope_kv_write(const void* qkv, int dt, const float* no
 // float32) added first if it is given (x0ne-core/kernels/cuda/swiglu.cu:5-11).
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ gate_up, const float* __restrict__ bias, T* __restrict__ out, int inter) {
+__global__ void swiglu_kernel(const T* gate_up, const float* __restrict__ bias, T* __restrict__ out, int inter) {
     pdl_prologue();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
     if (i >= inter) return;
@@ -690,7 +700,7 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, const float* __rest
 
 // 8 values per thread with 16-byte accesses (inter % 8 == 0 and aligned rows).
 template <typename T>
-__global__ void swiglu_vec_kernel(const T* __restrict__ gate_up, const float* __restrict__ bias, T* __restrict__ out, int inter, int64_t total8) {
+__global__ void swiglu_vec_kernel(const T* gate_up, const float* __restrict__ bias, T* __restrict__ out, int inter, int64_t total8) {
     pdl_prologue();
     const int per_row = inter / 8;
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total8; e += (int64_t)gridDim.x * blockDim.x) {
@@ -827,7 +837,7 @@ X0NE_API int x0ne_embedding(const void* table, int dt, const int32_t* tokens, fl
 // embedding term (`table` null: not added) are optional; `step` is one vector of the pass.
 // ----------------------------------------------------------------------------------------
 template <typename T, typename E>
-__global__ void open_pass_kernel(float* __restrict__ resid, const T* __restrict__ delta, const E* __restrict__ table,
+__global__ void open_pass_kernel(float* resid, const T* delta, const E* __restrict__ table,
                                  const int32_t* __restrict__ tokens, float scale, const float* __restrict__ step, int hidden, int vocab) {
     pdl_prologue();
     const int row = blockIdx.x;
@@ -835,12 +845,21 @@ __global__ void open_pass_kernel(float* __restrict__ resid, const T* __restrict_
     const int t = table != nullptr ? tokens[row] : -1;
     const E* e = (table != nullptr && t >= 0 && t < vocab) ? table + (int64_t)t * hidden : nullptr;
     const T* d = delta != nullptr ? delta + (int64_t)row * hidden : nullptr;
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
-        float v = r[i];
-        if (d != nullptr) v = v + to_f32(d[i]);
-        if (e != nullptr) v = v + to_f32(e[i]) * scale;
-        if (step != nullptr) v = v + step[i];
-        r[i] = v;
+    constexpr int AT_ONCE = 4;          // (a store ahead of the next loads would hold them up)
+    for (int i0 = threadIdx.x; i0 < hidden; i0 += AT_ONCE * blockDim.x) {
+        float v[AT_ONCE];
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k) {
+            const int i = i0 + k * blockDim.x;
+            if (i >= hidden) continue;
+            v[k] = r[i];
+            if (d != nullptr) v[k] = v[k] + to_f32(d[i]);
+            if (e != nullptr) v[k] = v[k] + to_f32(e[i]) * scale;
+            if (step != nullptr) v[k] = v[k] + step[i];
+        }
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k)
+            if (i0 + k * blockDim.x < hidden) r[i0 + k * blockDim.x] = v[k];
     }
 }
 
@@ -968,8 +987,8 @@ X0NE_API int x0ne_embed_sum(EmbedSumArgs a, int dt, int n_rows, cudaStream_t str
 // One block per row; the sum of squares is a fixed-order block sum.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void concat_rows_kernel(const float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ bias_d,
-                                   const float* __restrict__ w_d, float eps_d, const float* __restrict__ x0, T* __restrict__ out, int hidden) {
+__global__ void concat_rows_kernel(const float* resid, const T* delta, const float* __restrict__ bias_d,
+                                   const float* __restrict__ w_d, float eps_d, const float* x0, T* __restrict__ out, int hidden) {
     __shared__ float sh[32];
     pdl_prologue();
     const int64_t row = blockIdx.x;

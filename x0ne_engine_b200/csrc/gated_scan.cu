@@ -509,7 +509,7 @@ __global__ void channel_gates_vec_kernel(GatedRaw x, float* __restrict__ out, in
 // Head gates: a block per (sequence, head).  All threads work out the gates of GS_GATE_TOKENS tokens, one thread walks the
 // running maximum through them (an addition and a maximum per token), all threads turn that into decays and write strengths.
 #define GS_GATE_TOKENS 1024
-__global__ void __launch_bounds__(256) head_gates_kernel(GatedRaw x, float* __restrict__ gates, float* __restrict__ state, int64_t state_stride,
+__global__ void __launch_bounds__(256) head_gates_kernel(GatedRaw x, float* __restrict__ gates, float* state, int64_t state_stride,
                                                          const int32_t* __restrict__ seq_first_row, const int32_t* __restrict__ seq_slot, int heads) {
     __shared__ __align__(16) float is[GS_GATE_TOKENS + 8], fs[GS_GATE_TOKENS + 8], ms[GS_GATE_TOKENS];     // ms: the maximum before a token
     pdl_launch_dependents();

@@ -51,7 +51,7 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 // the tiles (16 weight rows each) blockIdx.x, blockIdx.x + gridDim.x, ...; the copies run ahead
 // across the tile boundary, so the stream does not drain while a tile's partial sums are reduced.
 template <int MT, typename OutT, bool SWIGLU, int DEPTH>
-__global__ void __launch_bounds__(SM_WARPS * 32) gemm_smallm_kernel(const bf16* __restrict__ W, const bf16* __restrict__ X,
+__global__ void __launch_bounds__(SM_WARPS * 32) gemm_smallm_kernel(const bf16* __restrict__ W, const bf16* X,
                                                                     OutT* __restrict__ Y, int M, int N, int K, int ldy,
                                                                     int n_tiles, GluParams glu) {
     constexpr int SETS = SWIGLU ? 2 : 1;

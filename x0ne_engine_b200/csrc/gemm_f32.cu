@@ -17,7 +17,7 @@
 #define TM 8
 #define TN 4
 
-__global__ void __launch_bounds__(256) gemm_f32_nt_kernel(const float* __restrict__ A, const float* __restrict__ W,
+__global__ void __launch_bounds__(256) gemm_f32_nt_kernel(const float* A, const float* W,
                                                            float* __restrict__ C, int M, int N, int K, int lda,
                                                            int ldw, int ldc, int64_t sa, int64_t sw, int64_t sc) {
     __shared__ float As[BK][BM + 4];

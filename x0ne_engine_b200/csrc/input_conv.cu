@@ -66,7 +66,7 @@ template <> struct IcRaw<bf16> {
 
 // Any width and number of taps: a thread per channel; every input is read where it lies.
 template <typename T>
-__global__ void input_conv_any_kernel(const T* __restrict__ h, const float* __restrict__ w, float* __restrict__ state, int64_t state_stride,
+__global__ void input_conv_any_kernel(const T* h, const float* __restrict__ w, float* state, int64_t state_stride,
                                       int64_t off, T* __restrict__ out, const int32_t* __restrict__ seq_first_row,
                                       const int32_t* __restrict__ seq_slot, int width, int taps) {
     pdl_prologue();
@@ -94,7 +94,7 @@ __global__ void input_conv_any_kernel(const T* __restrict__ h, const float* __re
 
 // TAPS at compile time, 8 channels per thread; a stretch's rows are all asked for before the first is used.
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) input_conv_vec_kernel(const T* __restrict__ h, const float* __restrict__ w, float* __restrict__ state,
+__global__ void __launch_bounds__(128) input_conv_vec_kernel(const T* h, const float* __restrict__ w, float* state,
                                                              int64_t state_stride, int64_t off, T* __restrict__ out,
                                                              const int32_t* __restrict__ seq_first_row, const int32_t* __restrict__ seq_slot,
                                                              int width) {
@@ -145,11 +145,11 @@ __global__ void __launch_bounds__(128) input_conv_vec_kernel(const T* __restrict
 #pragma unroll
         for (int i = 0; i < KEPT; ++i) {
             const int at = n_tok - KEPT + i;
-            float v[8];
-            if (at >= 0) ic_load8(src + (int64_t)at * width, v);
-            else ic_load8(st + (int64_t)(at + KEPT) * width, v);
-            ic_store8(st + (int64_t)i * width, v);
+            if (at >= 0) ic_load8(src + (int64_t)at * width, win[i]);
+            else ic_load8(st + (int64_t)(at + KEPT) * width, win[i]);
         }
+#pragma unroll
+        for (int i = 0; i < KEPT; ++i) ic_store8(st + (int64_t)i * width, win[i]);
     }
 }
 

@@ -10,7 +10,7 @@
 //   g = min(gate, limit); u = clamp(up, -limit, limit); out = g * sigmoid(slope * g) * (u + shift)
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void glu_clipped_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int inter, int64_t total, float limit,
+__global__ void glu_clipped_kernel(const T* gate_up, T* __restrict__ out, int inter, int64_t total, float limit,
                                    float slope, float shift) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -24,7 +24,7 @@ __global__ void glu_clipped_kernel(const T* __restrict__ gate_up, T* __restrict_
 
 // 8 values per thread with 16-byte accesses (inter % 8 == 0 and aligned rows).
 template <typename T>
-__global__ void glu_clipped_vec_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int inter, int64_t total8, float limit,
+__global__ void glu_clipped_vec_kernel(const T* gate_up, T* __restrict__ out, int inter, int64_t total8, float limit,
                                        float slope, float shift) {
     pdl_prologue();
     const int per_row = inter / 8;
@@ -125,7 +125,7 @@ __device__ __forceinline__ void store8f(float* p, const float* v) {
 // into the cache.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void kv_write_blend_kernel(const T* __restrict__ src, int ld, int k_col, int v_col, T* __restrict__ v_first,
+__global__ void kv_write_blend_kernel(const T* src, int ld, int k_col, int v_col, T* v_first,
                                       const float* __restrict__ lambda, int mode, PagedCache cache,
                                       const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int vec) {
     pdl_launch_dependents();
@@ -210,7 +210,7 @@ X0NE_API int x0ne_kv_write_blend(const void* src, int dt, int ld, int k_col, int
 // computation for the positions it covers.  One block per row.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void latent_prepare_kernel(const T* __restrict__ src, int ld, int dkv_col, const T* __restrict__ q_abs,
+__global__ void latent_prepare_kernel(const T* src, int ld, int dkv_col, const T* q_abs,
                                       int64_t q_abs_head_stride, const float* __restrict__ norm_w, float eps,
                                       const float* __restrict__ freq, float mag, const float* __restrict__ table,
                                       int table_positions, T* __restrict__ q_out, int heads, int dim, int rot, int rank,
@@ -307,7 +307,7 @@ X0NE_API int x0ne_latent_prepare(const void* src, int dt, int ld, int dkv_col, c
 // positions it covers.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void whole_norm_rope_kv_write_kernel(const T* __restrict__ src, int ld, int k_col, int v_col,
+__global__ void whole_norm_rope_kv_write_kernel(const T* src, int ld, int k_col, int v_col,
                                                 const float* __restrict__ norm_q, const float* __restrict__ norm_k, float eps,
                                                 const float* __restrict__ freq, int rot, const float* __restrict__ table,
                                                 int table_positions, T* __restrict__ q_out, int q_heads, PagedCache cache,
@@ -410,7 +410,7 @@ __device__ __forceinline__ void wn_rotated_piece(const T* __restrict__ s, const 
 #define WN_MAX_PIECES 4
 template <typename T, bool STAGE>
 __global__ void __launch_bounds__(256) whole_norm_rope_kv_write_vec_kernel(
-    const T* __restrict__ src, int ld, int k_col, int v_col, const float* __restrict__ norm_q, const float* __restrict__ norm_k,
+    const T* src, int ld, int k_col, int v_col, const float* __restrict__ norm_q, const float* __restrict__ norm_k,
     float eps, const float* __restrict__ freq, int rot, const float* __restrict__ table, int table_positions, T* __restrict__ q_out,
     int q_heads, PagedCache cache, const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int write_kv) {
     extern __shared__ float cs[];
@@ -587,7 +587,7 @@ X0NE_API int x0ne_whole_norm_rope_kv_write(const void* src, int dt, int ld, int 
 // Squared ReLU in place or out of place: out = max(x, 0)^2, float32 arithmetic.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void relu2_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t total) {
+__global__ void relu2_kernel(const T* x, T* __restrict__ out, int64_t total) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const float v = fmaxf(to_f32(x[i]), 0.f);
@@ -595,7 +595,7 @@ __global__ void relu2_kernel(const T* __restrict__ x, T* __restrict__ out, int64
     }
 }
 template <typename T>
-__global__ void relu2_vec_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t total8) {
+__global__ void relu2_vec_kernel(const T* x, T* __restrict__ out, int64_t total8) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total8; i += (int64_t)gridDim.x * blockDim.x) {
         float v[8];
@@ -636,7 +636,7 @@ X0NE_API int x0ne_relu2(const void* x, void* out, int dt, int64_t total, cudaStr
 // sums of squares, the logarithm and the products are float32.  Rows without a page write no keys or values.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void head_norm_kv_write_kernel(const T* __restrict__ src, int ld, int k_col, int v_col, const float* __restrict__ norm_q,
+__global__ void head_norm_kv_write_kernel(const T* src, int ld, int k_col, int v_col, const float* __restrict__ norm_q,
                                           const float* __restrict__ norm_k, float eps, float temp_coef, int temp_every, int v_unit,
                                           T* __restrict__ q_out, int q_heads, PagedCache cache, const int32_t* __restrict__ row_slot,
                                           const int32_t* __restrict__ row_pos, int n_rows) {
@@ -681,11 +681,20 @@ __global__ void head_norm_kv_write_kernel(const T* __restrict__ src, int ld, int
         ss = warp_sum(ss);
         scale = 1.0f / sqrtf(ss / (float)n + eps);
     }
-    for (int i = lane; i < n; i += 32) {
-        float v = to_f32(x[i]) * scale;
-        if (w != nullptr) v *= w[i];
-        if (normed && mul != 1.f) v *= mul;
-        dst[i] = from_f32<T>(v);
+    constexpr int AT_ONCE = 4;          // (a store ahead of the next loads would hold them up)
+    for (int i0 = lane; i0 < n; i0 += 32 * AT_ONCE) {
+        float v[AT_ONCE];
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k) {
+            const int i = i0 + 32 * k;
+            if (i >= n) continue;
+            v[k] = to_f32(x[i]) * scale;
+            if (w != nullptr) v[k] *= w[i];
+            if (normed && mul != 1.f) v[k] *= mul;
+        }
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k)
+            if (i0 + 32 * k < n) dst[i0 + 32 * k] = from_f32<T>(v[k]);
     }
 }
 
@@ -720,7 +729,7 @@ X0NE_API int x0ne_head_norm_kv_write(const void* src, int dt, int ld, int k_col,
 //          z > 0: a z^2 + z / 2;  z <= 0: b (exp(z) - 1 - z) + z / 2      (a, b >= 0 given by the caller)
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void bias_act_kernel(const T* __restrict__ x, const float* __restrict__ bias, T* __restrict__ out, int width, int64_t total,
+__global__ void bias_act_kernel(const T* x, const float* __restrict__ bias, T* __restrict__ out, int width, int64_t total,
                                 int act, float a, float b) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -733,7 +742,7 @@ __global__ void bias_act_kernel(const T* __restrict__ x, const float* __restrict
 
 // the same with 8 values per thread: `width` a multiple of 8 and 16-byte aligned rows
 template <typename T>
-__global__ void bias_act_vec_kernel(const T* __restrict__ x, const float* __restrict__ bias, T* __restrict__ out, int width, int n_rows,
+__global__ void bias_act_vec_kernel(const T* x, const float* __restrict__ bias, T* __restrict__ out, int width, int n_rows,
                                     int act, float a, float b) {
     pdl_launch_dependents();
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -786,7 +795,7 @@ X0NE_API int x0ne_bias_act(const void* x, const float* bias, void* out, int dt, 
 // write no keys or values.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void rope_pairs_kv_write_kernel(const T* __restrict__ src, const float* __restrict__ bias, int ld, int k_col, int v_col, const float* __restrict__ freq,
+__global__ void rope_pairs_kv_write_kernel(const T* src, const float* __restrict__ bias, int ld, int k_col, int v_col, const float* __restrict__ freq,
                                            const float* __restrict__ table, int table_positions, int rot, int maps, int dim, float mag,
                                            float unit_eps, T* __restrict__ q_out, int q_heads, int q_padded, PagedCache cache,
                                            const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int n_rows,
@@ -870,7 +879,7 @@ __global__ void rope_pairs_kv_write_kernel(const T* __restrict__ src, const floa
 // The same for one map per head without unit norm, 8 values per thread: dim, rot, the value width, the row pitch and the
 // columns are multiples of 8.  A block takes 8 x blockDim.x values of a row.
 template <typename T>
-__global__ void __launch_bounds__(128) rope_pairs_kv_write_vec_kernel(const T* __restrict__ src, const float* __restrict__ bias, int ld, int k_col, int v_col,
+__global__ void __launch_bounds__(128) rope_pairs_kv_write_vec_kernel(const T* src, const float* __restrict__ bias, int ld, int k_col, int v_col,
                                                                       const float* __restrict__ freq, const float* __restrict__ table, int table_positions,
                                                                       int rot, int dim, float mag, T* __restrict__ q_out, int q_heads, PagedCache cache,
                                                                       const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int write_kv) {
@@ -976,7 +985,7 @@ X0NE_API int x0ne_rope_pairs_kv_write(const void* src, const float* bias, int dt
 // (gate null: no gate).  One warp per (row, head); the difference, the norm and the gate are float32.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void diff_heads_kernel(const float* __restrict__ att, const T* __restrict__ gate, int64_t gate_ld, T* __restrict__ out, int n_rows,
+__global__ void diff_heads_kernel(const float* att, const T* gate, int64_t gate_ld, T* __restrict__ out, int n_rows,
                                   int heads, int vd, float lambda, float eps, float post) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
@@ -1299,7 +1308,7 @@ X0NE_API int x0ne_latent_rows(LatentRowsArgs a, void* cq_out, int dt, PagedCache
 
 // q: [rows][q_ld], head h at column h * (dim + rot); q_abs: [heads][head_stride] of rows of `rank` values.
 template <typename T, int PIECE>
-__global__ void __launch_bounds__(128) latent_queries_kernel(const T* __restrict__ q, int64_t q_ld, const T* __restrict__ q_abs, int64_t head_stride, LatentTurn turn,
+__global__ void __launch_bounds__(128) latent_queries_kernel(const T* q, int64_t q_ld, const T* q_abs, int64_t head_stride, LatentTurn turn,
                                                              const int32_t* __restrict__ row_pos, T* __restrict__ q_out, int heads, int dim, int rank) {
     pdl_launch_dependents();
     const int row = blockIdx.x, pos = row_pos[row], half = turn.rot / 2, per_head = rank / PIECE, qw = rank + turn.rot;
@@ -1349,7 +1358,7 @@ X0NE_API int x0ne_latent_queries(const void* q, int64_t q_ld, const void* q_abs,
 // head_stride values apart (what a product per head leaves).
 // ----------------------------------------------------------------------------------------
 template <typename T, int PIECE>
-__global__ void __launch_bounds__(128) heads_gate_kernel(const T* __restrict__ x, int64_t head_stride, const T* __restrict__ gate, int64_t gate_ld, T* __restrict__ out,
+__global__ void __launch_bounds__(128) heads_gate_kernel(const T* x, int64_t head_stride, const T* gate, int64_t gate_ld, T* __restrict__ out,
                                                          int heads, int V) {
     pdl_prologue();
     const int row = blockIdx.x, i = (blockIdx.y * blockDim.x + threadIdx.x) * PIECE;
@@ -1518,7 +1527,7 @@ X0NE_API int x0ne_head_products(HeadProductArgs a, cudaStream_t stream) {
 // ----------------------------------------------------------------------------------------
 // x = cap tanh(x / cap) in place, float32.
 // ----------------------------------------------------------------------------------------
-__global__ void soft_cap_kernel(float* __restrict__ x, int64_t total, float cap) {
+__global__ void soft_cap_kernel(float* x, int64_t total, float cap) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) x[i] = soft_capped(x[i], cap);
 }

@@ -31,7 +31,7 @@
 // Router: one warp per row.  z [rows][ldz] float32 (the router's n outputs first; the shared
 // expert's gate logit at column sg_col when sgate is given).
 // ----------------------------------------------------------------------------------------
-__global__ void moe_route_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ correction, int n, int groups,
+__global__ void moe_route_kernel(const float* z, int ldz, const float* __restrict__ correction, int n, int groups,
                                  int keep, int top, int n_rows, int32_t* __restrict__ chosen, float* __restrict__ weights,
                                  float* __restrict__ sgate, int sg_col, int mode, int group_top, int normalize, float weight_scale) {
     extern __shared__ float rt_smem[];
@@ -168,9 +168,9 @@ __global__ void moe_route_kernel(const float* __restrict__ z, int ldz, const flo
 //   n_tiles_out             how many tiles exist (optional)
 // ----------------------------------------------------------------------------------------
 #define GP_OWN 8        // choices of a thread that stay in registers
-__global__ void moe_group_kernel(const int32_t* __restrict__ chosen, int pairs, int experts, int32_t* __restrict__ offsets,
-                                 int32_t* __restrict__ listed, int32_t* __restrict__ tiles, int max_tiles, int tile_m,
-                                 int32_t* __restrict__ n_tiles_out) {
+__global__ void moe_group_kernel(const int32_t* chosen, int pairs, int experts, int32_t* offsets,
+                                 int32_t* listed, int32_t* tiles, int max_tiles, int tile_m,
+                                 int32_t* n_tiles_out) {
     extern __shared__ int gp_smem[];
     int* count = gp_smem;                 // [experts]
     int* start = count + experts;         // [experts + 1]
@@ -238,8 +238,8 @@ __global__ void moe_group_kernel(const int32_t* __restrict__ chosen, int pairs, 
 // Tile 32 pairs x 64 outputs x 16 k, 256 threads, 2 x 4 outputs per thread.
 // ----------------------------------------------------------------------------------------
 template <typename T, int ACT>
-__global__ void __launch_bounds__(256) moe_product_kernel(const T* __restrict__ a, int64_t lda, const T* __restrict__ w, int N, int K,
-                                                          const int32_t* __restrict__ listed, const int32_t* __restrict__ tiles,
+__global__ void __launch_bounds__(256) moe_product_kernel(const T* a, int64_t lda, const T* __restrict__ w, int N, int K,
+                                                          const int32_t* listed, const int32_t* tiles,
                                                           int top, void* __restrict__ out, int pair_block) {
     __shared__ float As[16][MOE_TILE_M + 4];
     __shared__ float Ws[16][64 + 4];
@@ -328,9 +328,9 @@ __global__ void __launch_bounds__(256) moe_product_kernel(const T* __restrict__ 
 //                          + sgate[row] * shared[row], in float32, choices in order.  One block per row.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void moe_combine_kernel(const float* __restrict__ y, const T* __restrict__ x, const int32_t* __restrict__ chosen,
-                                   const float* __restrict__ weights, int top, int experts, const T* __restrict__ shared,
-                                   const float* __restrict__ sgate, T* __restrict__ out, int hidden) {
+__global__ void moe_combine_kernel(const float* y, const T* x, const int32_t* chosen,
+                                   const float* weights, int top, int experts, const T* shared,
+                                   const float* sgate, T* __restrict__ out, int hidden) {
     pdl_prologue();
     const int row = blockIdx.x;
     const int32_t* ch = chosen + (int64_t)row * top;

@@ -43,8 +43,8 @@ struct MtShared {
 template <int MODE>
 __global__ void __launch_bounds__(MT_THREADS) moe_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                             const __grid_constant__ CUtensorMap map_w, void* __restrict__ out,
-                                                            int N, int K, const int32_t* __restrict__ listed,
-                                                            const int32_t* __restrict__ tiles, const int32_t* __restrict__ n_real_p,
+                                                            int N, int K, const int32_t* listed,
+                                                            const int32_t* tiles, const int32_t* n_real_p,
                                                             int max_tiles, int n_tiles_n, int* status) {
     extern __shared__ unsigned char mt_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(mt_raw) + 1023) & ~(uintptr_t)1023);
@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(MT_THREADS) moe_tc_kernel(const __grid_constan
 }
 
 // xs[place] = x[listed[place] / top] for the places that hold a pair (their number is offsets[experts]).
-__global__ void moe_gather_rows_kernel(const bf16* __restrict__ x, int K, const int32_t* __restrict__ listed,
-                                       const int32_t* __restrict__ offsets, int experts, int top, bf16* __restrict__ xs) {
+__global__ void moe_gather_rows_kernel(const bf16* x, int K, const int32_t* listed,
+                                       const int32_t* offsets, int experts, int top, bf16* __restrict__ xs) {
     pdl_prologue();
     const int place = blockIdx.x;
     if (place >= offsets[experts]) return;

@@ -59,8 +59,8 @@ __device__ __forceinline__ float ssm_softplus(float v) { return v > 20.f ? v : l
 // The state is only read here: the scan, which runs later in the stream, leaves the new last inputs.
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void causal_conv_silu_kernel(const T* __restrict__ x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias,
-                                        const float* __restrict__ state, int64_t state_stride, int64_t conv_off, T* __restrict__ out,
+__global__ void causal_conv_silu_kernel(const T* x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias,
+                                        const float* state, int64_t state_stride, int64_t conv_off, T* __restrict__ out,
                                         const int32_t* __restrict__ row_slot, const int32_t* __restrict__ row_pos, int n_rows,
                                         int channels, int taps) {
     pdl_launch_dependents();
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
 #pragma unroll
             for (int k = 0; k < SSM_CONV_TAPS; ++k) wk[k][i] = k < taps ? w[(int64_t)(c + i) * taps + taps - 1 - k] : 0.f;
     }
-    pdl_wait();             // (x and the state are not __restrict__: reads that nothing may alias could be moved ahead of the wait)
+    pdl_wait();
     // rows first - BEFORE .. first + RUN - 1, as they are stored
     Raw8<T> raw[BEFORE + SSM_CONV_RUN];
 #pragma unroll
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
 
 template <typename T>
 __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(
-        const T* __restrict__ x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ state,
+        const T* x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias, const float* state,
         int64_t state_stride, int64_t conv_off, T* __restrict__ out, const int32_t* __restrict__ row_slot,
         const int32_t* __restrict__ row_pos, int n_rows, int channels, int taps, int rows_per_block) {
     // the taps of this block's 128 x 8 channels, laid out [tap][channel of the thread's eight][thread]: a warp's reads of

@@ -23,8 +23,8 @@
 // token shift
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void token_shift_mix_kernel(const T* __restrict__ h, const float* __restrict__ mu, int n_mix, T* __restrict__ mixes,
-                                       int64_t mix_stride, const float* __restrict__ state, int64_t state_stride,
+__global__ void token_shift_mix_kernel(const T* h, const float* __restrict__ mu, int n_mix, T* __restrict__ mixes,
+                                       int64_t mix_stride, const float* state, int64_t state_stride,
                                        int64_t last_off, const int32_t* __restrict__ row_slot,
                                        const int32_t* __restrict__ row_pos, int n_rows, int width) {
     pdl_prologue();
@@ -73,8 +73,8 @@ __device__ __forceinline__ void wkv_store8(float* p, const float* v) {
 // The token shift with 8 values per thread (width, strides and offsets multiples of 8, 16-byte aligned bases):
 // block (row, 8 x blockDim.x columns).
 template <typename T>
-__global__ void token_shift_mix_vec_kernel(const T* __restrict__ h, const float* __restrict__ mu, int n_mix, T* __restrict__ mixes,
-                                           int64_t mix_stride, const float* __restrict__ state, int64_t state_stride,
+__global__ void token_shift_mix_vec_kernel(const T* h, const float* __restrict__ mu, int n_mix, T* __restrict__ mixes,
+                                           int64_t mix_stride, const float* state, int64_t state_stride,
                                            int64_t last_off, const int32_t* __restrict__ row_slot,
                                            const int32_t* __restrict__ row_pos, int n_rows, int width) {
     pdl_prologue();
@@ -133,10 +133,10 @@ __device__ __forceinline__ float wkv_tree_sum(float (&q)[G]) {
 }
 
 template <typename T, int NB, int PRODUCERS, int U_>
-__global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
-                                                                         const float* __restrict__ z, const float* __restrict__ w0,
-                                                                         const float* __restrict__ u, const T* __restrict__ h,
-                                                                         float* __restrict__ o, float* __restrict__ state, int64_t state_stride,
+__global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* r, const T* k, const T* v,
+                                                                         const float* z, const float* __restrict__ w0,
+                                                                         const float* __restrict__ u, const T* h,
+                                                                         float* __restrict__ o, float* state, int64_t state_stride,
                                                                          const int32_t* __restrict__ seq_first_row, const int32_t* __restrict__ seq_slot,
                                                                          int heads, int N, int width) {
     constexpr int G = NB / WKV_GI;                  // groups of key channels = working threads that share a column
@@ -307,10 +307,10 @@ __global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* _
 // One token per sequence (more are worked through one after the other): block (NB, GY); thread (j, y) takes the groups
 // y, y + GY, ... of column j.
 template <typename T, int NB, int GY>
-__global__ void __launch_bounds__(NB * GY) wkv_step_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
-                                                          const float* __restrict__ z, const float* __restrict__ w0,
-                                                          const float* __restrict__ u, const T* __restrict__ h,
-                                                          float* __restrict__ o, float* __restrict__ state, int64_t state_stride,
+__global__ void __launch_bounds__(NB * GY) wkv_step_kernel(const T* r, const T* k, const T* v,
+                                                          const float* z, const float* __restrict__ w0,
+                                                          const float* __restrict__ u, const T* h,
+                                                          float* __restrict__ o, float* state, int64_t state_stride,
                                                           const int32_t* __restrict__ seq_first_row, const int32_t* __restrict__ seq_slot,
                                                           int heads, int N, int width) {
     constexpr int G = NB / WKV_GI;
@@ -380,9 +380,9 @@ __global__ void __launch_bounds__(NB * GY) wkv_step_kernel(const T* __restrict__
 
 // Any N: the state stays in global memory (read and written per token); thread j owns column j.
 template <typename T>
-__global__ void wkv_scan_any_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
-                                    const float* __restrict__ z, const float* __restrict__ w0, const float* __restrict__ u,
-                                    const T* __restrict__ h, float* __restrict__ o, float* __restrict__ state, int64_t state_stride,
+__global__ void wkv_scan_any_kernel(const T* r, const T* k, const T* v,
+                                    const float* z, const float* __restrict__ w0, const float* __restrict__ u,
+                                    const T* h, float* __restrict__ o, float* state, int64_t state_stride,
                                     const int32_t* __restrict__ seq_first_row, const int32_t* __restrict__ seq_slot, int heads,
                                     int N, int width) {
     extern __shared__ float wk_smem[];       // r, k, w of the token: 3 N
@@ -427,7 +427,7 @@ __global__ void wkv_scan_any_kernel(const T* __restrict__ r, const T* __restrict
 // head norm, weight and gate: one warp per (row, head)
 // ----------------------------------------------------------------------------------------
 template <typename T>
-__global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* __restrict__ weight, const T* __restrict__ gate,
+__global__ void head_norm_gate_kernel(const float* o, const float* __restrict__ weight, const T* gate,
                                       T* __restrict__ out, int n_rows, int heads, int N, float eps) {
     pdl_prologue();
     const int lane = threadIdx.x & 31;
@@ -447,7 +447,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
 
 // The same with 8 values per lane: LANES = N / 8 lanes (a power of two up to 32) work on one (row, head).
 template <typename T, int LANES>
-__global__ void head_norm_gate_vec_kernel(const float* __restrict__ o, const float* __restrict__ weight, const T* __restrict__ gate,
+__global__ void head_norm_gate_vec_kernel(const float* o, const float* __restrict__ weight, const T* gate,
                                           T* __restrict__ out, int64_t items, int heads, float eps) {
     pdl_prologue();
     constexpr int N = LANES * 8;
@@ -582,7 +582,7 @@ X0NE_API int x0ne_head_norm_gate(const float* o, const float* weight, const void
 
 // out = tanh(x): float32 in, the activation type out (the inner activation of the decay's two small products)
 template <typename T>
-__global__ void tanh_rows_kernel(const float* __restrict__ x, T* __restrict__ out, int64_t total) {
+__global__ void tanh_rows_kernel(const float* x, T* __restrict__ out, int64_t total) {
     pdl_prologue();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = from_f32<T>(tanhf(x[i]));
