@@ -65,3 +65,14 @@ def test_the_check_sees_breaches():
     assert breaches(src % "k") == ["k: const float* __restrict__ x"]
     assert breaches((src % "k").replace("pdl_prologue();", "")) == []
     assert breaches("__global__ void k(float* __restrict__ resid) { pdl_wait(); float v = resid[0]; }") == ["k: float* __restrict__ resid"]
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*tcgen05.cu"))), ids=os.path.basename)
+def test_kernels_let_their_successors_start_only_with_their_tensor_memory_in_hand(path):
+    """A block that waits for tensor memory which a block of its successor holds, while that one waits for it, waits for good."""
+    with open(path) as f:
+        own = [(name, body) for name, _, body in kernels(f.read()) if "tcgen05.alloc" in body]
+    assert own
+    for name, body in own:
+        assert re.search(r"tcgen05\.alloc.*__syncthreads\(\);.*pdl_launch_dependents\(\);", body, re.S), name
+        assert "pdl_launch_dependents" not in body[:body.index("tcgen05.alloc")], name

@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(FT_THREADS, 2) flex_prefill_tc_kernel(const __
     const int n_walk = slot < 0 || n_rows <= 0 ? 0 : n_kept + pg_last - pg_first + 1;
     auto page_at = [&](int i) { return i < n_kept ? i : pg_first + i - n_kept; };
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         mbar_init(&sh->q_full, 1);
         for (int b = 0; b < 2; ++b) {
@@ -141,6 +140,7 @@ __global__ void __launch_bounds__(FT_THREADS, 2) flex_prefill_tc_kernel(const __
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem_s = sh->tmem_base, tmem_o = tmem_s + 128;       // S / P: two buffers of 64 columns; O: 64 nbv columns
     bool ok = !sh->failed;

@@ -131,7 +131,6 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attention_prefill_tc_kernel(co
     const int j_lo = a.window > 0 ? max(0, pos_first - a.window + 1) : 0;
     const int kt_lo = j_lo / 64, n_kt = pos_last / 64 - kt_lo + 1;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         mbar_init(&sh->q_full, 1);
         for (int b = 0; b < 2; ++b) {
@@ -155,6 +154,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 2) attention_prefill_tc_kernel(co
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
     const uint32_t tmem_s = tmem, tmem_o = tmem + 128;       // S: two buffers of 64 columns; O: HD columns

@@ -47,7 +47,8 @@ void x0ne_set_error(const char* fmt, ...);
 // while the kernel before it in the stream is still running (its blocks are scheduled and run
 // their prologue early); `pdl_wait` then blocks until that kernel has finished and its writes
 // are visible.  A kernel calls `pdl_launch_dependents` at once, to let its own successor start
-// early in turn, and `pdl_wait` before it touches anything an earlier kernel may have written,
+// early in turn (one that takes tensor memory: once it has it, or a successor's block could take the
+// columns it is still waiting for and then wait for it), and `pdl_wait` before it touches anything an earlier kernel may have written,
 // and before its own first write.  Only reads of weights may come before the wait, and of the pass's
 // tables (rows, slots, positions, tiles, pages), which copies brought before the pass's first kernel.
 // What the wait orders has to look ordered to the compiler too.  Through a `const __restrict__` pointer

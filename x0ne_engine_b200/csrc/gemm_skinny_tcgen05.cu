@@ -78,7 +78,6 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_tc_kernel(const __g
     const int kb_lo = (int)(((int64_t)k_blocks * slice) / slices), kb_hi = (int)(((int64_t)k_blocks * (slice + 1)) / slices);
     const int n_kb = kb_hi - kb_lo;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < SK_STAGES; ++s) {
             mbar_init(&sh->full[s], 1);
@@ -96,6 +95,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2) gemm_skinny_tc_kernel(const __g
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
 

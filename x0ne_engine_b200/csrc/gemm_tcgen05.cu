@@ -80,7 +80,6 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
     const int tiles = m_tiles * n_tiles;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC_STAGES; ++s) {
             mbar_init(&sh->full[s], 1);
@@ -101,6 +100,7 @@ __global__ void __launch_bounds__(TC_THREADS) gemm_tc_kernel(const __grid_consta
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
 
@@ -305,7 +305,6 @@ __global__ void __launch_bounds__(TC2_THREADS) gemm_tc_pair_kernel(const __grid_
     const int k_blocks = (K + TC_BK - 1) / TC_BK;
     const int tiles = m_tiles * n_tiles;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC2_STAGES; ++s) {
             mbar_init(&sh->full[s], 1);
@@ -326,6 +325,7 @@ __global__ void __launch_bounds__(TC2_THREADS) gemm_tc_pair_kernel(const __grid_
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     cluster_sync();          // both blocks' barriers are initialised before either block uses the other's
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;

@@ -53,7 +53,6 @@ __global__ void __launch_bounds__(MT_THREADS) moe_tc_kernel(const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k_blocks = (K + MT_BK - 1) / MT_BK;
 
-    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < MT_STAGES; ++s) {
             mbar_init(&sh->full[s], 1);
@@ -74,6 +73,7 @@ __global__ void __launch_bounds__(MT_THREADS) moe_tc_kernel(const __grid_constan
     }
     tc_fence_before();
     __syncthreads();
+    pdl_launch_dependents();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
     pdl_wait();          // the table of tiles, the list and the A rows were written by the kernels before this one
