@@ -9,13 +9,15 @@ FORMS = [
     (128, 128, 0, 0, 0, 0, ""), (64, 64, 0, 70, 0, 0, "sink"), (8, 8, 0, 0, 0, 0, "slope"), (96, 40, 0, 0, 100, 0, "gate"),
     (128, 256, 0, 150, 0, 67, "wide f32"), (72, 200, 0, 0, 64, 0, "sink f32 inside"), (320, 0, 256, 90, 0, 0, "sink gate"), (160, 0, 128, 0, 0, 3, "wide"),
     (128, 64, 0, 0, 130, 0, "sig inside"), (64, 136, 0, 0, 0, 0, "slope late"), (128, 128, 0, 0, 0, 0, "late inside"), (24, 16, 0, 1, 0, 0, "sig"),
+    (128, 128, 0, 0, 0, 0, "gone"), (64, 64, 0, 70, 0, 67, "gone sink"), (320, 0, 256, 0, 0, 0, "gone gate"), (128, 64, 0, 0, 130, 0, "gone sig"),
 ]
 
 
 @pytest.mark.parametrize("dk,dv,vfk,window,chunk,keep,what", FORMS)
 def test_both_kernels_give_the_plain_kernels_results(dk, dv, vfk, window, chunk, keep, what, monkeypatch):
     """Sequences of 1, 127, 128, 129 and 300 rows that start inside and at the start of pages, scattered pages, and rows of the last
-    page past a sequence's end that hold NaN.  `late`: keys that grow along the sequence, so that accumulators are rescaled."""
+    page past a sequence's end that hold NaN.  `late`: keys that grow along the sequence, so that accumulators are rescaled.
+    `gone`: pages that the table does not name or names past the last one, and a page number 0 that is nobody's and holds NaN."""
     from test_rovurax_gpu import plain_kernel_in_float32, scattered_cache
     from x0ne_engine_b200.csrc import ops
     G, H, pages = (1 if vfk else 2), 6, 8
@@ -35,6 +37,14 @@ def test_both_kernels_give_the_plain_kernels_results(dk, dv, vfk, window, chunk,
                 keys(page)[:, max(past, 0):] = float("nan")
                 if not vfk:
                     page[G * 64 * dk:G * 64 * (dk + vd)].view(G, 64, vd)[:, max(past, 0):] = float("nan")
+    if "gone" in what:
+        own = torch.nonzero(table == 0)
+        if len(own):
+            spare = next(p for p in range(view.n_pages) if not bool((table == p).any()))
+            pool[spare] = pool[0]
+            table[own[0, 0], own[0, 1]] = spare
+        pool[0] = float("nan")
+        table[0, 0], table[2, 1], table[4, 0] = -1, view.n_pages + 3, -1          # (slot 4's first rows see no key at all)
     g = torch.Generator().manual_seed(3)
     n_rows = sum(n for _, _, n in seqs)
     inside = "inside" in what

@@ -153,20 +153,22 @@ __global__ void __launch_bounds__(FT_THREADS, 2) flex_prefill_tc_kernel(const __
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
         };
         if (warp == 9) {
+            // A page that the sequence does not have becomes the one past the last: its copy brings zeros, which a weight of zero
+            // leaves alone (another sequence's page may hold NaN or infinities, and 0 times those is NaN).
             auto page_of = [&](int i) -> int {
-                if (i >= n_walk) return -1;
+                if (i >= n_walk) return cache.n_pages;
                 const int pg = cache.page_table[(int64_t)slot * cache.table_stride + page_at(i) % cache.ring_pages];
-                return pg < 0 || pg >= cache.n_pages ? -1 : pg;
+                return pg < 0 || pg > cache.n_pages ? cache.n_pages : pg;
             };
             int pages[3] = {page_of(0), page_of(1), page_of(2)};        // looked up well ahead of the copies that need them
             int k_issued = 0, v_issued = 0;
             auto load_k = [&](int i, int page) {
                 const int st = i & 1;
                 if (leader) {
-                    sh->page_ok[i & 3] = page >= 0;
+                    sh->page_ok[i & 3] = page < cache.n_pages;
                     mbar_expect_tx(&sh->k_full[st], kt_bytes);
                     for (int nb = 0; nb < a.nbk; ++nb)
-                        ft_tma_3d(ks + st * kt_bytes + nb * 64 * 128, &map_k, nb * 64, kh * 64, max(page, 0), &sh->k_full[st]);
+                        ft_tma_3d(ks + st * kt_bytes + nb * 64 * 128, &map_k, nb * 64, kh * 64, page, &sh->k_full[st]);
                 }
                 __syncwarp();
                 ++k_issued;
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(FT_THREADS, 2) flex_prefill_tc_kernel(const __
                         if (leader) {
                             mbar_expect_tx(&sh->v_full[i & 1], vt_bytes);
                             for (int nb = 0; nb < a.nbv; ++nb)
-                                ft_tma_3d(vs + (i & 1) * vt_bytes + nb * 64 * 128, &map_v, nb * 64, kh * 64, max(pages[0], 0), &sh->v_full[i & 1]);
+                                ft_tma_3d(vs + (i & 1) * vt_bytes + nb * 64 * 128, &map_v, nb * 64, kh * 64, pages[0], &sh->v_full[i & 1]);
                         }
                         __syncwarp();
                         ++v_issued;
