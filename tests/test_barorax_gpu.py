@@ -543,3 +543,21 @@ def test_staged_scan_and_register_convolution_at_the_edges_of_their_stages(inner
         assert (y - want).abs().max() <= 2 ** -7 * want.abs().max(), f"scan, sequence {s}"
         # (a token's hardware exponential is off by up to 2^-21 of its argument's size; states forget)
         assert (state[slots[s], :inner * n].double().cpu().view(inner, n) - st["S"]).abs().max() <= 2e-4 * st["S"].abs().max()
+
+
+@pytest.mark.parametrize("rows,inner,taps", [(300, 264, 4), (20, 264, 4), (300, 264, 6), (40, 33, 3)])
+def test_convolution_of_bfloat16_rows_is_the_float32_one_rounded_once(rows, inner, taps):
+    """The same numbers in both types, through every kernel of the convolution: the sums and the activation are the same float32 work, so a
+    bfloat16 run's results are the float32 run's, rounded.  Arguments of the activation from -100 to 100: its denominator goes past 2^126."""
+    from x0ne_engine_b200.csrc import ops
+    g = torch.Generator().manual_seed(rows + taps)
+    xz = torch.randn(rows, inner, generator=g).bfloat16().to(DEV)
+    w = (0.6 * torch.randn(inner, taps, generator=g)).to(DEV)
+    b = torch.linspace(-100.0, 100.0, inner).to(DEV)
+    state = torch.randn(1, inner * taps, generator=g).to(DEV)
+    out = []
+    for dtype in (torch.float32, torch.bfloat16):
+        u = torch.zeros((rows, inner), dtype=dtype, device=DEV)
+        ops.causal_conv_silu(xz.to(dtype), w, b, state, inner, u, i32([0] * rows), i32(list(range(rows))), rows, inner)
+        out.append(u)
+    assert torch.equal(out[1], out[0].bfloat16())

@@ -48,9 +48,6 @@ __device__ __forceinline__ float ssm_exp_prod(float a, float b) {
 }
 
 __device__ __forceinline__ float ssm_silu(float v) { return v / (1.0f + expf(-v)); }
-// the same for results that are stored as bfloat16: the hardware's exponential and reciprocal, errors near 2^-21
-template <typename T> __device__ __forceinline__ float ssm_silu_for(float v) { return ssm_silu(v); }
-template <> __device__ __forceinline__ float ssm_silu_for<bf16>(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 __device__ __forceinline__ float ssm_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 // ----------------------------------------------------------------------------------------
@@ -89,7 +86,7 @@ __global__ void causal_conv_silu_kernel(const T* x, int64_t ld, const float* __r
         else if (slot >= 0) v = state[(int64_t)slot * state_stride + conv_off + (int64_t)(taps - 1 + above - back) * channels + c];
         acc = fmaf(wk[k], v, acc);
     }
-    out[(int64_t)row * channels + c] = from_f32<T>(ssm_silu_for<T>(acc));
+    out[(int64_t)row * channels + c] = from_f32<T>(ssm_silu(acc));
 }
 
 // The same for 8 consecutive channels per thread (channels and row pitch multiples of 8, 16-byte aligned rows): 16-byte
@@ -128,8 +125,9 @@ __device__ __forceinline__ void ssm_store8(bf16* p, const float* v) {
 #define SSM_CONV_TAPS 4         // most taps it keeps
 
 // The same with a thread's taps and its stretch of rows in registers: all rows are asked for at once, each is read by one thread of a
-// column (and by the next stretch's for its first taps).  2,048 rows of 4,096 channels, 4 taps, bfloat16: 48 -> 27 us, with the
-// hardware's exponential and reciprocal behind it 16 (33.5 MB: 5.1 us at the copy rate; what is left is the activation).
+// column (and by the next stretch's for its first taps).  2,048 rows of 4,096 channels, 4 taps, bfloat16: 48 -> 27 us
+// (33.5 MB: 5.1 us at the copy rate; what is left is mostly the activation, a full exponential and division in both types: with the
+// hardware's approximations it took 16, at less than float32's precision).
 template <typename T>
 __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
         const T* x, int64_t ld, const float* __restrict__ w, const float* __restrict__ bias, const float* state, int64_t state_stride,
@@ -191,7 +189,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
+            for (int i = 0; i < 8; ++i) acc[i] = ssm_silu(acc[i]);
             ssm_store8(out + (int64_t)(first + r) * channels + c, acc);
         }
         return;
@@ -217,7 +215,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_run_kernel(
             for (int i = 0; i < 8; ++i) acc[i] = fmaf(wk[back][i], v[i], acc[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
+        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu(acc[i]);
         ssm_store8(out + (int64_t)row * channels + c, acc);
     }
 }
@@ -268,7 +266,7 @@ __global__ void __launch_bounds__(128) causal_conv_silu_vec_kernel(
             for (int i = 0; i < 8; ++i) acc[i] = fmaf(w_s[(k * 8 + i) * 128 + tid], v[i], acc[i]);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu_for<T>(acc[i]);
+        for (int i = 0; i < 8; ++i) acc[i] = ssm_silu(acc[i]);
         ssm_store8(out + (int64_t)row * channels + c, acc);
     }
 }
