@@ -1512,7 +1512,8 @@ def selective_scan(u: torch.Tensor, xz: torch.Tensor, z_col: int, dt_raw: torch.
     out = (S . C + D u) * silu(z).  u, xz (the convolution's input at column 0, z at z_col) and out in the activation type;
     dt_raw, A (negative), bc (B at b_col, C at c_col), D, state float32.  `one_token`: every sequence brings one row (a decode
     step); the same bits, from a form of the kernel without idle places.
-    `max_rows`: the most rows a sequence brings, where that is known (0: it is not); it chooses the kernel of bfloat16 runs."""
+    `max_rows`: the most rows a sequence brings, where that is known (0: it is not); it chooses the kernel of bfloat16 runs, with the
+    same bits.  (In bfloat16 runs the number of sequences and channels may choose the order of a token's sum; in float32 runs nothing does.)"""
     lib = _lib("core")
     for t, what in ((u, "scan input"), (xz, "projection"), (out, "scan output")):
         _need(t, u.dtype, what)

@@ -10,10 +10,11 @@
 //          S[c][n] = exp(dt A[c][n]) S[c][n] + dt u[t][c] B[t][n]
 //          y[t][c] = (sum_n S[c][n] C[t][n] + D[c] u[t][c]) * silu(z[t][c])
 //
-// Step sizes, decays, states and every sum are float32 whatever the activation type.  One device function makes a token's
-// step, for prompts and for one-token steps alike, and the sums over n run in an order that depends on N only (a thread's
-// own states in ascending order, then the threads of a channel as a shuffle tree; how many threads share a channel depends on N alone), so a token's result is the same bits
-// however its sequence was cut into passes and whatever else the pass holds.
+// Step sizes, decays, states and every sum are float32 whatever the activation type.  Every kernel makes a token's step by the same
+// operations, and the sums over n run in one order: a thread's own states in ascending order, then the threads of a channel as a shuffle
+// tree.  How many threads share a channel is one function's choice (ssm_split), for prompts and for one-token steps alike.  In float32 runs
+// it depends on N alone, so a token's result is the same bits however its sequence was cut into passes and whatever else a pass holds;
+// in bfloat16 runs on the channels and the number of sequences too, so it is the same bits in every pass with as many sequences.
 #include "common.cuh"
 
 #define SSM_THREADS 128    // per block of the scan: channels x the threads that share a channel's states
@@ -392,12 +393,22 @@ template <int NS> __device__ __forceinline__ void ssm_load_states(float (&v)[NS]
     else v[0] = p[0];
 }
 
+// What a state's decay is made from (`a` of A) and how, and in which order the threads of a channel (SPLIT) add up.  bfloat16 runs of up to 32
+// states take log2 e into A once and go from the far neighbour to the near one, which leaves every thread of the staged kernel
+// with sums of its own.
+template <typename T, int NS, int SPLIT> struct SsmOrder {
+    static constexpr bool STAGED = sizeof(T) == 2 && NS * SPLIT <= 32;
+    static __device__ __forceinline__ float factor(float a) { return STAGED ? a * 1.4426950408889634f : a; }
+    static __device__ __forceinline__ float decay(float dt, float f) { return STAGED ? ssm_ex2(dt * f) : SsmMath<T>::decay(dt, f); }
+    static __device__ __forceinline__ int neighbour(int level) { return STAGED ? SPLIT / 2 / level : level; }      // level: 1, 2, 4 .. SPLIT / 2
+};
+
 // A pass in which every sequence brings one row (or few): a thread reads its token's values itself, nothing is staged and
-// no thread waits for another.  The operations of a token and their order are the staged kernel's, so the bits are.
+// no thread waits for another.  The operations of a token and their order are the other kernels', so the bits are.
 template <typename T, int NS, int SSM_SPLIT>
 __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArgs a) {
     constexpr int SSM_CH = SSM_THREADS / SSM_SPLIT;
-    constexpr bool STAGED = sizeof(T) == 2 && NS * SSM_SPLIT <= 32;     // whether the scan of many rows is the staged kernel below
+    typedef SsmOrder<T, NS, SSM_SPLIT> Order;
     pdl_launch_dependents();
     const int tid = threadIdx.x;
     const int cl = tid / SSM_SPLIT, part = tid % SSM_SPLIT;
@@ -409,7 +420,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArg
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
         const int n = part * NS + i;
-        An[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] * (STAGED ? 1.4426950408889634f : 1.f) : 0.f;
+        An[i] = live && n < a.N ? Order::factor(a.A[(int64_t)c * a.N + n]) : 0.f;
     }
     if (live) {
         Dc = a.D != nullptr ? a.D[c] : 0.f;
@@ -438,11 +449,11 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_step_kernel(SsmArg
         for (int i = 0; i < NS; ++i) {
             const int n = part * NS + i;
             const float bn = n < a.N ? a.bc[r * a.bc_ld + a.b_col + n] : 0.f, cn = n < a.N ? a.bc[r * a.bc_ld + a.c_col + n] : 0.f;
-            S[i] = fmaf(STAGED ? ssm_ex2(dt * An[i]) : SsmMath<T>::decay(dt, An[i]), S[i], dtu * bn);
+            S[i] = fmaf(Order::decay(dt, An[i]), S[i], dtu * bn);
             acc = fmaf(S[i], cn, acc);
         }
 #pragma unroll
-        for (int w = 1; w < SSM_SPLIT; w <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, STAGED ? SSM_SPLIT / 2 / w : w);
+        for (int w = 1; w < SSM_SPLIT; w <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, Order::neighbour(w));
         if (part == 0 && live)
             out[r * a.channels + c] = from_f32<T>(fmaf(Dc, uv, acc) * SsmMath<T>::silu(to_f32(xz[r * a.xz_ld + a.z_col + c])));
     }
@@ -460,6 +471,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_kernel(SsmArgs a) 
     constexpr int THREADS = SSM_THREADS;
     constexpr int SSM_CH = THREADS / SSM_SPLIT;                 // channels per block
     constexpr int NP = NS * SSM_SPLIT;                          // states per channel as the block holds them
+    typedef SsmOrder<T, NS, SSM_SPLIT> Order;
     constexpr int PER_CH = (SSM_TC * SSM_CH + THREADS - 1) / THREADS;   // staged (token, channel) values per thread
     constexpr int PER_N = (SSM_TC * NP + THREADS - 1) / THREADS;
     __shared__ float s_dt[SSM_TC][SSM_CH], s_u[SSM_TC][SSM_CH], s_z[SSM_TC][SSM_CH];
@@ -475,7 +487,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_kernel(SsmArgs a) 
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
         const int n = part * NS + i;
-        An[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] : 0.f;
+        An[i] = live && n < a.N ? Order::factor(a.A[(int64_t)c * a.N + n]) : 0.f;
     }
     if (live) Dc = a.D != nullptr ? a.D[c] : 0.f;
     // the staging thread's own (token, channel) and (token, n) places
@@ -562,7 +574,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_kernel(SsmArgs a) 
                 const float dtu = dt * uv[k];
 #pragma unroll
                 for (int i = 0; i < NS; ++i) {
-                    dec[k][i] = SsmMath<T>::decay(dt, An[i]);
+                    dec[k][i] = Order::decay(dt, An[i]);
                     in[k][i] = dtu * s_b[tl0 + k][part * NS + i];
                 }
             }
@@ -578,7 +590,7 @@ __global__ void __launch_bounds__(SSM_THREADS) selective_scan_kernel(SsmArgs a) 
 #pragma unroll
             for (int w = 1; w < SSM_SPLIT; w <<= 1) {
 #pragma unroll
-                for (int k = 0; k < U; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], w);
+                for (int k = 0; k < U; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], Order::neighbour(w));
             }
             if (part == 0 && live) {
 #pragma unroll
@@ -612,6 +624,7 @@ __global__ void __launch_bounds__(SSM_THREADS + SSM_STAGERS, 2) selective_scan_s
     constexpr int TP = CH * SSM_TC / SSM_STAGERS;                  // tokens of one channel a staging thread brings per stage
     constexpr int PER_N = (SSM_TC * NP + SSM_STAGERS - 1) / SSM_STAGERS;
     static_assert(TP == 4 || TP == 2, "a staging thread's tokens are stored at once");
+    typedef SsmOrder<bf16, NS, SPLIT> Order;
     typedef typename SsmVec<TP>::T Vec;
     __shared__ __align__(16) float s_dt[2][CH][PITCH], s_in[2][CH][PITCH], s_u[2][CH][PITCH], s_z[2][CH][PITCH];   // s_z: the gate, then the result
     __shared__ __align__(16) float s_b[2][SSM_TC][NP], s_c[2][SSM_TC][NP];
@@ -628,7 +641,7 @@ __global__ void __launch_bounds__(SSM_THREADS + SSM_STAGERS, 2) selective_scan_s
 #pragma unroll
     for (int i = 0; i < NS; ++i) {
         const int n = part * NS + i;
-        A2[i] = live && n < a.N ? a.A[(int64_t)c * a.N + n] * 1.4426950408889634f : 0.f;
+        A2[i] = live && n < a.N ? Order::factor(a.A[(int64_t)c * a.N + n]) : 0.f;
     }
     if (live && a.D != nullptr) Dc = a.D[c];
     const bool owns = !works && c_own < a.channels;
@@ -727,7 +740,7 @@ __global__ void __launch_bounds__(SSM_THREADS + SSM_STAGERS, 2) selective_scan_s
                     ssm_load_states<NS>(B, &s_b[b][tl0 + k][part * NS]);
 #pragma unroll
                     for (int i = 0; i < NS; ++i) {
-                        dec[k][i] = ssm_ex2(dt[k] * A2[i]);
+                        dec[k][i] = Order::decay(dt[k], A2[i]);
                         put[k][i] = in[k] * B[i];
                     }
                 }
@@ -784,22 +797,25 @@ __global__ void __launch_bounds__(SSM_THREADS + SSM_STAGERS, 2) selective_scan_s
     if (part == 0) ssm_keep_inputs<bf16>(a, st, xz, row0, n_tok, c);
 }
 
-// How many threads share a channel in the other kernels: 4, 8 or 16 (more threads per channel are more warps to hide the latency of a token's
-// dependent steps with, at more instructions in all; a single prompt's scan is bound by that latency, many sequences'
-// by the instructions).
-// A float32 run's choice depends on N alone, so that a token has the same bits in every pass; a bfloat16 run takes the
-// fewest threads per channel that still give every scheduler of the GPU a few warps.
+// How many threads share a channel, in every kernel that may see a run's tokens.  float32 runs: N alone chooses, so that a token has the
+// same bits in every pass.  bfloat16 runs of up to 32 states: 8 where 4 would leave more than a quarter of the multiprocessors without
+// a block of the staged scan; wider ones the fewest that still give every scheduler of the GPU a few warps.
+static int ssm_split(bool bf16_run, int64_t n_seqs, int64_t channels, int N, int64_t sm_count) {
+    if (!bf16_run) return N > 32 ? 16 : 4;
+    if (N <= 32) return N > 16 || (N > 4 && n_seqs * ((channels + 31) / 32) * 4 < sm_count * 3) ? 8 : 4;
+    return 16;
+}
+
 template <typename T>
 static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int rows, cudaStream_t stream) {
     const bool one_token = rows == SSM_ONE_ROW;
+    const int split = ssm_split(sizeof(T) == 2, n_seqs, a.channels, a.N, sm_count);
     // sequences of a few rows stay with the kernel of 128 threads a block, of which many fit on a multiprocessor: 16 sequences of 9 /
     // 13 / 20 rows, a layer of 4,096 channels, 64.0 / 74.4 / 93.0 us with it, 74.3 / 82.3 / 80.1 staged; one sequence of 9: 39.4 and 39.7
     if (sizeof(T) == 2 && rows == SSM_MANY_ROWS && a.N <= 32) {
-        // 8 threads per channel where 4 would leave more than a quarter of the multiprocessors without a block
-        const bool eight = a.N > 16 || (a.N > 4 && (int64_t)n_seqs * ((a.channels + 31) / 32) * 4 < (int64_t)sm_count * 3);
-        const int per = eight ? 16 : 32;
+        const int per = SSM_THREADS / split;
         const dim3 sgrid((unsigned)((a.channels + per - 1) / per), (unsigned)n_seqs), sblock(SSM_THREADS + SSM_STAGERS);
-        if (eight) {
+        if (split == 8) {
             if (a.N <= 8) x0ne_launch(selective_scan_staged_kernel<1, 8>, sgrid, sblock, 0, stream, a);
             else if (a.N <= 16) x0ne_launch(selective_scan_staged_kernel<2, 8>, sgrid, sblock, 0, stream, a);
             else x0ne_launch(selective_scan_staged_kernel<4, 8>, sgrid, sblock, 0, stream, a);
@@ -809,12 +825,6 @@ static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int
             else x0ne_launch(selective_scan_staged_kernel<4, 4>, sgrid, sblock, 0, stream, a);
         }
         X0NE_LAUNCH_CHECK();
-    }
-    int split = a.N > 32 ? 16 : 4;
-    if (sizeof(T) == 2) {
-        const int64_t want_warps = (int64_t)sm_count * 4 * 3;
-        const int most = a.N > 32 || !one_token ? 16 : 8;         // (one token's bits are the staged scan's where both take 8)
-        while (split < most && split < a.N && (int64_t)n_seqs * a.channels * split / 32 < want_warps) split *= 2;
     }
     const int ns = (a.N + split - 1) / split;
     const dim3 grid((unsigned)((a.channels + SSM_THREADS / split - 1) / (SSM_THREADS / split)), (unsigned)n_seqs), block(SSM_THREADS);
@@ -828,16 +838,18 @@ static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int
         if (ns <= 1) SSM_GO(1, 4, 4);
         else if (ns <= 2) SSM_GO(2, 4, 4);
         else if (ns <= 4) SSM_GO(4, 4, 4);
-        else if (ns <= 6) SSM_GO(6, 4, 2);
-        else SSM_GO(8, 4, 2);
+        else if constexpr (sizeof(T) == 4) {
+            if (ns <= 6) SSM_GO(6, 4, 2);
+            else SSM_GO(8, 4, 2);
+        }
     } else if (split == 8) {
-        if (ns <= 1) SSM_GO(1, 8, 4);
-        else if (ns <= 2) SSM_GO(2, 8, 4);
-        else SSM_GO(4, 8, 2);
+        if constexpr (sizeof(T) == 2) {
+            if (ns <= 1) SSM_GO(1, 8, 4);
+            else if (ns <= 2) SSM_GO(2, 8, 4);
+            else SSM_GO(4, 8, 2);
+        }
     } else {
-        if (ns <= 1) SSM_GO(1, 16, 4);
-        else if (ns <= 2) SSM_GO(2, 16, 4);
-        else if (ns <= 3) SSM_GO(3, 16, 2);
+        if (ns <= 3) SSM_GO(3, 16, 2);
         else if (ns <= 4) SSM_GO(4, 16, 2);
         else if (ns <= 6) SSM_GO(6, 16, 1);
         else SSM_GO(8, 16, 1);
