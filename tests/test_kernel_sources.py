@@ -76,3 +76,9 @@ def test_kernels_let_their_successors_start_only_with_their_tensor_memory_in_han
     for name, body in own:
         assert re.search(r"tcgen05\.alloc.*__syncthreads\(\);.*pdl_launch_dependents\(\);", body, re.S), name
         assert "pdl_launch_dependents" not in body[:body.index("tcgen05.alloc")], name
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))), ids=os.path.basename)
+def test_rules_ask_the_device_for_its_multiprocessors(path):
+    with open(path) as f:
+        assert not re.search(r"\b148\b", re.sub(r"//[^\n]*", "", f.read()))

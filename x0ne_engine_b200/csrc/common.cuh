@@ -87,6 +87,18 @@ struct OncePerDevice {
     }
 };
 
+// Multiprocessors of the current device (asked for once per device); rules that look at how a launch fills the GPU go by it.
+static inline int x0ne_sm_count() {
+    static int count[64] = {};
+    const int dev = OncePerDevice::device();
+    int n = dev >= 0 ? count[dev] : 0;
+    if (n <= 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev >= 0 ? dev : 0) != cudaSuccess || n <= 0) return 1;
+        if (dev >= 0) count[dev] = n;
+    }
+    return n;
+}
+
 template <typename... KArgs, typename... Args>
 static inline cudaError_t x0ne_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                       Args... args) {

@@ -731,7 +731,7 @@ X0NE_API int x0ne_swiglu(const void* gate_up, const float* bias, void* out, int 
     if (inter % 8 == 0 && (((uintptr_t)gate_up | (uintptr_t)bias | (uintptr_t)out) & 15) == 0 && ((int64_t)inter * esize) % 16 == 0) {
         const int64_t total8 = (int64_t)n_rows * (inter / 8);
         int64_t blocks = (total8 + 255) / 256;
-        if (blocks > 148 * 16) blocks = 148 * 16;
+        if (blocks > x0ne_sm_count() * 16) blocks = x0ne_sm_count() * 16;
         if (dt == X0NE_F32)
             x0ne_launch(swiglu_vec_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, (const float*)gate_up, bias, (float*)out, inter, total8);
         else if (dt == X0NE_BF16)

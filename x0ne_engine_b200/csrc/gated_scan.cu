@@ -752,7 +752,7 @@ X0NE_API int x0ne_channel_gates(GatedRaw x, float* out, int n_rows, int hd, cuda
                      gs_aligned16(x.lower) && gs_aligned16(out);
     const int64_t total = (int64_t)n_rows * hd / (vec ? 4 : 1);
     const int64_t blocks = (total + 255) / 256;
-    const dim3 grid((unsigned)(blocks < 148 * 64 ? blocks : 148 * 64));
+    const dim3 grid((unsigned)(blocks < x0ne_sm_count() * 64 ? blocks : x0ne_sm_count() * 64));
     if (vec) x0ne_launch(channel_gates_vec_kernel, grid, dim3(256), 0, stream, x, out, total, hd);
     else x0ne_launch(channel_gates_kernel, grid, dim3(256), 0, stream, x, out, total, hd);
     X0NE_LAUNCH_CHECK();

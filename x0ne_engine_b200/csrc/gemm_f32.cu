@@ -295,9 +295,9 @@ X0NE_API int x0ne_gemm_f32_nt_batched(const float* A, const float* W, float* C, 
             // the largest tile that still gives every multiprocessor several (64 x 128), one (64 x 64), else small ones; measured at 100 to
             // 2,048 rows: 64 x 128 / 64 x 64 / 32 x 64 at 2,048 rows of 12288 x 2048 2288 / 2600 / 3225 us (3,072 tiles), of 2048 x 2048 572 / 440 / 547
             // (512), at 100 rows 161 / 99 / 70 (32)
-            const int64_t m64 = (M + 63) / 64, m32 = (M + 31) / 32;
-            if (batch * m64 * ((N + 127) / 128) >= 6 * 148) gemm_f32_tiles<64, 128, 8, 8, false, 1>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
-            else if (batch * m64 * ((N + 63) / 64) >= 148 || m32 > 65535) gemm_f32_tiles<64, 64, 4, 8, true, 4>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+            const int64_t m64 = (M + 63) / 64, m32 = (M + 31) / 32, sms = x0ne_sm_count();
+            if (batch * m64 * ((N + 127) / 128) >= 6 * sms) gemm_f32_tiles<64, 128, 8, 8, false, 1>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
+            else if (batch * m64 * ((N + 63) / 64) >= sms || m32 > 65535) gemm_f32_tiles<64, 64, 4, 8, true, 4>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
             else gemm_f32_tiles<32, 64, 4, 4, true, 1>(A, W, C, M, N, K, lda, ldw, ldc, batch, sa, sw, sc, stream);
         }
         X0NE_LAUNCH_CHECK();

@@ -1535,6 +1535,6 @@ X0NE_API int x0ne_soft_cap(float* x, int64_t total, float cap, cudaStream_t stre
     X0NE_REQUIRE(total >= 0 && cap > 0.f, "soft_cap: %lld values, cap %g", (long long)total, cap);
     if (total == 0) return 0;
     const int64_t blocks = (total + 255) / 256;
-    x0ne_launch(soft_cap_kernel, dim3((unsigned)(blocks < 148 * 32 ? blocks : 148 * 32)), dim3(256), 0, stream, x, total, cap);
+    x0ne_launch(soft_cap_kernel, dim3((unsigned)(blocks < x0ne_sm_count() * 32 ? blocks : x0ne_sm_count() * 32)), dim3(256), 0, stream, x, total, cap);
     X0NE_LAUNCH_CHECK();
 }

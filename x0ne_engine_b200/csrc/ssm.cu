@@ -867,13 +867,7 @@ X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int rows, cudaSt
     X0NE_REQUIRE(a.xz_ld >= a.channels && a.z_col >= 0 && a.z_col + a.channels <= a.xz_ld && a.b_col >= 0 && a.c_col >= 0 &&
                      a.b_col + a.N <= a.bc_ld && a.c_col + a.N <= a.bc_ld, "selective_scan: columns lie outside their rows");
     if (n_seqs == 0) return 0;
-    static int sm_count[64] = {};
-    const int dev = OncePerDevice::device();
-    int sms = dev >= 0 ? sm_count[dev] : 0;
-    if (sms <= 0) {
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev >= 0 ? dev : 0) != cudaSuccess || sms <= 0) sms = 148;
-        if (dev >= 0) sm_count[dev] = sms;
-    }
+    const int sms = x0ne_sm_count();
     if (dt == X0NE_F32) return selective_scan_launch<float>(a, n_seqs, sms, rows, stream);
     if (dt == X0NE_BF16) return selective_scan_launch<bf16>(a, n_seqs, sms, rows, stream);
     X0NE_REQUIRE(false, "selective_scan: unknown dtype tag %d", dt);

@@ -505,8 +505,7 @@ static int wkv_scan_launch(const T* r, const T* k, const T* v, const float* z, c
                            float* state, int64_t state_stride, const int32_t* seq_first_row, const int32_t* seq_slot, int n_seqs,
                            int heads, int N, int width, int one_token, cudaStream_t stream) {
     const dim3 grid(n_seqs, heads);
-    int sms = 0, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+    const int sms = x0ne_sm_count();
 #define WKV_ARGS r, k, v, z, w0, u, h, o, state, state_stride, seq_first_row, seq_slot, heads, N, width
 #define WKV_SCAN_AS(NB, P, U) x0ne_launch(wkv_scan_kernel<T, NB, P, U>, dim3(n_seqs, heads, NB / WKV_CB), dim3(2 * NB + P), 0, stream, WKV_ARGS)
 #define WKV_SCAN(NB)                                                                                     \
