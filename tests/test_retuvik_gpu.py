@@ -289,6 +289,53 @@ def test_gated_experts_over_grouped_pairs(dtype, rows, E, top, hidden, ff):
         assert tc                                          # these shapes are the tensor-core kernel's
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("top", [1, 4, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("hidden", [132, 1028])
+def test_weighted_sum_over_choices_at_the_edges_of_its_forms(dtype, top, hidden):
+    """Numbers of choices on both sides of every change of form, identity choices among them, with and without a shared expert and its gate:
+    one chain of multiply-adds in the choices' order."""
+    from x0ne_engine_b200.csrc import ops
+    g = torch.Generator().manual_seed(top + hidden)
+    rows, E = 37, 6
+    y, x = torch.randn(rows * top, hidden, generator=g), torch.randn(rows, hidden, generator=g).to(dtype)
+    chosen = torch.randint(0, E + 2, (rows, top), generator=g).to(torch.int32)
+    weights, sgate = torch.rand(rows, top, generator=g), torch.rand(rows, generator=g)
+    shared = torch.randn(rows, hidden, generator=g).to(dtype)
+    picked = torch.where((chosen < E)[:, :, None], y.view(rows, top, hidden), x.float()[:, None].expand(rows, top, hidden)).double()
+    for sh, sg in ((None, None), (shared, None), (shared, sgate)):
+        want = (weights.double()[:, :, None] * picked).sum(dim=1)
+        if sh is not None:
+            want = want + (1.0 if sg is None else sg.double()[:, None]) * sh.double()
+        out = torch.empty((rows, hidden), dtype=dtype, device=DEV)
+        dev = lambda t: None if t is None else t.to(DEV)      # noqa: E731
+        ops.moe_combine(dev(y), dev(x), dev(chosen), dev(weights), top, E, dev(sh), dev(sg), out, rows)
+        bound = ((top + 1) * 2.0 ** -24 if dtype == torch.float32 else 2.0 ** -8) * want.abs().max() * (4 if dtype == torch.float32 else 1)
+        assert (out.double().cpu() - want).abs().max() <= bound
+
+
+@pytest.mark.parametrize("pairs", [1, 1023, 1025, 8191, 8192, 8193, 16385, 40000])
+def test_grouping_lists_every_pair_once_whatever_their_number(pairs):
+    """Numbers of pairs on both sides of a sweep of the block, identity choices and an expert without pairs among them."""
+    from x0ne_engine_b200.csrc import ops
+    E, tile = 11, 128
+    chosen = torch.randint(0, E + 2, (pairs,), generator=torch.Generator().manual_seed(pairs))
+    chosen[chosen == 4] = 5
+    n_tiles = ops.moe_max_tiles(pairs, E, tile)
+    i32 = lambda *shape: torch.full(shape, -7, dtype=torch.int32, device=DEV)      # noqa: E731
+    offsets, listed, tiles, n_real = i32(E + 1), i32(pairs + 1), i32(n_tiles, 3), i32(1)
+    ops.moe_group(chosen.to(torch.int32).to(DEV), pairs, E, offsets, listed, tiles, tile, n_real)
+    counts = [int((chosen == e).sum()) for e in range(E)]
+    first = [sum(counts[:e]) for e in range(E + 1)]
+    assert offsets.tolist() == first
+    got = listed.tolist()
+    for e in range(E):
+        assert sorted(got[first[e]:first[e + 1]]) == torch.nonzero(chosen == e).flatten().tolist()
+    assert all(v == -7 for v in got[first[E]:])
+    want = [[e, first[e] + i, min(tile, counts[e] - i)] for e in range(E) for i in range(0, counts[e], tile)]
+    assert int(n_real[0]) == len(want) and tiles[:len(want)].tolist() == want and bool((tiles[len(want):, 2] == 0).all())
+
+
 SLOPE_CASES = [  # q_heads, kv_heads, dk, dv, window
     (4, 2, 48, None, 100),
     (6, 2, 20, 12, 37),

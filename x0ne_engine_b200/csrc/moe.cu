@@ -167,7 +167,7 @@ __global__ void moe_route_kernel(const float* z, int ldz, const float* __restric
 //   tiles   [max_tiles][3]  expert, first place, count (count 0: the tile does not exist); tiles of tile_m pairs
 //   n_tiles_out             how many tiles exist (optional)
 // ----------------------------------------------------------------------------------------
-#define GP_OWN 8        // choices of a thread that stay in registers
+#define GP_OWN 8        // choices that a thread asks for together
 __global__ void moe_group_kernel(const int32_t* chosen, int pairs, int experts, int32_t* offsets,
                                  int32_t* listed, int32_t* tiles, int max_tiles, int tile_m,
                                  int32_t* n_tiles_out) {
@@ -176,21 +176,34 @@ __global__ void moe_group_kernel(const int32_t* chosen, int pairs, int experts, 
     int* start = count + experts;         // [experts + 1]
     int* tile0 = start + experts + 1;     // [experts + 1]
     pdl_prologue();
-    // a thread's first choices stay in registers for both walks, asked for together (8,192 pairs: 15 -> 6 us)
-    int own[GP_OWN];
+    // a thread asks for GP_OWN choices together, one sweep of the block after the other, and keeps those of the first sweep for both walks
+    // (8,192 pairs over 32 experts 7.4 us, 16,384 12.3 -> 11.7, 65,536 41.4 -> 34.9 with the later sweeps read together too)
+    const int sweep = GP_OWN * blockDim.x;
+    auto read = [&](int (&v)[GP_OWN], int p0) {
 #pragma unroll
-    for (int i = 0; i < GP_OWN; ++i) {
-        const int p = threadIdx.x + i * blockDim.x;
-        own[i] = p < pairs ? chosen[p] : -1;
-    }
+        for (int i = 0; i < GP_OWN; ++i) {
+            const int p = p0 + threadIdx.x + i * blockDim.x;
+            v[i] = p < pairs ? chosen[p] : -1;
+        }
+    };
+    auto add = [&](const int (&v)[GP_OWN]) {
+#pragma unroll
+        for (int i = 0; i < GP_OWN; ++i)
+            if (v[i] >= 0 && v[i] < experts) atomicAdd(&count[v[i]], 1);
+    };
+    auto list = [&](const int (&v)[GP_OWN], int p0) {
+#pragma unroll
+        for (int i = 0; i < GP_OWN; ++i)
+            if (v[i] >= 0 && v[i] < experts) listed[start[v[i]] + atomicAdd(&count[v[i]], 1)] = p0 + threadIdx.x + i * blockDim.x;
+    };
+    int own[GP_OWN], later[GP_OWN];
+    read(own, 0);
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < GP_OWN; ++i)
-        if (own[i] >= 0 && own[i] < experts) atomicAdd(&count[own[i]], 1);
-    for (int p = threadIdx.x + GP_OWN * blockDim.x; p < pairs; p += blockDim.x) {
-        const int e = chosen[p];
-        if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
+    add(own);
+    for (int p0 = sweep; p0 < pairs; p0 += sweep) {
+        read(later, p0);
+        add(later);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -219,12 +232,10 @@ __global__ void moe_group_kernel(const int32_t* chosen, int pairs, int experts, 
     __syncthreads();
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < GP_OWN; ++i)
-        if (own[i] >= 0 && own[i] < experts) listed[start[own[i]] + atomicAdd(&count[own[i]], 1)] = threadIdx.x + i * blockDim.x;
-    for (int p = threadIdx.x + GP_OWN * blockDim.x; p < pairs; p += blockDim.x) {
-        const int e = chosen[p];
-        if (e >= 0 && e < experts) listed[start[e] + atomicAdd(&count[e], 1)] = p;
+    list(own, 0);
+    for (int p0 = sweep; p0 < pairs; p0 += sweep) {
+        read(later, p0);
+        list(later, p0);
     }
 }
 
@@ -367,8 +378,9 @@ __device__ __forceinline__ void cmb_store4(bf16* p, const float* v) {
     *reinterpret_cast<uint2*>(p) = u;
 }
 #define CMB_MAX_TOP 16
-// TOP: the most choices a row may have (registers for 16 leave a third of the threads on a multiprocessor: 2,048 rows of 2,048 with 4
-// choices 31 us, with registers for 4 14).
+// TOP: the most choices a row may have; registers for more than it has leave fewer threads on a multiprocessor.  2,048 rows of 2,048, replayed one
+// after the other: 4 choices 9.2 us with registers for 4; 5 / 6 / 8 choices 31.6 / 36.5 / 37.1 us with registers for 16, 17.5 / 22.0 / 24.9 with registers for 8;
+// 9 and 16 choices 44.3 and 57.2.
 template <typename T, int TOP>
 __global__ void moe_combine_vec_kernel(const float* y, const T* x, const int32_t* chosen,
                                        const float* weights, int top, int experts, const T* shared,
@@ -482,9 +494,11 @@ X0NE_API int x0ne_moe_combine(const float* y, const void* x, int dt, const int32
                 sgate, (T*)out, hidden)
         if (dt == X0NE_F32) {
             if (top <= 4) CMB_GO(float, 4);
+            else if (top <= 8) CMB_GO(float, 8);
             else CMB_GO(float, CMB_MAX_TOP);
         } else {
             if (top <= 4) CMB_GO(bf16, 4);
+            else if (top <= 8) CMB_GO(bf16, 8);
             else CMB_GO(bf16, CMB_MAX_TOP);
         }
 #undef CMB_GO
