@@ -60,3 +60,12 @@ def test_fill_of_the_weight_streaming_kernel():
     assert routes.Shape(6144, 4096).smallm_fill == pytest.approx(192 / 296)          # two tiles each on 192
     assert routes.Shape(5120, 25600).smallm_fill == pytest.approx(160 / 296)
     assert routes.Shape(5120, 25600).long_rows and not routes.Shape(6144, 4096).long_rows
+
+
+@pytest.mark.parametrize("n,k,rows,expect", [
+    (12288, 2048, 767, "library"), (12288, 2048, 768, "library"), (12288, 2048, 1535, "library"), (12288, 2048, 1536, "tc_pair"), (12288, 2048, 2048, "tc_pair"),
+    (6144, 2048, 768, "library"), (6144, 2048, 2048, "library"), (6144, 2048, 2049, "tc_pair"), (9216, 1536, 2048, "library"), (2048, 2048, 1024, "library"),
+    (6144, 1024, 2048, "library"), (24576, 4096, 768, "tc_pair"),
+])
+def test_gated_products_of_many_rows_go_where_they_were_measured_ahead(n, k, rows, expect):
+    assert routes.kernel_for(rows, n, k, fused=True) == expect

@@ -92,9 +92,13 @@ RULES: List[Rule] = [
     Rule("skinny", (17, 48), False, lambda s: s.weight_bytes >= 64 * MB,
          "10240 x 5120 at 32 rows: skinny 20.1 us, library 21.1; 5120 x 8192: 17.0 / 19.4; at 64 rows the library is ahead on both"),
     # ---- many rows
-    Rule("library", (768, 2048), True, lambda s: s.k <= 1024,
-         "gate|up 6144 x 1024 at 1,024 / 1,536 / 2,048 rows: library 23.1 / 26.7 / 36.9 us with the activation's launch, tc_pair 28.0 / 29.4 / 38.1 "
-         "(a tile of 16 steps over K does not cover its epilogue); at 4,096 rows 64.1 against 63.7"),
+    Rule("library", (768, 2048), True, lambda s: s.k <= 1024 or (s.k <= 2048 and s.weight_bytes < 48 * MB),
+         "gate|up 6144 x 2048 at 768 / 2,048 rows: library 20.3 / 48.4 us with the activation's launch, tc_pair 26.2 / 52.4; 9216 x 1536 23.6 / 53.4 against "
+         "32.9 / 55.4; 2048 x 2048 11.0 / 19.9 against 24.8 / 25.7; 6144 x 1024 at 2,048 rows 36.9 against 38.1 (a tile of so few steps over K hardly "
+         "covers its epilogue, and few tiles leave pairs of blocks without one)"),
+    Rule("library", (768, 1535), True, lambda s: s.k <= 2048,
+         "gate|up 12288 x 2048 at 768 / 1,024 / 1,300 rows: library 35.9 / 48.5 / 59.1 us with the activation's launch, tc_pair 39.9 / 55.3 / 65.7; "
+         "at 1,536 / 2,048 67.7 / 96.8 against 68.3 / 93.9 (weights in L2; from memory 95.7 against 86.0 at 2,048)"),
     Rule("tc_pair", (1536, 1 << 30), False, lambda s: s.k <= 2048 and s.n >= 2 * s.k,
          "squared ReLU behind 9216 x 2048 at 2,048 rows: 56.6 us in the epilogue, library 59.8 with the launch; 6144 x 2048: 56.5 / 60.7 "
          "(at 4,096: 82.5 / 114.9); 18432 x 4096 stays with the library, 213.7 against 220.6", act=True),
