@@ -123,6 +123,19 @@ __global__ void token_shift_mix_vec_kernel(const T* h, const float* __restrict__
 #define WKV_PRODUCERS 128
 #define WKV_WIDE_PRODUCERS 256
 
+// A value as a staging thread keeps it until it is put down: in a register of its own (halves of one would have to be packed and unpacked).
+template <typename T> struct WkvRaw;
+template <> struct WkvRaw<float> {
+    typedef float R;
+    static __device__ __forceinline__ R load(const float* p) { return *p; }
+    static __device__ __forceinline__ float value(R r) { return r; }
+};
+template <> struct WkvRaw<bf16> {
+    typedef uint32_t R;
+    static __device__ __forceinline__ R load(const bf16* p) { return *reinterpret_cast<const unsigned short*>(p); }
+    static __device__ __forceinline__ float value(R r) { return __uint_as_float(r << 16); }
+};
+
 template <int G>
 __device__ __forceinline__ float wkv_tree_sum(float (&q)[G]) {
 #pragma unroll
@@ -172,7 +185,8 @@ __global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* r
     float* S = state + (int64_t)slot * state_stride + (int64_t)head * N * N;
     const int n_stages = (row1 - row0 + TB - 1) / TB;
 
-    T fr[PER], fk[PER], fv[PV];          // a staging thread's share of one stage, on its way (as it was read: a conversion would wait for it)
+    typedef WkvRaw<T> Raw;
+    typename Raw::R fr[PER], fk[PER], fv[PV];          // a staging thread's share of one stage, on its way (as it was read: a conversion would wait for it)
     float fz[PER];
     auto fetch = [&](int at_stage) {
         const int t0 = row0 + at_stage * TB;
@@ -181,28 +195,28 @@ __global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* r
             // every fetch is made, from an address inside the sequence's rows, so that none waits for another;
             // rows past the sequence's last are not used, channels past the head's last are zeroed in `put`
             const int64_t at = (int64_t)min(t0 + ptb + x * TSTEP, row1 - 1) * ld + (int64_t)head * N + min(pi, N - 1);
-            fr[x] = r[at];
-            fk[x] = k[at];
+            fr[x] = Raw::load(r + at);
+            fk[x] = Raw::load(k + at);
             fz[x] = z[at];
         }
 #pragma unroll
         for (int x = 0; x < PV; ++x) {
             const int e = pt + x * PRODUCERS, t = e / WKV_CB, c = e % WKV_CB;
-            fv[x] = v[(int64_t)min(t0 + t, row1 - 1) * ld + (int64_t)head * N + min(j0 + c, N - 1)];
+            fv[x] = Raw::load(v + (int64_t)min(t0 + t, row1 - 1) * ld + (int64_t)head * N + min(j0 + c, N - 1));
         }
     };
     auto put = [&](int buf) {
 #pragma unroll
         for (int x = 0; x < PER; ++x) {
             const int t = ptb + x * TSTEP;
-            rs[buf][t][pi] = pi < N ? to_f32(fr[x]) : 0.f;
-            ks[buf][t][pi] = pi < N ? to_f32(fk[x]) : 0.f;
+            rs[buf][t][pi] = pi < N ? Raw::value(fr[x]) : 0.f;
+            ks[buf][t][pi] = pi < N ? Raw::value(fk[x]) : 0.f;
             ws[buf][t][pi] = pi < N ? expf(-expf(fz[x] + w0r)) : 0.f;
         }
 #pragma unroll
         for (int x = 0; x < PV; ++x) {
             const int e = pt + x * PRODUCERS, c = e % WKV_CB;
-            vs[buf][e / WKV_CB][c] = j0 + c < N ? to_f32(fv[x]) : 0.f;
+            vs[buf][e / WKV_CB][c] = j0 + c < N ? Raw::value(fv[x]) : 0.f;
         }
     };
     auto write_out = [&](int at_stage, int buf) {       // the results of a stage the working threads are done with
