@@ -134,14 +134,22 @@ __global__ void attention_rows_kernel(const T* q, T* __restrict__ out, PagedCach
 // value at a time) and reads every row once per item; here a block of 4 warps copies a tile's rows to shared memory, 16 bytes at a
 // time, and a warp takes 4 items.  Tiles still begin at each row's first visible key, lanes own the same keys and every sum runs in
 // the plain kernel's order, so the bits are its bits: with a window the rows of a block begin up to 15 keys apart, and a tile
-// in shared memory holds that many more.  Rows of one sequence at consecutive positions go together; others in turn.
-// 700 rows of two sequences, 16 heads over 8 of 128: 1,561 -> 399 us.
+// in shared memory holds that many more.  Rows of one sequence at consecutive positions go together; others in turn, which
+// is slow, so a pass's table of tiles, where it is given, keeps a block's rows to one sequence.
+// 700 rows of two sequences, 16 heads over 8 of 128: 1,457 -> 395 us, at 500 earlier keys 5,068 -> 1,207; 16 sequences of 8 rows there 1,079 -> 416.
+struct ApTiles {                           // tiles of consecutive rows of one sequence (null: rows are cut up without regard to sequences)
+    const int32_t* seq;                    // [n] tile -> sequence
+    const int32_t* row0;                   // [n] tile -> first row
+    const int32_t* seq_first_row;          // [sequences + 1]
+    int32_t n, per_tile;                   // tiles, blocks that share one
+};
 #define AP_ITEMS 4                         // of a warp
 #define AP_ROWS (32 + 4 * AP_ITEMS - 1)    // of a tile
+#define AP_TILE_ROWS 64                    // rows of the tiles that 32-bit passes are cut into
 template <int NV>
 __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos,
                                                                int n_rows, int q_heads, float scale, int window, AttnExtra ex, int block_rows,
-                                                               int block_heads) {
+                                                               int block_heads, ApTiles tiles_of) {
     extern __shared__ __align__(16) float ap_smem[];
     const int hd = cache.head_dim, vd = ex.v_from_k > 0 ? ex.v_from_k : cache_v_dim(cache);
     const int kp = hd + 4, vp = ex.v_from_k > 0 ? kp : vd;                    // (a warp's 16-byte reads of 32 key rows meet no bank twice)
@@ -154,7 +162,15 @@ __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, f
     const int rep = q_heads / cache.kv_heads, chunks = (rep + block_heads - 1) / block_heads;
     const int kh = blockIdx.y / chunks, head0 = kh * rep + blockIdx.y % chunks * block_heads;
     const int heads = min(block_heads, (kh + 1) * rep - head0);
-    const int group = (gridDim.x - 1 - blockIdx.x) * block_rows, group_end = min(n_rows, group + block_rows);      // long rows first
+    const int block = gridDim.x - 1 - blockIdx.x;                            // (long rows first)
+    int group = block * block_rows, group_end = n_rows, group_step = n_rows;
+    if (tiles_of.seq != nullptr) {
+        const int tile = block / tiles_of.per_tile, seq = tiles_of.seq[tile];
+        const bool cut = tile + 1 < tiles_of.n && tiles_of.seq[tile + 1] == seq;        // the sequence goes on in the next tile
+        group = tiles_of.row0[tile] + block % tiles_of.per_tile * block_rows;
+        group_end = cut ? tiles_of.row0[tile + 1] : tiles_of.seq_first_row[seq + 1];
+        group_step = tiles_of.per_tile * block_rows;
+    }
     const int64_t v_plane = (int64_t)cache.kv_heads * cache.page_size * hd;
     const int64_t q_ld = ex.q_ld > 0 ? ex.q_ld : (int64_t)q_heads * hd;
     const float* base = (const float*)cache.base;
@@ -163,11 +179,12 @@ __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, f
         if (ex.chunk > 0) lo = max(lo, pos - pos % ex.chunk);
         return lo;
     };
-    for (int first = group; first < group_end;) {
+    for (; group < group_end; group += group_step)
+    for (int first = group, last_row = min(group_end, group + block_rows); first < last_row;) {
         // rows first .. first + n - 1: one sequence, consecutive positions, first keys close enough for one tile
         const int slot = row_slot[first], pos0 = row_pos[first], lo0 = first_key(pos0);
         int n = 1, tiles = (pos0 - lo0) / 32 + 1;
-        while (first + n < group_end && row_slot[first + n] == slot && row_pos[first + n] == pos0 + n && first_key(pos0 + n) - lo0 < 4 * AP_ITEMS) {
+        while (first + n < last_row && row_slot[first + n] == slot && row_pos[first + n] == pos0 + n && first_key(pos0 + n) - lo0 < 4 * AP_ITEMS) {
             tiles = max(tiles, (pos0 + n - first_key(pos0 + n)) / 32 + 1);
             ++n;
         }
@@ -182,7 +199,7 @@ __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, f
         float m[AP_ITEMS], l[AP_ITEMS], acc[AP_ITEMS][NV];
 #pragma unroll
         for (int i = 0; i < AP_ITEMS; ++i) {
-            const int it = warp * AP_ITEMS + i;
+            const int it = i * 4 + warp;
             const bool live = it < n * heads;
             pos[i] = live ? pos0 + it / heads : -1;
             lo[i] = live ? first_key(pos[i]) : lo0;
@@ -210,14 +227,23 @@ __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, f
             float s[AP_ITEMS];
 #pragma unroll
             for (int i = 0; i < AP_ITEMS; ++i) s[i] = 0.f;
-            const float* qw = qs + warp * AP_ITEMS * hd;
-            if (spread == 0) {
+            const float* qw = qs + warp * hd;                   // (item i of the warp: 4 i rows on)
+            if (n * heads <= 4) {                               // an item per warp at most
+                const float* kr = ks + min(lane + lo[0] - lo0, n_keys - 1) * kp;
+                for (int d = 0; d < hd; d += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(kr + d), q4 = *reinterpret_cast<const float4*>(qw + d);
+                    s[0] = fmaf(q4.x, k4.x, s[0]);
+                    s[0] = fmaf(q4.y, k4.y, s[0]);
+                    s[0] = fmaf(q4.z, k4.z, s[0]);
+                    s[0] = fmaf(q4.w, k4.w, s[0]);
+                }
+            } else if (spread == 0) {
                 const float* kr = ks + min(lane, n_keys - 1) * kp;
                 for (int d = 0; d < hd; d += 4) {
                     const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
 #pragma unroll
                     for (int i = 0; i < AP_ITEMS; ++i) {
-                        const float4 q4 = *reinterpret_cast<const float4*>(qw + i * hd + d);
+                        const float4 q4 = *reinterpret_cast<const float4*>(qw + 4 * i * hd + d);
                         s[i] = fmaf(q4.x, k4.x, s[i]);
                         s[i] = fmaf(q4.y, k4.y, s[i]);
                         s[i] = fmaf(q4.z, k4.z, s[i]);
@@ -231,7 +257,7 @@ __global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, f
                 for (int d = 0; d < hd; d += 4) {
 #pragma unroll
                     for (int i = 0; i < AP_ITEMS; ++i) {
-                        const float4 k4 = *reinterpret_cast<const float4*>(kr[i] + d), q4 = *reinterpret_cast<const float4*>(qw + i * hd + d);
+                        const float4 k4 = *reinterpret_cast<const float4*>(kr[i] + d), q4 = *reinterpret_cast<const float4*>(qw + 4 * i * hd + d);
                         s[i] = fmaf(q4.x, k4.x, s[i]);
                         s[i] = fmaf(q4.y, k4.y, s[i]);
                         s[i] = fmaf(q4.z, k4.z, s[i]);
@@ -324,7 +350,8 @@ static size_t ap_smem_bytes(int hd, int vd, bool v_from_k) {
 
 // float32 queries, cache and results; keys of up to 512 and values of up to 256 values, both multiples of four; no kept first keys.
 X0NE_API int x0ne_attention_prompt_f32(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos, int n_rows,
-                                       int q_heads, float scale, int window, AttnExtra ex, cudaStream_t stream) {
+                                       int q_heads, float scale, int window, AttnExtra ex, const int32_t* tile_seq, const int32_t* tile_row0, int n_tiles,
+                                       const int32_t* seq_first_row, cudaStream_t stream) {
     X0NE_REQUIRE(n_rows >= 0 && q_heads > 0 && cache.kv_heads > 0 && q_heads % cache.kv_heads == 0,
                  "attention: %d q heads over %d kv heads", q_heads, cache.kv_heads);
     const int hd = cache.head_dim, vd = ex.v_from_k > 0 ? ex.v_from_k : cache_v_dim(cache), rep = q_heads / cache.kv_heads;
@@ -333,10 +360,18 @@ X0NE_API int x0ne_attention_prompt_f32(const float* q, float* out, PagedCache ca
                      q_ld % 4 == 0 && cache.page_stride % 4 == 0 && ((((uintptr_t)q) | ((uintptr_t)cache.base)) & 15) == 0,
                  "attention: keys of %d and values of %d, or what is asked of them, are not for the kernel of several rows", hd, vd);
     if (n_rows == 0) return 0;
-    const int block_heads = rep < 4 * AP_ITEMS ? rep : 4 * AP_ITEMS, block_rows = 4 * AP_ITEMS / block_heads;
+    const int block_heads = rep < 4 * AP_ITEMS ? rep : 4 * AP_ITEMS;
     const int64_t chunks = (rep + block_heads - 1) / block_heads;
+    // fewer rows to a block (down to an item per warp) while that does not give more blocks than multiprocessors: 16 rows of 16 heads of 64 at
+    // 500 keys 373 us in 16 blocks, 274 in 64
+    int block_rows = 4 * AP_ITEMS / block_heads;
+    while (block_rows > 1 && block_rows * block_heads > 4 && 2 * ((n_rows + block_rows - 1) / block_rows) * chunks * cache.kv_heads <= x0ne_sm_count()) block_rows /= 2;
     X0NE_REQUIRE(chunks * cache.kv_heads <= 65535, "attention: too many heads");
-    const dim3 grid((unsigned)((n_rows + block_rows - 1) / block_rows), (unsigned)(chunks * cache.kv_heads));
+    X0NE_REQUIRE(tile_seq == nullptr || (n_tiles > 0 && tile_row0 != nullptr && seq_first_row != nullptr), "attention: %d tiles, or their rows are missing", n_tiles);
+    const ApTiles tiles{tile_seq, tile_row0, seq_first_row, n_tiles, AP_TILE_ROWS / block_rows};       // (larger tiles: their blocks come round again)
+    const int64_t blocks = tile_seq != nullptr ? (int64_t)n_tiles * tiles.per_tile : (n_rows + block_rows - 1) / block_rows;
+    X0NE_REQUIRE(blocks <= 0x7fffffff, "attention: too many tiles");
+    const dim3 grid((unsigned)blocks, (unsigned)(chunks * cache.kv_heads));
     const size_t smem = ap_smem_bytes(hd, vd, ex.v_from_k > 0);
     static OncePerDevice configured;
     if (configured.need()) {
@@ -346,9 +381,9 @@ X0NE_API int x0ne_attention_prompt_f32(const float* q, float* out, PagedCache ca
         }
         configured.done();
     }
-    if (vd <= 64) x0ne_launch(attention_prompt_kernel<2>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
-    else if (vd <= 128) x0ne_launch(attention_prompt_kernel<4>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
-    else x0ne_launch(attention_prompt_kernel<8>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads);
+    if (vd <= 64) x0ne_launch(attention_prompt_kernel<2>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads, tiles);
+    else if (vd <= 128) x0ne_launch(attention_prompt_kernel<4>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads, tiles);
+    else x0ne_launch(attention_prompt_kernel<8>, grid, dim3(128), smem, stream, q, out, cache, row_slot, row_pos, n_rows, q_heads, scale, window, ex, block_rows, block_heads, tiles);
     X0NE_LAUNCH_CHECK();
 }
 

@@ -235,7 +235,7 @@ _SIGNATURES = {
     "x0ne_glu_clipped": [_P, _P, _I, _I, _I, _F, _F, _F, _P],
     "x0ne_kv_write_blend": [_P, _I, _I, _I, _I, _P, _P, _I, None, _P, _P, _I, _P],
     "x0ne_latent_prepare": [_P, _I, _I, _I, _P, _L, _P, _F, _P, _F, _P, _I, _P, _I, _I, _I, _I, None, _P, _P, _I, _I, _P],
-    "x0ne_attention_prompt_f32": [_P, _P, None, _P, _P, _I, _I, _F, _I, "ex", _P],
+    "x0ne_attention_prompt_f32": [_P, _P, None, _P, _P, _I, _I, _F, _I, "ex", _P, _P, _I, _P, _P],
     "x0ne_attention_rows_ex": [_P, _P, _I, None, _P, _P, _I, _I, _F, _I, "ex", _P],
     "x0ne_gemm_f32_nt_batched": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _L, _L, _L, _P],
     "x0ne_attention_flex_prefill": [_P, _P, None, _P, _P, _I, _P, _P, _P, _I, _F, _I, "ex", _P],
@@ -648,10 +648,12 @@ def qk_norm_rope_kv_write(qkv: torch.Tensor, q_norm: Optional[torch.Tensor], k_n
 
 def attention_rows(q: torch.Tensor, out: torch.Tensor, cache: PagedCacheArg, row_slot: torch.Tensor,
                    row_pos: torch.Tensor, n_rows: int, q_heads: int, scale: float, window: int = 0,
-                   extra: Optional[AttnExtraArg] = None, prompt: bool = False) -> None:
+                   extra: Optional[AttnExtraArg] = None, prompt: bool = False, tiles: Optional[tuple] = None) -> None:
     """The plain attention kernel: keys up to 2,048 wide, values up to 512, any window (0 = none), and
     what `extra` asks for (see `attn_extra`).  With `extra.q_ld` the queries are rows of a wider buffer.  `prompt`: sequences bring
-    several rows, one after the other; in 32-bit a kernel in which they share the reading of their keys gives the same bits."""
+    several rows, one after the other; in 32-bit a kernel in which they share the reading of their keys gives the same bits.
+    `tiles`: (tile -> sequence, tile -> first row, number of tiles, sequence -> first row) of the pass, so that no block of that kernel
+    walks one sequence after the other."""
     lib = _lib("core")
     _need(out, torch.float32 if extra is not None and extra.out_f32 else q.dtype, "attention output")
     _need(row_slot, torch.int32, "row slots")
@@ -669,8 +671,11 @@ def attention_rows(q: torch.Tensor, out: torch.Tensor, cache: PagedCacheArg, row
     ex = extra if extra is not None else AttnExtraArg()
     if prompt and q.dtype == torch.float32 and cache.head_dim % 4 == 0 and cache.head_dim <= 512 and vd % 4 == 0 and 0 < vd <= 256 and ex.keep_first == 0 \
             and ex.q_ld % 4 == 0 and cache.page_stride % 4 == 0 and q.data_ptr() % 16 == 0 and (cache.base or 0) % 16 == 0:
+        tile_seq, tile_row0, n_tiles, seq_first_row = tiles or (None, None, 0, None)
+        for t in (tile_seq, tile_row0, seq_first_row) if tiles else ():
+            _need(t, torch.int32, "tiles")
         _check(lib, lib.x0ne_attention_prompt_f32(_ptr(q), _ptr(out), cache, _ptr(row_slot), _ptr(row_pos), n_rows, q_heads, scale, window, ex,
-                                                  _stream()), "attention_rows")
+                                                  _ptr(tile_seq), _ptr(tile_row0), n_tiles, _ptr(seq_first_row), _stream()), "attention_rows")
     elif extra is None:
         _check(lib, lib.x0ne_attention_rows(_ptr(q), _ptr(out), dtype_tag(q.dtype), cache, _ptr(row_slot),
                                             _ptr(row_pos), n_rows, q_heads, scale, window,
