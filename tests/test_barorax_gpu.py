@@ -557,7 +557,7 @@ def test_scan_of_many_rows_of_few_and_one_token_steps_give_the_same_bits(inner, 
     first = [T * s for s in range(n_seqs + 1)]
     every = (slice(0, n_seqs * T), sum(([s] * T for s in slots), []), list(range(T)) * n_seqs, first, slots, n_seqs, inner, n, taps)
     got = []
-    for known in (dict(), dict(max_rows=T)):
+    for known in (dict(form=1), dict(form=2)):
         state = start.clone()
         _, y = run_mixer(ops, xz, w, b, dt_raw, dt_bias, A, bc, D, state, *every, **known)
         got.append((y, state))
@@ -602,7 +602,7 @@ def test_passes_of_few_rows_and_a_sequence_cut_across_every_kernel(n):
     state = torch.zeros((len(lens), inner * (n + taps - 1)), device=DEV)
     slots = list(range(len(lens)))
     u, y = run_mixer(ops, xz, w, b, dt_raw, dt_bias, A, bc, D, state, slice(0, sum(lens)), sum(([s] * k for s, k in zip(slots, lens)), []),
-                     sum((list(range(k)) for k in lens), []), first, slots, len(lens), inner, n, taps, max_rows=16)
+                     sum((list(range(k)) for k in lens), []), first, slots, len(lens), inner, n, taps, form=2)
     for s in slots:
         rows = slice(first[s], first[s + 1])
         check(u[rows], y[rows], state[s], list(range(first[s], first[s + 1])), 2e-5)
@@ -610,9 +610,9 @@ def test_passes_of_few_rows_and_a_sequence_cut_across_every_kernel(n):
     xz, w, b, dt_raw, dt_bias, A, bc, D = scan_inputs(g, sum(cuts), inner, n, taps, torch.bfloat16)
     state = torch.zeros((2, inner * (n + taps - 1)), device=DEV)
     at, parts = 0, []
-    for k in cuts:
+    for i, k in enumerate(cuts):
         parts.append(run_mixer(ops, xz, w, b, dt_raw, dt_bias, A, bc, D, state, slice(at, at + k), [1] * k, list(range(at, at + k)), [0, k], [1], 1, inner, n, taps,
-                               max_rows=k, one_token=k == 1))
+                               form=1 + i % 2, one_token=k == 1))
         at += k
     check(torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts]), state[1], list(range(at)), 1e-4)
 

@@ -216,7 +216,7 @@ _SIGNATURES = {
     "x0ne_gemm_bf16_skinny_tcgen05_act": [_P, _P, _I, _P, _I, _I, _I, _I, _I, _P, _I, _F, _P],
     "x0ne_diff_heads": [_P, _P, _L, _P, _I, _I, _I, _I, _F, _F, _F, _P],
     "x0ne_causal_conv_silu": [_P, _L, _I, _P, _P, _P, _L, _L, _P, _P, _P, _I, _I, _I, _P],
-    "x0ne_selective_scan": ["ssm", _I, _I, _I, _P],
+    "x0ne_selective_scan": ["ssm", _I, _I, _I, _L, _I, _I, _P],
     "x0ne_add2_group_rmsnorm": [_P, _P, _P, _P, _P, _I, _P, _I, _I, _I, _F, _P],
     "x0ne_open_pass": [_P, _P, _I, _P, _I, _P, _F, _P, _I, _I, _I, _P],
     "x0ne_head_norm_kv_write": [_P, _I, _I, _I, _I, _P, _P, _F, _F, _I, _I, _P, _I, None, _P, _P, _I, _P],
@@ -1505,20 +1505,17 @@ def causal_conv_silu(xz: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Ten
                                           _stream()), "causal_conv_silu")
 
 
-SSM_FEW_ROWS = 16        # (csrc/ssm.cu: selective_scan_launch)
-
-
 def selective_scan(u: torch.Tensor, xz: torch.Tensor, z_col: int, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor], A: torch.Tensor,
                    bc: torch.Tensor, b_col: int, c_col: int, D: Optional[torch.Tensor], out: torch.Tensor, state: torch.Tensor,
                    conv_off: int, taps: int, seq_first_row: torch.Tensor, seq_slot: torch.Tensor, n_seqs: int,
-                   one_token: bool = False, max_rows: int = 0) -> None:
+                   one_token: bool = False, max_rows: int = 0, n_rows: int = 0, form: int = 0) -> None:
     """Per sequence and channel, token by token over the sequence's rows, from and into its state row (S [channels, N] at
     0, the convolution's last taps - 1 inputs at conv_off): dt = softplus(dt_raw + dt_bias); S = exp(dt A) S + dt u B;
     out = (S . C + D u) * silu(z).  u, xz (the convolution's input at column 0, z at z_col) and out in the activation type;
     dt_raw, A (negative), bc (B at b_col, C at c_col), D, state float32.  `one_token`: every sequence brings one row (a decode
     step); the same bits, from a form of the kernel without idle places.
-    `max_rows`: the most rows a sequence brings, where that is known (0: it is not); it chooses the kernel of bfloat16 runs, with the
-    same bits.  (In bfloat16 runs the number of sequences and channels may choose the order of a token's sum; in float32 runs nothing does.)"""
+    `n_rows` (0: all of u's), `max_rows`: the rows of all sequences together, and the most that one of them brings, where that is known (0: it is
+    not); they choose the kernel of bfloat16 runs, with the same bits.  `form` names one of the two for comparisons (1: staged, 2: the other).  (In bfloat16 runs the number of sequences and channels may choose the order of a token's sum; in float32 runs nothing does.)"""
     lib = _lib("core")
     for t, what in ((u, "scan input"), (xz, "projection"), (out, "scan output")):
         _need(t, u.dtype, what)
@@ -1534,7 +1531,8 @@ def selective_scan(u: torch.Tensor, xz: torch.Tensor, z_col: int, dt_raw: torch.
     arg = SsmArg(_ptr(u), _ptr(xz), xz.shape[-1], int(z_col), _ptr(dt_raw), _ptr(dt_bias), _ptr(A), _ptr(bc), bc.shape[-1], int(b_col),
                  int(c_col), _ptr(D), _ptr(out), _ptr(state), state.stride(0), int(conv_off), _ptr(seq_first_row), _ptr(seq_slot),
                  int(channels), int(N), int(taps))
-    _check(lib, lib.x0ne_selective_scan(arg, dtype_tag(u.dtype), n_seqs, 1 if one_token else 2 if 0 < max_rows <= SSM_FEW_ROWS else 0, _stream()), "selective_scan")
+    _check(lib, lib.x0ne_selective_scan(arg, dtype_tag(u.dtype), n_seqs, 1 if one_token else 0, int(n_rows) or u.shape[0], int(max_rows), int(form),
+                                        _stream()), "selective_scan")
 
 
 # ---------------------------------------------------------------------------------------------

@@ -20,9 +20,6 @@
 #define SSM_THREADS 128    // per block of the scan: channels x the threads that share a channel's states
 #define SSM_TC 32          // tokens staged at a time
 #define SSM_STAGERS 256    // staging threads of the bfloat16 scan
-#define SSM_MANY_ROWS 0    // what a scan is told of the rows its sequences bring: nothing, one each, at most 16 each
-#define SSM_ONE_ROW 1
-#define SSM_FEW_ROWS 2
 #define SSM_MAX_TAPS 16
 
 // exp(a * b) for a * b <= 0, closer than the library's exponential (whose error of up to two units in the last place, met
@@ -806,13 +803,29 @@ static int ssm_split(bool bf16_run, int64_t n_seqs, int64_t channels, int N, int
     return 16;
 }
 
+// Whether a bfloat16 run of several rows per sequence takes the staged scan: its blocks of 384 threads, two to a multiprocessor, go through 32
+// tokens at a time, the other kernel's of 128 through 4.  In the units of one full wave of staged blocks a sequence of r rows costs the GPU
+// 2.75 + 1.75 us per stage staged, and 0.6 + 0.113 us per row in the other; a sequence alone takes at least its own stages, or 2.3 + 0.32 us per
+// row, and the other sequences hold the longest one up a little.  (Constants fitted to 351 launches of 1 to 64 sequences, 2,048 to 8,192 channels of
+// 8 to 32 states; the choice is the faster kernel in all but seven, and within 11 % there.)  At 4,096 channels of 16, staged against the other: one
+// sequence of 9 / 64 / 512 rows 4.3 / 7.6 / 40.8 us against 4.5 / 12.6 / 84.8; 16 of 16 / 33 / 64 rows 25.7 / 39.4 / 48.1 against 17.7 / 31.6 / 51.1; 64 of 4 / 40 rows
+// 84.3 / 174 against 31.4 / 144; 63 of one row beside one of 64 78.9 against 42.2.
+static bool ssm_staged_ahead(int64_t n_seqs, int64_t rows, int64_t max_rows, int64_t channels, int split, int64_t sm_count) {
+    const double avg = (double)rows / (double)n_seqs, longest = max_rows > avg ? (double)(max_rows < rows ? max_rows : rows) : avg;
+    const double rest = n_seqs > 1 ? ((double)rows - longest) / (double)(n_seqs - 1) : 0.0;          // rows of the other sequences
+    const double wave = (double)((channels * split + SSM_THREADS - 1) / SSM_THREADS) / (double)(2 * sm_count);         // a sequence's share of one
+    const double waves = (double)n_seqs * wave, part = waves > 1.0 ? ceil(waves) / waves : 1.0;      // (staged: the last wave may be part empty)
+    auto staged = [](double r) { return 2.75 + 1.75 * (r / SSM_TC + 0.5); };
+    const double s_rest = (double)(n_seqs - 1) * wave * staged(rest), f_rest = (double)(n_seqs - 1) * wave * (0.6 + 0.113 * rest);
+    const double s_busy = part * (s_rest + wave * staged(longest)), s_alone = staged(longest) + 0.4 * s_rest;
+    const double f_busy = f_rest + wave * (0.6 + 0.113 * longest), f_alone = 2.3 + 0.32 * longest + 0.4 * f_rest;
+    return (s_busy > s_alone ? s_busy : s_alone) < (f_busy > f_alone ? f_busy : f_alone);
+}
+
 template <typename T>
-static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int rows, cudaStream_t stream) {
-    const bool one_token = rows == SSM_ONE_ROW;
+static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int one_token, int64_t n_rows, int max_rows, int form, cudaStream_t stream) {
     const int split = ssm_split(sizeof(T) == 2, n_seqs, a.channels, a.N, sm_count);
-    // sequences of a few rows stay with the kernel of 128 threads a block, of which many fit on a multiprocessor: 16 sequences of 9 /
-    // 13 / 20 rows, a layer of 4,096 channels, 64.0 / 74.4 / 93.0 us with it, 74.3 / 82.3 / 80.1 staged; one sequence of 9: 39.4 and 39.7
-    if (sizeof(T) == 2 && rows == SSM_MANY_ROWS && a.N <= 32) {
+    if (sizeof(T) == 2 && !one_token && a.N <= 32 && (form == 1 || (form == 0 && ssm_staged_ahead(n_seqs, n_rows, max_rows, a.channels, split, sm_count)))) {
         const int per = SSM_THREADS / split;
         const dim3 sgrid((unsigned)((a.channels + per - 1) / per), (unsigned)n_seqs), sblock(SSM_THREADS + SSM_STAGERS);
         if (split == 8) {
@@ -858,8 +871,9 @@ static int selective_scan_launch(const SsmArgs& a, int n_seqs, int sm_count, int
     X0NE_LAUNCH_CHECK();
 }
 
-// `rows`: what is known of the sequences' rows (SSM_*_ROW*).
-X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int rows, cudaStream_t stream) {
+// `one_token`: every sequence brings one row.  `n_rows`: the rows of all sequences together; `max_rows`: the most one of them brings (0: not
+// known).  `form`: the kernel of a bfloat16 run with several rows per sequence, which have the same bits (0: by the rule above, 1: staged, 2: the other).
+X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int one_token, int64_t n_rows, int max_rows, int form, cudaStream_t stream) {
     X0NE_REQUIRE(n_seqs >= 0 && n_seqs <= 65535 && a.channels > 0 && a.N > 0 && a.N <= 128 && a.taps >= 1 && a.taps <= SSM_MAX_TAPS,
                  "selective_scan: %d sequences, %d channels of %d states (at most %d), %d taps", n_seqs, a.channels, a.N, 128, a.taps);
     X0NE_REQUIRE(a.conv_off >= (int64_t)a.channels * a.N && a.state_stride >= a.conv_off + (int64_t)(a.taps - 1) * a.channels,
@@ -868,7 +882,7 @@ X0NE_API int x0ne_selective_scan(SsmArgs a, int dt, int n_seqs, int rows, cudaSt
                      a.b_col + a.N <= a.bc_ld && a.c_col + a.N <= a.bc_ld, "selective_scan: columns lie outside their rows");
     if (n_seqs == 0) return 0;
     const int sms = x0ne_sm_count();
-    if (dt == X0NE_F32) return selective_scan_launch<float>(a, n_seqs, sms, rows, stream);
-    if (dt == X0NE_BF16) return selective_scan_launch<bf16>(a, n_seqs, sms, rows, stream);
+    if (dt == X0NE_F32) return selective_scan_launch<float>(a, n_seqs, sms, one_token, n_rows, max_rows, form, stream);
+    if (dt == X0NE_BF16) return selective_scan_launch<bf16>(a, n_seqs, sms, one_token, n_rows, max_rows, form, stream);
     X0NE_REQUIRE(false, "selective_scan: unknown dtype tag %d", dt);
 }
