@@ -61,3 +61,17 @@ def test_pass_tables_match_the_restatement(seed):
             assert np.array_equal(s[row, :upto], want_t[row, :upto]), (row, r0, r1)
     with pytest.raises(ops.KernelError, match="plan_pass"):
         ops.plan_pass(slots, starts, first_row, tokens, 0, total, want_sorted, tile_rows, total, torch.zeros((9, 1), dtype=torch.int32))
+
+
+@pytest.mark.parametrize("tokens", [[5], [1, 2, 3], [True, 2], [np.int32(4), 2], ["5"], [5.7], (3, 4), np.arange(3), [2 ** 63], [None], [[1, 2]], [[1], [2, 3]], [],
+                                    [torch.tensor([5])], [torch.tensor(5), 6], torch.tensor([7, 8]), [1, "x"]])
+def test_token_ids_are_read_and_refused_as_numpy_does(tokens):
+    from x0ne_engine_b200.engine.engine import _token_ids
+
+    def read(f):
+        try:
+            got = f(tokens)
+            return got.dtype, got.tolist()
+        except Exception as e:      # noqa: BLE001
+            return type(e)
+    assert read(_token_ids) == read(lambda t: np.asarray(t, dtype=np.int64))

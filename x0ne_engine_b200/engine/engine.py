@@ -51,9 +51,9 @@ def padded_rows(n: int) -> int:
 
 
 def _token_ids(tokens) -> np.ndarray:
-    """A sequence's token ids as int64.  Lists of Python ints, what callers hold, go through `array`: 9,456 ids in 0.15 ms against
-    0.45 through NumPy's own reading of lists; anything else is NumPy's to read."""
-    if type(tokens) is list:
+    """A sequence's token ids as int64.  Lists of Python ints, what callers hold, go through `array`: 9,456 ids in 0.12 ms against
+    0.24 through NumPy's own reading of lists (0.30 and 0.38 on a slower host); anything else is NumPy's to read."""
+    if type(tokens) is list and tokens and type(tokens[0]) is int:
         try:
             return np.frombuffer(array("q", tokens), dtype=np.int64)
         except (TypeError, OverflowError):
