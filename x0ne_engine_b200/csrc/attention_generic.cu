@@ -146,8 +146,10 @@ struct ApTiles {                           // tiles of consecutive rows of one s
 #define AP_ITEMS 4                         // of a warp
 #define AP_ROWS (32 + 4 * AP_ITEMS - 1)    // of a tile
 #define AP_TILE_ROWS 64                    // rows of the tiles that 32-bit passes are cut into
+// (Four blocks of keys and values of 128 fit the shared memory of a multiprocessor to the kilobyte: a 129th register per thread would leave three, 406 ->
+// 474 us for two sequences of 249 and 451 rows.)
 template <int NV>
-__global__ void __launch_bounds__(128) attention_prompt_kernel(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos,
+__global__ void __launch_bounds__(128, NV <= 4 ? 4 : 2) attention_prompt_kernel(const float* q, float* out, PagedCache cache, const int32_t* row_slot, const int32_t* row_pos,
                                                                int n_rows, int q_heads, float scale, int window, AttnExtra ex, int block_rows,
                                                                int block_heads, ApTiles tiles_of) {
     extern __shared__ __align__(16) float ap_smem[];
