@@ -123,14 +123,16 @@ __global__ void token_shift_mix_vec_kernel(const T* h, const float* __restrict__
 #define WKV_PRODUCERS 128
 #define WKV_WIDE_PRODUCERS 256
 
-// A value as a staging thread keeps it until it is put down: in a register of its own (halves of one would have to be packed and unpacked).
-template <typename T> struct WkvRaw;
-template <> struct WkvRaw<float> {
-    typedef float R;
-    static __device__ __forceinline__ R load(const float* p) { return *p; }
-    static __device__ __forceinline__ float value(R r) { return r; }
+// A value as a staging thread keeps it until it is put down (a conversion at once would wait for it).  Two bfloat16 values share a register, or
+// each has one of its own: sharing costs instructions, which launches of many blocks feel (16 sequences of 10 tokens 27.5 us, 25.5 without; 64 of 20
+// 139.6 and 131.7), and registers, which a launch that waits for latencies feels (the layer of one sequence of 2,048 tokens takes 1.1 % longer with one
+// each).
+template <typename T, bool SHARED> struct WkvRaw {
+    typedef T R;
+    static __device__ __forceinline__ R load(const T* p) { return *p; }
+    static __device__ __forceinline__ float value(R r) { return to_f32(r); }
 };
-template <> struct WkvRaw<bf16> {
+template <> struct WkvRaw<bf16, false> {
     typedef uint32_t R;
     static __device__ __forceinline__ R load(const bf16* p) { return *reinterpret_cast<const unsigned short*>(p); }
     static __device__ __forceinline__ float value(R r) { return __uint_as_float(r << 16); }
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(2 * NB + PRODUCERS) wkv_scan_kernel(const T* r
     float* S = state + (int64_t)slot * state_stride + (int64_t)head * N * N;
     const int n_stages = (row1 - row0 + TB - 1) / TB;
 
-    typedef WkvRaw<T> Raw;
+    typedef WkvRaw<T, (U_ > 1)> Raw;
     typename Raw::R fr[PER], fk[PER], fv[PV];          // a staging thread's share of one stage, on its way (as it was read: a conversion would wait for it)
     float fz[PER];
     auto fetch = [&](int at_stage) {
