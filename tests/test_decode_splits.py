@@ -79,19 +79,18 @@ def test_unknown_capacity_falls_back_to_a_margin(monkeypatch):
     assert 1 <= s <= 8 and 64 * s <= 296
 
 
-@pytest.mark.parametrize("n_rows,n_seqs,heads,kv_heads,hd,visible,decode,shared", [
-    (2, 1, 16, 8, 128, 500, False, True), (15, 1, 16, 8, 128, 15, False, False), (16, 1, 16, 8, 128, 16, False, True), (700, 2, 16, 8, 128, 500, False, True), (30, 2, 16, 8, 128, 32, False, False),
-    (32, 32, 16, 8, 128, 500, True, False), (33, 32, 16, 16, 64, 500, False, False), (33, 32, 16, 16, 128, 500, False, True), (64, 16, 16, 16, 64, 500, False, True),
-    (63, 16, 16, 16, 64, 500, False, False),
+@pytest.mark.parametrize("n_rows,n_seqs,visible,decode,shared", [
+    (2, 1, 500, False, True), (31, 1, 31, False, False), (32, 1, 32, False, True), (63, 2, 64, False, False), (64, 2, 64, False, True), (63, 2, 65, False, True),
+    (33, 32, 500, False, True), (32, 32, 500, True, False), (2, 1, 0, False, False),
 ])
-def test_rows_of_a_32_bit_pass_share_their_keys_where_that_was_measured_ahead(n_rows, n_seqs, heads, kv_heads, hd, visible, decode, shared):
+def test_rows_of_a_32_bit_pass_share_their_keys_where_that_was_measured_ahead(n_rows, n_seqs, visible, decode, shared):
     from types import SimpleNamespace
     from x0ne_engine_b200.parts.attention import prompt_form, visible_keys
     table = object()
     ctx = SimpleNamespace(decode=decode, n_seqs=n_seqs, tile_seq=table, tile_row0=table, n_tiles=3, seq_first_row=table, max_context=700)
-    got = prompt_form(ctx, n_rows, heads, kv_heads, hd, visible)
+    got = prompt_form(ctx, n_rows, visible)
     assert got["prompt"] is shared and got["tiles"] == (table, table, 3, table)
     ctx.n_tiles = 0
-    assert prompt_form(ctx, n_rows, heads, kv_heads, hd, visible)["tiles"] is None
+    assert prompt_form(ctx, n_rows, visible)["tiles"] is None
     extra = SimpleNamespace(chunk=100, keep_first=8)
     assert visible_keys(ctx, 0) == 700 and visible_keys(ctx, 50) == 50 and visible_keys(ctx, 50, extra) == 58 and visible_keys(ctx, 0, extra) == 100

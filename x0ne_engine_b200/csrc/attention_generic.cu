@@ -136,7 +136,7 @@ __global__ void attention_rows_kernel(const T* q, T* __restrict__ out, PagedCach
 // the plain kernel's order, so the bits are its bits: with a window the rows of a block begin up to 15 keys apart, and a tile
 // in shared memory holds that many more.  Rows of one sequence at consecutive positions go together; others in turn, which
 // is slow, so a pass's table of tiles, where it is given, keeps a block's rows to one sequence.
-// 700 rows of two sequences, 16 heads over 8 of 128: 1,457 -> 395 us, at 500 earlier keys 5,068 -> 1,207; 16 sequences of 8 rows there 1,079 -> 416.
+// 700 rows of two sequences, 16 heads over 8 of 128: 1,457 -> 337 us, at 500 earlier keys 5,093 -> 1,170; 16 sequences of 8 rows there 1,085 -> 457.
 struct ApTiles {                           // tiles of consecutive rows of one sequence (null: rows are cut up without regard to sequences)
     const int32_t* seq;                    // [n] tile -> sequence
     const int32_t* row0;                   // [n] tile -> first row

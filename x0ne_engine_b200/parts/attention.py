@@ -13,14 +13,13 @@ from .base import MIXERS, CacheNeed, Mixer
 from .linear import Linear
 
 
-def prompt_form(ctx, n_rows: int, q_heads: int, kv_heads: int, head_dim: int, visible: int) -> dict:
+def prompt_form(ctx, n_rows: int, visible: int) -> dict:
     """How a 32-bit pass runs the plain attention: a warp per (row, head), or rows that share the reading of their keys (the same bits).  The
-    second is behind where there is little to share: single tokens (one warp has it all), a few rows each that see a tile of keys at most (16 q heads
-    over 8 of 128, 16 sequences of two or four rows from position 0: 6.7 and 9.8 us against 12.3 and 12.4; one of 16 rows 18.8 against 13.4), and narrow
-    heads of their own over sequences of a row or two (16 heads of 64, 31 sequences of one row and one of two at 500 keys: 479 against 665).  Elsewhere
-    it is ahead (16 over 8 of 128 at 500 keys: one sequence of 2 / 64 / 300 rows 476 / 743 / 2,512 us against 260 / 352 / 637; 31 of one row and one
-    of 64 1,015 against 503)."""
-    shared = not ctx.decode and (visible > 32 or n_rows >= 16 * ctx.n_seqs) and (q_heads > kv_heads or head_dim >= 128 or n_rows >= 4 * ctx.n_seqs)
+    second is behind where there is little to share: single tokens (one warp has it all), and few rows each that see a tile or two of keys (16 q
+    heads over 8 of 128, 16 sequences of two or four rows from position 0: 6.7 and 9.5 us against 12.8 and 13.4).  Elsewhere it is ahead (at 500
+    keys one sequence of 2 / 64 / 300 rows 475 / 742 / 2,525 us against 276 / 361 / 665, 31 of one row and one of 64 1,023 against 526; 16 heads of 64
+    over as many there 601 against 506)."""
+    shared = not ctx.decode and (visible > 64 or n_rows >= 32 * ctx.n_seqs)
     tiles = (ctx.tile_seq, ctx.tile_row0, ctx.n_tiles, ctx.seq_first_row) if ctx.tile_seq is not None and ctx.n_tiles > 0 else None
     return dict(prompt=shared, tiles=tiles)
 
@@ -36,7 +35,7 @@ def run_attention(ctx, q, out, view, n_rows, q_heads, scale, window):
     shape, else the plain kernel (which is also the whole 32-bit path)."""
     if not ops.fast_attention_takes(view, q.dtype):
         ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window,
-                           **prompt_form(ctx, n_rows, q_heads, view.kv_heads, view.head_dim, visible_keys(ctx, window)))
+                           **prompt_form(ctx, n_rows, visible_keys(ctx, window)))
     elif ctx.decode:
         # up to 8 splits merge inside a thread-block cluster and need no scratch; several clusters
         # per (sequence, kv head) leave one partial result each in a scratch of the workspace
@@ -91,7 +90,7 @@ def run_attention_ex(ctx, q, out, view, n_rows, q_heads, scale, window, extra):
     shape, else the plain kernel (which is also the whole 32-bit path)."""
     if not ops.attention_flex_takes(view, q.dtype, extra.v_from_k, ctx.decode):
         ops.attention_rows(q, out, view, ctx.row_slot, ctx.row_pos, n_rows, q_heads, scale, window, extra,
-                           **prompt_form(ctx, n_rows, q_heads, view.kv_heads, view.head_dim, visible_keys(ctx, window, extra)))
+                           **prompt_form(ctx, n_rows, visible_keys(ctx, window, extra)))
     elif ctx.decode:
         visible = visible_keys(ctx, window, extra)
         splits = flex_decode_splits(ctx, n_rows, view.kv_heads, q_heads, visible)
