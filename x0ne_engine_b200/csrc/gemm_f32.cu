@@ -83,10 +83,11 @@ __global__ void __launch_bounds__(256) gemm_f32_nt_kernel(const float* A, const 
 //
 // Many rows: a tile of BM x BN outputs, TM x TN per thread (its rows and columns in pieces of four, so that a warp's 16-byte reads of shared
 // memory meet no bank twice), 16 values of k at a time in two buffers, the next ones on their way to registers meanwhile; with AHEAD
-// the next k's values are read while the current one's products are made.  Bound by the multiply-adds and the waits between
-// them (72 TFLOP/s; cuBLAS' float32 product reaches 54).  700 rows against W 4096 x 2048 / 2048 x 2048 / 12288 x 2048 / 2048 x 6144:
-// 556 / 287 / 1203 / 870 us with the kernel above, 338 / 196 / 899 / 576 here; 100 rows 218 / 165 / 309 / 667 -> 88 / 70 / 206 / 205.
-// Two columns per instruction (fma.rn.f32x2) changed nothing: 345-403 / 321 / 996 / 881.
+// the next k's values are read while the current one's products are made.  700 rows against W 4096 x 2048 / 2048 x 2048 / 12288 x 2048 /
+// 2048 x 6144: 556 / 287 / 1203 / 870 us with the kernel above, 338 / 196 / 899 / 576 here; 100 rows 218 / 165 / 309 / 667 -> 88 / 70 / 206 / 205.
+// That is 30 to 45 TFLOP/s, where the multiply-add units end at about 75 by count and clock: the rest is waits for shared memory and between
+// dependent multiply-adds.  cuBLAS' float32 product, which is free in its order, reaches 54 on 700 x 12288 x 2048 (656 us).
+// Two columns per instruction (fma.rn.f32x2) were slower on all four but the first: 345-403 / 321 / 996 / 881.
 template <int BM_, int BN_, int TM_, int TN_, bool AHEAD, int BLOCKS>
 __global__ void __launch_bounds__(BM_ / TM_ * (BN_ / TN_), BLOCKS) gemm_f32_tile_kernel(const float* A, const float* W, float* C, int M, int N, int K, int64_t lda,
                                                                                int64_t ldw, int64_t ldc, int64_t sa, int64_t sw, int64_t sc) {
@@ -183,9 +184,10 @@ __global__ void __launch_bounds__(BM_ / TM_ * (BN_ / TN_), BLOCKS) gemm_f32_tile
     }
 }
 
-// Few rows (at most 4 RM): bound by the bytes of W.  A block takes 32 outputs of every row, a thread one of them for RM rows; W's rows and
-// x stream through a ring of copies, FEW_K values of k a stage, and are read along k.  1 to 8 rows against W 4096 x 2048 / 12288 x 2048 /
-// 2048 x 6144: 215 / 305 / 650 us with the kernel above (a tile of 128 rows, a few blocks), 22 / 49 / 57 here; 64 rows 219 / 306 / 672 -> 84 / 187 / 175.
+// Few rows (at most 4 RM).  A block takes 32 outputs of every row, a thread one of them for RM rows; W's rows and x stream through a ring of
+// copies, FEW_K values of k a stage, and are read along k.  1 to 8 rows against W 4096 x 2048 / 12288 x 2048 / 2048 x 6144: 215 / 305 / 650 us with
+// the kernel above (a tile of 128 rows, a few blocks), 22 / 49 / 57 here; 64 rows 219 / 306 / 672 -> 84 / 187 / 175.  Bound by a block's walk along
+// k, not by the bytes of W (5 / 15 / 8 us): 1 to 8 rows take 19.5 us at K 2,048 for any N from 16 to 4,096 and 37 at K 4,096.
 #define FEW_K 64
 #define FEW_STAGES 4
 __device__ __forceinline__ void few_copy16(float* dst, const float* src, bool ok) {
