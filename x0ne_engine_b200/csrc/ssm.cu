@@ -807,7 +807,7 @@ static int ssm_split(bool bf16_run, int64_t n_seqs, int64_t channels, int N, int
 // tokens at a time, the other kernel's of 128 through 4.  In the units of one full wave of staged blocks a sequence of r rows costs the GPU
 // 2.75 + 1.75 us per stage staged, and 0.6 + 0.113 us per row in the other; a sequence alone takes at least its own stages, or 2.3 + 0.32 us per
 // row, and the other sequences hold the longest one up a little.  (Constants fitted to 351 launches of 1 to 64 sequences, 2,048 to 8,192 channels of
-// 8 to 32 states; the choice is the faster kernel in all but seven, and within 11 % there.)  At 4,096 channels of 16, staged against the other: one
+// 8 to 32 states; the choice is within 4 % of the faster kernel in all but ten, and within 11 % there.)  At 4,096 channels of 16, staged against the other: one
 // sequence of 9 / 64 / 512 rows 4.3 / 7.6 / 40.8 us against 4.5 / 12.6 / 84.8; 16 of 16 / 33 / 64 rows 25.7 / 39.4 / 48.1 against 17.7 / 31.6 / 51.1; 64 of 4 / 40 rows
 // 84.3 / 174 against 31.4 / 144; 63 of one row beside one of 64 78.9 against 42.2.
 static bool ssm_staged_ahead(int64_t n_seqs, int64_t rows, int64_t max_rows, int64_t channels, int split, int64_t sm_count) {
