@@ -50,6 +50,28 @@ def test_every_form_gives_the_same_bits(n, k):
     ops.check_tc_status(x.device)
 
 
+@pytest.mark.parametrize("n,k", [(4096, 2048), (12288, 2048), (2048, 6144)])
+def test_more_blocks_than_multiprocessors(n, k):
+    """Launches of several rounds of blocks, many of them one behind the other: a block of every form ends whatever order its warps end in."""
+    rows = 700
+    x, w = normal((rows, k), 7), normal((n, k), 8)
+    want = torch.zeros((rows, n), device=DEV)
+    product(x, w, want, rows, 16, 1)
+    at = torch.randint(0, rows, (40,), generator=torch.Generator().manual_seed(9)).to(DEV)
+    exact, size = x[at].double() @ w.double().T, x[at].double().abs() @ w.double().abs().T
+    assert bool(((want[at].double() - exact).abs() <= BOUND(k) * size).all())
+    for nx, cl in FORMS:
+        y = torch.full((rows + 1, n), 3.0, device=DEV)
+        for _ in range(20):
+            product(x, w, y, rows, nx, cl)
+        assert torch.equal(y[:rows], want) and bool((y[rows] == 3.0).all()), (nx, cl)
+    y = torch.zeros((rows, n), device=DEV)
+    for _ in range(1000):
+        ops.gemm_f32_nt(x, w, y, rows)
+    assert torch.equal(y, want)
+    ops.check_tc_status(x.device)
+
+
 def test_strided_batches():
     b, m, n, k = 3, 21, 150, 576
     a, w = normal((m, b, k), 3).transpose(0, 1), normal((b, n, k), 4)

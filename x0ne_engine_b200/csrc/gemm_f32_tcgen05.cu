@@ -33,6 +33,9 @@ template <int NX> struct SpConfig {
     static constexpr int BLOCKS = NX <= 32 ? 2 : 1;
     // Warps that split x.  Where registers run out (the adding warps hold up to 128 sums a thread), warpgroups trade them: 640 threads start
     // with 96 each, the adding 256 take GROW and the other 384 keep SHRINK (256 GROW + 384 SHRINK <= 640 x 96).
+    // The pool may be just as large as what is asked for, so nobody takes registers back before the adding warps are through with
+    // theirs: a barrier of all warps (of the cluster, or of the block alone) stands between every warp's first trade and its second, and behind it
+    // the adding warps give back without waiting for anything.
     static constexpr int X_WARP = NX >= 64 ? 16 : 14, X_WARPS = NX >= 64 ? 4 : 2, THREADS = 32 * (X_WARP + X_WARPS);
     static constexpr int START = 96, GROW = NX >= 96 ? 168 : 136, SHRINK = NX >= 96 ? 48 : 64;
     static constexpr bool SHIFT_REGS = NX >= 64;
@@ -93,6 +96,9 @@ __device__ __forceinline__ bool sp_irregular(float v) {
     const uint32_t e = __float_as_uint(v) & 0x7fffffffu;
     return e >= 0x7f800000u || e - 1u < ((127u - 60u) << 23) - 1u;
 }
+
+// All warps of the block, from either side of the split into roles.
+template <int THREADS> __device__ __forceinline__ void sp_all_warps() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 
 // NX: rows of x per block.  CL: blocks of a cluster, each with 8 / CL parts of K.
 //
@@ -241,7 +247,10 @@ __global__ void __launch_bounds__(SpConfig<NX>::THREADS, SpConfig<NX>::BLOCKS) g
                 }
             }
             __syncwarp();
-            if constexpr (Cfg::SHIFT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::START));
+            if constexpr (Cfg::SHIFT_REGS) {
+                sp_all_warps<Cfg::THREADS>();
+                asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::START));
+            }
         }
     } else {
         if constexpr (Cfg::SHIFT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::SHRINK));
@@ -398,7 +407,10 @@ __global__ void __launch_bounds__(SpConfig<NX>::THREADS, SpConfig<NX>::BLOCKS) g
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
         __syncwarp();
-        if constexpr (Cfg::SHIFT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::START));
+        if constexpr (Cfg::SHIFT_REGS) {
+            if (CL == 1) sp_all_warps<Cfg::THREADS>();
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::START));
+        }
     }
     if constexpr (CL > 1) {
         __syncwarp();
