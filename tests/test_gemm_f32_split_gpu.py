@@ -1,5 +1,5 @@
-"""The float32 product on the tensor cores (operands split into two TF32 values): every form of it against float64 and against each
-other, and the values that have no split."""
+"""The float32 product on the tensor cores (operands split into three bfloat16 values): every form of it against float64 and against each
+other, rows of a single term, and the values that have no split."""
 import pytest
 import torch
 
@@ -7,10 +7,11 @@ from x0ne_engine_b200.csrc import ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-FORMS = [(16, 1), (16, 2), (16, 4), (16, 8), (32, 1), (32, 4), (32, 8), (64, 1), (64, 4), (64, 8), (96, 1), (128, 1), (128, 8)]
-# Of a sum of |x w|: 2^-23 for what the split leaves out of each product (two low halves cut off at 2^-12 times 2^-11, and their own
-# product), 2^-22 for the tensor core cutting off 4 sums of a slab of 32 values, and 2^-24 for each float32 addition of a slab or a part.
-BOUND = lambda k: 2.0 ** -23 + 2.0 ** -22 + (-(-k // 256) + 8) * 2.0 ** -24
+FORMS = [(16, 1), (16, 2), (16, 4), (16, 8), (32, 1), (32, 4), (32, 8), (64, 1), (64, 4), (64, 8), (96, 1)]
+# Of a sum of |x w|: 2^-32 for what the split leaves out of each product (its two lowest parts, 2^-16 times 2^-16), 2^-22 for the tensor core cutting
+# off the sums of a slab of 32 values (two products of 16), 2^-24 for each float32 addition of a slab or a part, and of the part's small products
+# (2^-7 of the sum) 2^-23 for each of their 10 sums a slab.
+BOUND = lambda k: 2.0 ** -32 + 2.0 ** -22 + (-(-k // 256) + 10) * 2.0 ** -24 + 10 * -(-k // 256) * 2.0 ** -30
 
 
 def product(x, w, y, m, nx=0, cl=0):
@@ -47,6 +48,44 @@ def test_every_form_gives_the_same_bits(n, k):
     y = torch.zeros((rows, n), device=DEV)
     ops.gemm_f32_nt(odd, w, y, rows)
     assert torch.equal(y, want)
+    ops.check_tc_status(x.device)
+
+
+def test_rows_of_a_single_term():
+    """Nothing is lost where there is nothing to add: an identity gives x back, and a product alone is rounded once (2^-24, and 2^-29 in the
+    sum of its small parts), in a row of zeros and beside terms that do not reach its last bit."""
+    k = 640
+    x = normal((33, k), 10)
+    for nx, cl in FORMS:
+        y = torch.zeros((33, k), device=DEV)
+        product(x, torch.eye(k, device=DEV), y, 33, nx, cl)
+        assert torch.equal(y, x), (nx, cl)
+    w = normal((200, k), 11)
+    at = torch.arange(33, device=DEV) * 19
+    alone, beside = torch.zeros((33, k), device=DEV), normal((33, k), 12) * 2.0 ** -40
+    for rows, slack in ((alone, 0.0), (beside, 2.0 ** -24)):
+        rows[torch.arange(33), at] = normal((33,), 13) + 3.0
+        y = torch.zeros((33, 200), device=DEV)
+        ops.gemm_f32_nt(rows, w, y, 33)
+        exact = rows.double() @ w.double().T
+        term = (rows[torch.arange(33), at].double()[:, None] * w.double()[:, at].T).abs()
+        rest = rows.double().abs() @ w.double().abs().T - term
+        assert bool(((y.double() - exact).abs() <= (2.0 ** -24 + 2.0 ** -29) * exact.abs() + rest + slack * term).all())
+    ops.check_tc_status(x.device)
+
+
+def test_operands_of_far_apart_sizes():
+    """Operands near the low end of the float32 range whose products are of ordinary size: no room for their last bits below."""
+    k = 512
+    x, w = normal((20, k), 14), normal((140, k), 15)
+    x[3], w[100:110] = x[3] * 2.0 ** -112, w[100:110] * 2.0 ** 90
+    x[4] *= 2.0 ** -130
+    want = x.double() @ w.double().T
+    size = x.double().abs() @ w.double().abs().T
+    for nx, cl in [(0, 0)] + FORMS:
+        y = torch.zeros((20, 140), device=DEV)
+        product(x, w, y, 20, nx, cl)
+        assert bool(((y.double() - want).abs() <= k * 2.0 ** -24 * size + k * 2.0 ** -149).all()), (nx, cl)
     ops.check_tc_status(x.device)
 
 
@@ -91,7 +130,7 @@ def test_values_without_a_split():
     ops.gemm_f32_nt(x, w, clean, 20)
     x[3, 7], x[4, 9], x[5] = float("inf"), float("nan"), 0.0
     x[6] *= 1e-38                                        # results of 1e-37, operands without room for a low half
-    x[7, 0], w[:, 0] = 3.4e38, 0.25                       # rounds to an infinite TF32 value
+    x[7, 0], w[:, 0] = torch.finfo(torch.float32).max, 0.25   # rounds to an infinite TF32 value
     w[11, 2] = -float("inf")
     y = torch.zeros((20, 70), device=DEV)
     ops.gemm_f32_nt(x, w, y, 20)

@@ -277,9 +277,8 @@ extern "C" int x0ne_gemm_f32_split(const float* A, const float* W, float* C, int
                                    int form, int* status, cudaStream_t stream);       // gemm_f32_tcgen05.cu
 
 // K from which the tensor cores take a product.  The rule may look at W alone, so that a row's bits do not depend on what is computed with
-// it.  8 / 64 rows on multiply-add units against tensor cores: K 256 4.3 / 12.7 us and 5.3 / 7.0 (N 4096), 3.5 / 9.6 and 4.1 / 4.9 (N 1024); K 512
-// 7.3 / 23.4 and 6.5 / 8.6, 5.8 / 16.7 and 4.5 / 5.4; K 2,048 24.7 / 88 and 11.6 / 15.6 (N 4096).  Their error against 64 bits is the
-// smaller one from K 100 on (2-norm over 2-norm: K 132 2.1e-7 and 1.4e-7, 512 4.1e-7 and 1.4e-7, 2,048 8.1e-7 and 1.5e-7, 6,144 1.4e-6 and 1.7e-7).
+// it.  8 / 64 rows on multiply-add units against tensor cores: K 512 7.0 / 24.6 us and 7.5 / 10.2 (N 4096), 6.4 / 17.2 and 6.3 / 6.8 (N 1024); K 1,024 10.8 /
+// 31.5 and 6.5 / 8.1 (N 1024); K 2,048 24.4 / 89 and 13.3 / 18.6 (N 4096).
 #define F32_SPLIT_K 512
 
 // `batch` products of one shape: product b reads A + b sa and W + b sw and writes C + b sc.  `status`: one int in device memory, zero before the

@@ -954,7 +954,7 @@ def _f32_status(k: int, device) -> int:
 
 def gemm_f32_nt(a: torch.Tensor, w: torch.Tensor, c: torch.Tensor, m: int) -> None:
     """c[:m] = a[:m] @ w.T in float32, every output's sum in an order that K alone decides: one chain of multiply-adds, and from K 512 on
-    split operands on the tensor cores (gemm_f32_tcgen05.cu)."""
+    operands cut into three bfloat16 values each, without loss, on the tensor cores (gemm_f32_tcgen05.cu)."""
     lib = _lib("core")
     _need(a, torch.float32, "gemm input")
     _need(w, torch.float32, "gemm weight")
