@@ -1,0 +1,49 @@
+"""Sequences taken on one stream and stepped on another, and what an engine leaves behind it when it goes."""
+import gc
+
+import pytest
+import torch
+
+from helpers import model_folder, prompts_for
+
+pytestmark = pytest.mark.gpu
+LATE = 100_000_000          # cycles of a stream that is busy with something else
+
+
+def engine(dtype):
+    from x0ne_engine_b200 import Engine
+    return Engine.from_folder(model_folder("B", dtype), dtype=dtype, max_tokens=2048)
+
+
+@pytest.mark.parametrize("taken_on", ["a stream", "the default stream"])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_a_sequence_taken_behind_other_work_of_another_stream(dtype, taken_on):
+    eng = engine(dtype)
+    ids, more = prompts_for(eng.vocab_size, [150, 3], seed=2)
+    first = eng.new_sequence(160)
+    want = [eng.step([first], [ids]).clone(), eng.step([first], [more]).clone()]
+    torch.cuda.synchronize()
+    one = torch.cuda.Stream() if taken_on == "a stream" else torch.cuda.default_stream()
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(LATE)
+        slot = eng.new_sequence(160)
+    with torch.cuda.stream(other):
+        got = [eng.step([slot], [ids]), eng.step([slot], [more])]
+    torch.cuda.synchronize()
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    eng.cache.settle()
+    assert len(eng.cache._pushed) <= 1          # streams that are through are forgotten
+
+
+def test_an_engine_that_goes_waits_for_the_copies_out_of_its_pinned_tables():
+    eng = engine("float32")
+    slot = eng.new_sequence(64)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(LATE)
+    eng.step([slot], [[1, 2, 3]])
+    events = eng._stage_events
+    assert any(e is not None and not e.query() for e in events)
+    del eng
+    gc.collect()
+    assert all(e is None or e.query() for e in events)

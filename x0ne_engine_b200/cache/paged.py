@@ -88,8 +88,9 @@ class KVGroup:
         return True
 
     def push_row(self, slot: int) -> None:
-        """The slot's row of the page table to the device, ahead of whatever is launched next.  (A tensor copy of host memory waits for the
-        stream and costs the host 13 us a row; 16 prompts that arrive together push 16 rows before their first launch.)"""
+        """The slot's row of the page table to the device, ahead of whatever is launched next on this stream (`SequenceCache.settle` for
+        others).  (A tensor copy of host memory waits for the stream and costs the host 13 us a row; 16 prompts that arrive together push 16 rows
+        before their first launch.)"""
         if self.table.is_cuda:
             from ..csrc import ops
             row = 4 * self.table_stride
@@ -173,6 +174,39 @@ class SequenceCache:
                 elif src in self.states:
                     self.states[e] = self.states[src]
         self._reads = list(reads_cache_of)
+        self._pushed: Dict[int, Optional[torch.cuda.Event]] = {}         # by stream: behind the last rows and states that went out on it
+
+    # ---- streams
+    def _stream(self) -> int:
+        device = torch.device(self.device)
+        return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
+
+    def _note_push(self) -> None:
+        """Rows or states are on their way to the device on the current stream."""
+        if torch.device(self.device).type != "cuda":
+            return
+        stream = self._stream()
+        if stream == 0:
+            self._pushed[0] = None          # (the default stream is always there to be asked later: no event for every sequence)
+        else:
+            ev = self._pushed[stream] = torch.cuda.Event()
+            ev.record(torch.cuda.current_stream(self.device))
+
+    def settle(self) -> None:
+        """Puts what `acquire` and `ensure` sent on other streams ahead of what the current stream launches next."""
+        if not self._pushed:
+            return
+        here = self._stream()
+        for stream, ev in list(self._pushed.items()):
+            if stream == here:
+                continue
+            if ev is None:
+                ev = self._pushed[stream] = torch.cuda.Event()
+                ev.record(torch.cuda.default_stream(self.device))
+            if ev.query():
+                self._pushed.pop(stream, None)
+            else:
+                torch.cuda.current_stream(self.device).wait_event(ev)
 
     # ---- what parts see
     def kv_view(self, entry: int) -> PagedCacheArg:
@@ -223,6 +257,7 @@ class SequenceCache:
             g.push_row(slot)
         for t in {id(t): t for t in self.states.values()}.values():
             t[slot].zero_()
+        self._note_push()
         return slot
 
     def ensure(self, slot: int, tokens: int) -> None:
@@ -231,9 +266,13 @@ class SequenceCache:
             raise ValueError(f"slot {slot} is not held")
         if tokens > self.max_seq_len:
             raise CacheFull(f"slot {slot}: {tokens} tokens, a sequence holds at most {self.max_seq_len}")
+        pushed = False
         for g in self.groups:
             if g.ensure(slot, tokens):
                 g.push_row(slot)
+                pushed = True
+        if pushed:
+            self._note_push()
 
     def ensure_all(self, requests) -> None:
         """`ensure` for several (slot, tokens) at once: either all get their pages or none does."""

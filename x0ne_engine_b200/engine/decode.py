@@ -181,6 +181,7 @@ class DeviceBatch:
         """Queues one decode step for `live` and the copy of its picks to the host."""
         if live != self.live:
             self._compact(live)
+        self.engine.cache.settle()
         n = len(live)
         lengths = self.engine.cache.lengths
         bucket = context_bucket(max(int(lengths[self.slots[i]]) for i in live) + 1, self.engine.max_seq_len)

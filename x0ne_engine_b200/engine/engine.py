@@ -13,6 +13,7 @@ sequences of unequal length share a pass and padding never exists.
 """
 from __future__ import annotations
 
+import weakref
 from array import array
 from collections import OrderedDict
 from dataclasses import dataclass
@@ -88,6 +89,13 @@ class StepContext:
     sm_count: int = 0                              # multiprocessors of the device the pass runs on (set by the engine)
 
 
+def _last_copies(stage: List[torch.Tensor], events: List[Optional[torch.cuda.Event]]) -> None:
+    """Waits until nothing on the device reads `stage` any more."""
+    for ev in events:
+        if ev is not None:
+            ev.synchronize()
+
+
 def require_gpu(device) -> torch.device:
     device = torch.device(device)
     if device.type != "cuda":
@@ -123,6 +131,8 @@ class Engine:
         self._stage = [torch.zeros((9, width), dtype=torch.int32).pin_memory() for _ in range(4)]
         self._stage_events: List[Optional[torch.cuda.Event]] = [None] * len(self._stage)
         self._stage_at = 0
+        # (copies out of the stage go past torch's own bookkeeping of pinned memory, so it outlives the last of them here)
+        weakref.finalize(self, _last_copies, self._stage, self._stage_events).atexit = False
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         # short bfloat16 prompt passes: padded to a few row counts, their launches kept as graphs
         self.replayable = self.model.replayable()
@@ -226,6 +236,7 @@ class Engine:
             self.cache.ensure_all([(s, st + n) for s, st, n in zip(slots, starts, lens)])
         except CacheFull as e:
             raise StepError(f"the cache has no room for this step: {e}") from None
+        self.cache.settle()
 
         total = int(flat.shape[0])
         first_row = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
