@@ -39,6 +39,7 @@ def test_a_sequence_taken_behind_other_work_of_another_stream(dtype, taken_on):
 def test_an_engine_that_goes_waits_for_the_copies_out_of_its_pinned_tables():
     eng = engine("float32")
     slot = eng.new_sequence(64)
+    eng.step([slot], [[1, 2, 3]])           # (what is loaded and allocated once is there)
     torch.cuda.synchronize()
     torch.cuda._sleep(LATE)
     eng.step([slot], [[1, 2, 3]])
