@@ -67,6 +67,44 @@ def test_chunks_against_float64(lens, heads, decay):
     assert torch.isfinite(o3[:at]).all() and (torch.equal(o3[:max(0, at - 64)], o[:max(0, at - 64)]))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", ["r", "k", "v", "z", "state"])
+def test_values_that_are_not_finite_reach_what_they_reach_token_by_token(where, value):
+    """One value in the middle of the second of four chunks (or in the state the sequence starts from)."""
+    g = torch.Generator(device=DEV)
+    g.manual_seed(17)
+    rows, heads, width = 230, 2, 128
+    normal = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    rkv = {s: normal(rows, 128).bfloat16() for s in "rkv"}
+    h, z, w0, u = normal(rows, width).bfloat16(), normal(rows, 128) * 0.1, torch.full((128,), 0.01, device=DEV).log(), normal(128)
+    state = normal(1, heads * 4096 + width)
+    if where == "state":
+        state[0, 64 * 5 + 7] = value
+    elif where == "z":
+        z[100, 70] = value
+    else:
+        rkv[where][100, 70] = value
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    scratch = torch.empty(((rows // 64 + 1) * heads * ops.WKV_CHUNK_UNIT,), device=DEV)
+    got = []
+    for chunks in (False, True):
+        st, o = state.clone(), torch.zeros(rows, 128, device=DEV)
+        args = (rkv["r"], rkv["k"], rkv["v"], z, w0, u, h, o, st, i32([0, rows]), i32([0]), 1)
+        if chunks:
+            ops.wkv_chunk_scan(*args, rows, rows, heads, scratch)
+        else:
+            ops.wkv_scan(*args, heads, 64)
+        got.append((o, st))
+    (o1, s1), (o2, s2) = got
+    assert not bool(torch.isfinite(o1).all()) or where == "z"           # (a decay of zero is finite)
+    assert torch.equal(torch.isfinite(o1), torch.isfinite(o2)) and torch.equal(torch.isfinite(s1), torch.isfinite(s2))
+    if value != value:
+        assert torch.equal(o1.isnan(), o2.isnan()) and torch.equal(s1.isnan(), s2.isnan())
+    fine = torch.isfinite(o1)
+    assert float((o1 - o2)[fine].abs().max()) <= 1e-4 * float(o1[fine].abs().max())     # (two orders of float32 sums of a few hundred terms)
+
+
 def test_the_choice():
     def ctx(n_seqs, longest, decode=False):
         return types.SimpleNamespace(decode=decode, n_seqs=n_seqs, max_seq_rows=longest, sm_count=148)

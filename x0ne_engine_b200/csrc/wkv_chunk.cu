@@ -14,7 +14,8 @@
 // the token-by-token kernel.  Inside a block of 8 tokens A is made by multiply-adds over running products; everything else is a
 // product of matrices on mma.sync m16n8k8 with every float32 operand as two TF32 numbers (hi hi + hi lo + lo hi; v is exact as one), float32 sums.
 // States, decays and sums are float32.  The order of sums differs from the token-by-token kernels', which stay for 32-bit runs, steps and short runs.
-// An infinite state or decay gives NaN where the token-by-token kernel may give an infinity (an infinity has no low half).
+// Infinities and NaN have no two halves (a NaN can even lose itself in the rounding): where a chunk of a head meets one, its products are
+// made by multiply-adds of the whole values instead, so that it reaches what it reaches in the token-by-token kernel.
 // The scan of one sequence of 2,048 tokens, 32 heads: 148 -> 84 us (sums 20, states 12, outputs 56 each alone), 16 heads 142 -> 54, 64 heads 249 -> 162; 16
 // sequences of 128, 32 heads 121 -> 80.  The outputs' kernel, which is most of it, uses 56 % of its issue slots and 57 % of shared memory's
 // wavefronts (two blocks of 16 warps a multiprocessor; eight warps with blocks of 16 tokens took 69 us).  Error against float64 (2-norm over 2-norm), walk / chunks: 515 tokens
@@ -95,11 +96,12 @@ __global__ void __launch_bounds__(WC_THREADS, 3) wkv_chunk_sums_kernel(WkvChunkA
         k[x] = to_f32(a.k[at]);
         v[x] = to_f32(a.v[at]);
     }
-    float all = 1.f;
+    float all = 1.f, odd = 0.f;          // odd: NaN once a value is not finite
 #pragma unroll
     for (int x = WC_B - 1; x >= 0; --x) {
         const int t = b * WC_B + x;
         vs[t][i] = t < nt ? v[x] : 0.f;
+        odd = fmaf(vs[t][i], 0.f, odd);
         k[x] = t < nt ? k[x] * all : 0.f;                  // (with the decays of the block's later tokens)
         all *= t < nt ? wc_decay(w[x], w0) : 1.f;
     }
@@ -110,12 +112,23 @@ __global__ void __launch_bounds__(WC_THREADS, 3) wkv_chunk_sums_kernel(WkvChunkA
     for (int x = WC_BLOCKS - 1; x > 0; --x)
         if (x > b) after *= block_decay[x][i];
 #pragma unroll
-    for (int x = 0; x < WC_B; ++x) kd[b * WC_B + x][i] = k[x] * after;
+    for (int x = 0; x < WC_B; ++x) {
+        kd[b * WC_B + x][i] = k[x] * after;
+        odd = fmaf(k[x] * after, 0.f, odd);
+    }
     float* unit = wc_unit(a, seq, row0, c, head);
     if (b == 0) unit[WC_N * WC_N + i] = after * all;
-    __syncthreads();
+    const bool plain = __syncthreads_and(odd == 0.f);
     const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, i0 = 16 * (warp & 3), j0 = 16 * (warp >> 2);
     float sum[2][4] = {}, acc[2][4] = {}, low[2][4] = {};
+    if (!plain) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll 1
+                for (int s = 0; s < nt; ++s) sum[n][e] = fmaf(kd[s][i0 + g + 8 * (e >> 1)], vs[s][j0 + 8 * n + 2 * t + (e & 1)], sum[n][e]);
+    } else
 #pragma unroll
     for (int s = 0; s < WC_L; s += 8) {
         uint32_t hi[4], lo[4];
@@ -212,6 +225,8 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
     const int vrow = tid / 8, vcol = tid % 8 * 8;
     uint4 vals = make_uint4(0, 0, 0, 0);           // what the last part needs, on its way from the start
     float4 st[2];
+    float odd = 0.f;                               // NaN once a value is not finite
+    bool plain;
     {
         const int i = tid % WC_N, b = tid / WC_N;
         const float w0 = a.w0[head * WC_N + i];
@@ -236,6 +251,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
             const int t = b * WC_B + x;
             w[x] = t < nt ? wc_decay(w[x], w0) : 1.f;
             if (t >= nt) r[x] = k[x] = 0.f;
+            odd = fmaf(r[x], 0.f, fmaf(k[x], 0.f, fmaf(w[x], 0.f, odd)));
             sh.in.w[t][i] = w[x];
             sh.in.r[t][i] = __float2bfloat16_rn(r[x]);         // (exact: they came as bfloat16)
             sh.in.k[t][i] = __float2bfloat16_rn(k[x]);
@@ -249,7 +265,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
             sh.in.kd[b * WC_B + x][i] = k[x] * later;
             later *= w[x];
         }
-        __syncthreads();
+        plain = __syncthreads_and(odd == 0.f);
         float earlier = 1.f;
 #pragma unroll
         for (int x = 0; x < WC_BLOCKS - 1; ++x)
@@ -301,6 +317,17 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
     {
         const int m = warp < 1 ? 0 : warp < 4 ? 1 : warp < 9 ? 2 : 3, sb = warp - m * m;
         float sum[1][4] = {}, acc[1][4] = {}, low[1][4] = {};
+        if (!plain) {
+#pragma unroll 1
+            for (int i = 0; i < WC_N; ++i) {
+                float f0 = 1.f;
+#pragma unroll 1
+                for (int b = sb + 1; b < 2 * m; ++b) f0 *= sh.block_decay[b][i];
+                const float f1 = sb < 2 * m ? f0 * sh.block_decay[2 * m][i] : 1.f;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sum[0][e] = fmaf(sh.rd[16 * m + g + 8 * (e >> 1)][i] * (e >= 2 ? f1 : f0), sh.in.kd[sb * WC_B + 2 * t + (e & 1)][i], sum[0][e]);
+            }
+        } else
 #pragma unroll
         for (int i = 0; i < WC_N; i += 8) {
             float f[2][2];                                      // [place][half of the targets]: the blocks between
@@ -324,30 +351,31 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
         for (int e = 0; e < 4; ++e)
             if (e >= 2 || sb < 2 * m) sh.A[16 * m + g + 8 * (e >> 1)][sb * WC_B + 2 * t + (e & 1)] = sum[0][e];
     }
-    __syncthreads();
     // values and state take the place of what A was made of
-    bool finite = true;
-    {
-        const uint32_t q[4] = {vals.x, vals.y, vals.z, vals.w};
+    const float value[8] = {__uint_as_float(vals.x << 16), __uint_as_float(vals.x & 0xffff0000u), __uint_as_float(vals.y << 16), __uint_as_float(vals.y & 0xffff0000u),
+                            __uint_as_float(vals.z << 16), __uint_as_float(vals.z & 0xffff0000u), __uint_as_float(vals.w << 16), __uint_as_float(vals.w & 0xffff0000u)};
+    const float from[8] = {st[0].x, st[0].y, st[0].z, st[0].w, st[1].x, st[1].y, st[1].z, st[1].w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) odd = fmaf(value[e], 0.f, fmaf(from[e], 0.f, odd));
+    plain = __syncthreads_and(odd == 0.f);
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) *reinterpret_cast<float2*>(&sh.of.v[vrow][vcol + e]) = make_float2(value[e], value[e + 1]);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        const int at = tid + x * WC_THREADS;
+        uint32_t hi[4], lo[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            finite = finite && (q[e] & 0x7f80u) != 0x7f80u && (q[e] & 0x7f800000u) != 0x7f800000u;
-            *reinterpret_cast<float2*>(&sh.of.v[vrow][vcol + 2 * e]) = make_float2(__uint_as_float(q[e] << 16), __uint_as_float(q[e] & 0xffff0000u));
+            wc_split(from[4 * x + e], hi[e], lo[e]);
+            if (!plain) hi[e] = __float_as_uint(from[4 * x + e]);
         }
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-            const int at = tid + x * WC_THREADS;
-            const float y[4] = {st[x].x, st[x].y, st[x].z, st[x].w};
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) wc_split(y[e], hi[e], lo[e]);
-            *reinterpret_cast<uint4*>(&sh.of.s[0][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(&sh.of.s[1][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
+        *reinterpret_cast<uint4*>(&sh.of.s[0][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(&sh.of.s[1][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
-    const bool plain = __syncthreads_and(finite);
+    __syncthreads();
     const int m = warp & 3, j0 = 16 * (warp >> 2);
     float sum[2][4] = {}, acc[2][4] = {}, low[2][4] = {};
+    if (plain)
 #pragma unroll
     for (int i = 0; i < WC_N; i += 8) {
         uint32_t hi[4], lo[4];
@@ -379,12 +407,16 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
             }
             wc_add(sum, acc, low);
         }
-    } else {                // a value that is not finite must not meet the zeros of the tokens before it
+    } else {                // (nor may a value that is not finite meet the zeros of the tokens before it)
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int target = 16 * m + g + 8 * (e >> 1), j = j0 + 8 * n + 2 * t + (e & 1);
+#pragma unroll 1
+                for (int i = 0; i < WC_N; ++i)
+                    sum[n][e] = fmaf(sh.rd[target][i] * sh.before[2 * m + (e >> 1)][i], __uint_as_float(sh.of.s[0][i][j]), sum[n][e]);
+#pragma unroll 1
                 for (int s = 0; s <= target; ++s) sum[n][e] = fmaf(sh.A[target][s], sh.of.v[s][j], sum[n][e]);
             }
     }
