@@ -45,6 +45,29 @@ def test_products_of_listed_pairs(which, n, k):
     assert err <= (2.0 ** -19 * k ** 0.5 if which == 1 else 2.0 ** -8)      # float32 sums of k products of unit size; one rounding to bfloat16
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("which,n", [(0, 264), (1, 264), (2, 512)])
+def test_results_that_do_not_start_on_16_bytes(which, n, pair):
+    experts, pairs, k = 2, 150, 64
+    g = torch.Generator().manual_seed(n)
+    a, w = torch.randn(pairs, k, generator=g).bfloat16().to(DEV), torch.randn(experts, n, k, generator=g).bfloat16().to(DEV)
+    tile = ops.MOE_TC_TILE_ROWS * (2 if pair else 1)
+    i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=DEV)
+    n_tiles = ops.moe_max_tiles(pairs, experts, tile)
+    offsets, listed, tiles, n_real = i32(experts + 1), i32(pairs), i32(n_tiles, 3), i32(1)
+    ops.moe_group(torch.randint(0, experts, (pairs, 1), generator=g, dtype=torch.int32).to(DEV), pairs, experts, offsets, listed, tiles, tile, n_real)
+    width, dtype = n // 2 if which == 2 else n, torch.float32 if which == 1 else torch.bfloat16
+    got = []
+    for first in (0, 1):
+        out = torch.full((pairs * width + 8,), 3.0, dtype=dtype, device=DEV)
+        ops.moe_product_tc(which, a, w, listed, tiles, n_real, n_tiles, out[first:first + pairs * width].view(pairs, width), pair)
+        assert bool((out[:first] == 3.0).all()) and bool((out[first + pairs * width:] == 3.0).all())
+        got.append(out[first:first + pairs * width].clone())
+    ops.check_tc_status(torch.device(DEV))
+    assert torch.equal(got[0], got[1])
+
+
 def test_the_choice():
     take = lambda pairs, experts, ff=1024: ops.moe_tc_in_pairs(pairs, experts, 2 * ff, 2048, ff, 148)
     assert take(4096, 16) and take(16384, 16) and take(8192, 8, 1792)

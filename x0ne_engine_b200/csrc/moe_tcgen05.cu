@@ -78,7 +78,7 @@ __device__ __forceinline__ void mt_results(uint32_t trow, void* out, int N, int 
         if (n >= N) break;                          // (uniform over the warp)
         float v[32];
         tc_ld32(trow + c * 32, v);
-        if (MODE == MT_DOWN && n + 32 <= N && N % 4 == 0) {
+        if (MODE == MT_DOWN && n + 32 <= N && N % 4 == 0 && (((uintptr_t)out) & 15) == 0) {
             // rows of 64 bytes, four lanes each: a thread's own row would go out in 16-byte pieces, 32 rows at a time
 #pragma unroll
             for (int h = 0; h < 32; h += 16) {
@@ -440,7 +440,6 @@ X0NE_API int x0ne_moe_product_tc(int which, const void* a, int64_t a_rows, const
     X0NE_REQUIRE(which != 2 || N % MT_BN == 0, "moe_product_tc: gated experts of %d rows (blocks of %d)", N, MT_BN);
     X0NE_REQUIRE(status != nullptr && n_real != nullptr, "moe_product_tc: no status word or no tile count");
     X0NE_REQUIRE((((uintptr_t)a | (uintptr_t)w) & 15) == 0, "moe_product_tc: operands are not 16-byte aligned");
-    X0NE_REQUIRE((((uintptr_t)out) & 15) == 0, "moe_product_tc: results are not 16-byte aligned");
     if (max_tiles == 0) return 0;
     CUtensorMap map_a, map_w;
     if (int e = x0ne_tc_make_map(&map_a, a, a_rows, K, MT_BM)) return e;
