@@ -731,7 +731,8 @@ flex_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const int mi = lane >> 3, r8 = lane & 7;
     for (int it = it_a, stage = 0; it <= it_b; ++it) {
         if ((have >> stage) & 1u) {
-            if (alive) alive = __all_sync(0xffffffffu, mbar_wait(&full[warp][stage], (phase >> stage) & 1u, status, 28));
+            alive = __all_sync(0xffffffffu, mbar_wait(&full[warp][stage], (phase >> stage) & 1u, status, 28));
+            if (!alive) break;
             phase ^= 1u << stage;
             const int lp = it < n_kept ? it : pg_lo + it - n_kept, jw = lp * FX_PAGE + 16 * warp;
             bf16* ks = mine + stage * stage_elems;
@@ -859,7 +860,10 @@ flex_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             l[h] = 1.f;
         }
     }
-    __syncthreads();    // every warp is done with its tiles
+    if (!alive)             // copies that nobody waited for must land before the block's memory is used again or given back
+        for (int i = 0; i < stages; ++i)
+            if ((have >> i) & 1u) mbar_wait(&full[warp][i], (phase >> i) & 1u, status, 28);
+    if (!__syncthreads_and(alive)) return;          // (every warp is done with its tiles; what the status word reports has no results)
     const int ps = sh.vdp + 2;
 #pragma unroll
     for (int h = 0; h < 2 * HT; ++h) {
