@@ -1,4 +1,4 @@
-"""Sequences taken on one stream and stepped on another, and what an engine leaves behind it when it goes."""
+"""Sequences taken on one stream and stepped on another, what an engine leaves behind it when it goes, and steps that do not wait."""
 import gc
 
 import pytest
@@ -48,3 +48,30 @@ def test_an_engine_that_goes_waits_for_the_copies_out_of_its_pinned_tables():
     del eng
     gc.collect()
     assert all(e is None or e.query() for e in events)
+
+
+def test_a_32_bit_step_returns_with_its_work_queued_and_the_next_one_reports():
+    from x0ne_engine_b200 import Engine, Qwen3Config
+    from x0ne_engine_b200.csrc import ops
+    cfg = Qwen3Config(hidden_size=512, intermediate_size=576, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=2, head_dim=64, vocab_size=128,
+                      max_position_embeddings=256, rms_norm_eps=1e-6, rope_theta=10000.0, tie_word_embeddings=False, dtype="float32")
+    eng = Engine.random(cfg, seed=3, dtype="float32", max_tokens=256)
+    slot = eng.new_sequence(64)
+    want = eng.step([slot], [[1, 2, 3]]).clone()
+    eng.free_sequence(slot)
+    slot = eng.new_sequence(64)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(LATE)
+    got, queued = eng.step([slot], [[1, 2, 3]]), torch.cuda.Event()
+    queued.record()
+    assert not queued.query()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    ops.gemm_tc_status(eng.device).fill_(1 << 20)           # as a wait that ran out leaves it
+    eng.step([slot], [[4]])
+    torch.cuda.synchronize()
+    with pytest.raises(ops.KernelError, match="an earlier step"):
+        eng.step([slot], [[5]])
+    eng.step([slot], [[5]])
+    torch.cuda.synchronize()
+    eng.step([slot], [[6]])

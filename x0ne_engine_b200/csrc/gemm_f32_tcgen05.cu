@@ -260,6 +260,9 @@ __global__ void __launch_bounds__(SpConfig<NX>::THREADS, SpConfig<NX>::BLOCKS) g
         if constexpr (CL > 1) {
 #pragma unroll
             for (int p = 0; p < OWN; ++p) add_part(sum[p], max(0, min(slabs, (rank * OWN + p + 1) * part) - min(slabs, (rank * OWN + p) * part)));
+            if (!ok)
+#pragma unroll
+                for (int c = 0; c < COLS; ++c) sum[0][c] = INFINITY;
             __syncwarp();
             asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
             asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // every block of the cluster is done with its tiles
@@ -287,13 +290,13 @@ __global__ void __launch_bounds__(SpConfig<NX>::THREADS, SpConfig<NX>::BLOCKS) g
             __syncwarp();
             asm volatile("bar.sync 2, %0;" ::"n"(256 + SPLITTERS) : "memory");
             const int large = sh->large_w[quarter * 32 + lane], n = n0 + quarter * 32 + lane;
-            if (n < a.N && ok) {
+            if (n < a.N) {
                 const float* w = a.W + (int64_t)z * a.sw + (int64_t)n * a.ldw;
 #pragma unroll
                 for (int c = 0; c < COLS; ++c) {
                     const int m = m0 + half * COLS + c;
                     if (m < a.M) {
-                        float v = sum[0][c];
+                        float v = ok ? sum[0][c] : INFINITY;          // (after a wait that ran out: as for results that are not finite)
                         if (sp_irregular(v, large, sh->large_x[half * COLS + c])) v = sp_chain(a.A + (int64_t)z * a.sa + (int64_t)m * a.lda, w, a.K);
                         a.C[(int64_t)z * a.sc + (int64_t)m * a.ldc + n] = v;
                     }

@@ -1197,8 +1197,46 @@ def check_tc_status(device) -> None:
     tc_used = False
     st = int(gemm_tc_status(device))
     if st != 0:
-        gemm_tc_status(device).zero_()
+        clear_tc_status(device)
         raise KernelError(describe_tc_status(st))
+
+
+_tc_watched = {}         # by device: where the status word goes in host memory, and the event behind that copy
+
+
+def watch_tc_status(device) -> None:
+    """`check_tc_status` for a caller that does not wait: the word is copied to the host behind what has been launched, and `check_watched_tc_status`
+    raises once it has arrived."""
+    global tc_used
+    if not tc_used:
+        return
+    tc_used = False
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    if idx not in _tc_watched:
+        _tc_watched[idx] = (torch.zeros(1, dtype=torch.int32).pin_memory(), torch.cuda.Event())
+    word, event = _tc_watched[idx]
+    word.copy_(gemm_tc_status(device), non_blocking=True)
+    event.record()
+
+
+def check_watched_tc_status(device) -> None:
+    """Raises if a status word that `watch_tc_status` asked for has arrived and is not zero; does not wait for one."""
+    word, event = _tc_watched.get(device.index if device.index is not None else torch.cuda.current_device(), (None, None))
+    if word is None or not event.query():
+        return
+    st = int(word)
+    if st != 0:
+        clear_tc_status(device)
+        raise KernelError("an earlier step: " + describe_tc_status(st))
+
+
+def clear_tc_status(device) -> None:
+    """After a report: the word is zero again, here and where a copy of it has gone."""
+    gemm_tc_status(device).zero_()
+    word, event = _tc_watched.get(device.index if device.index is not None else torch.cuda.current_device(), (None, None))
+    if word is not None:
+        event.synchronize()
+        word.zero_()
 
 
 def describe_tc_status(st: int) -> str:

@@ -205,9 +205,12 @@ class Engine:
         one).  Returns float32 [number wanted, vocab] in the order of the sequences and of `want`.
         All checks happen before the first launch; a refused step changes nothing.
         """
+        from ..csrc import ops
         n_seqs = len(slots)
         if n_seqs == 0:
             return torch.empty((0, self.vocab_size), dtype=torch.float32, device=self.device)
+        if self.dtype == torch.float32:
+            ops.check_watched_tc_status(self.device)
         if len(tokens) != n_seqs or (want is not None and len(want) != n_seqs):
             raise StepError("slots, tokens and want must have one entry per sequence")
         if len(set(slots)) != n_seqs:
@@ -263,8 +266,12 @@ class Engine:
             self._run_pass(step, r0, min(total, r0 + chunk), order, logits, decode)
         for s, n in zip(slots, lens):
             self.cache.lengths[s] += n
-        from ..csrc import ops
-        ops.check_tc_status(self.device)
+        # (a 32-bit step returns with its work queued: a wait that ran out in it is reported by the next step or by the decode loop; the products of
+        # such a block are made by multiply-adds)
+        if self.dtype == torch.float32:
+            ops.watch_tc_status(self.device)
+        else:
+            ops.check_tc_status(self.device)
         if repeat is not None:
             logits = logits[torch.from_numpy(repeat).to(self.device)]
         return logits
