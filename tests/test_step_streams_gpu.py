@@ -75,3 +75,22 @@ def test_a_32_bit_step_returns_with_its_work_queued_and_the_next_one_reports():
     eng.step([slot], [[5]])
     torch.cuda.synchronize()
     eng.step([slot], [[6]])
+
+
+def test_the_word_for_waits_is_there_before_a_capture():
+    from x0ne_engine_b200.csrc import ops
+    from x0ne_engine_b200.engine.workspace import Workspace
+    kept, ops._tc_status = ops._tc_status, {}
+    try:
+        ws = Workspace(8, torch.device("cuda:0"))
+        x, w, y = ws.buffer("x", (8, 512), torch.float32).normal_(), torch.randn(96, 512, device="cuda:0"), ws.buffer("y", (8, 96), torch.float32)
+        word = ops._tc_status[0]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.gemm_f32_nt(x, w, y, 8)
+        assert ops._tc_status[0] is word
+        word.fill_(1 << 20)
+        graph.replay()
+        assert int(word) == 1 << 20 and torch.allclose(y, x @ w.T, rtol=1e-4, atol=1e-3)          # (a replay leaves a report as it is)
+    finally:
+        ops._tc_status = kept

@@ -21,6 +21,10 @@ class Workspace:
         self.device = device
         self._bufs: Dict[str, torch.Tensor] = {}
         self.frozen = False
+        if torch.device(device).type == "cuda":
+            # the word the kernels report waits in is made, and zeroed, ahead of any capture: inside one it would belong to the graph
+            from ..csrc import ops
+            ops.gemm_tc_status(torch.device(device))
 
     def buffer(self, name: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         t = self._bufs.get(name)
