@@ -49,7 +49,7 @@ def test_chunks_against_float64(lens, heads, decay):
         want, last = exact(*args, u.double().view(heads, 64), S)
         size, grown = exact(*[x.abs() for x in args], u.double().abs().view(heads, 64), S.abs())
         # of a term: its decays, at most n of two functions (2^-22 each and the argument's own rounding, which the exponent scales) and a
-        # product each; split operands and sums of 16 in the tensor core 2^-20
+        # product each; sums of 16 in the tensor core and in float32 2^-20
         bound = 2.0 ** -20 + n * 2.0 ** -21 * (1 + 4 * decay)
         assert bool(((o[a:b].double().view(n, heads, 64) - want).abs() <= bound * size).all()), s
         assert bool(((state[slot, :heads * 4096].double().view(heads, 64, 64) - last).abs() <= bound * grown).all()), s

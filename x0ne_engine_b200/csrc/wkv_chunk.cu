@@ -10,16 +10,19 @@
 //   wkv_chunk_states   per value of a head's state, chunk after chunk: B is replaced by the state that the chunk starts from
 //   wkv_chunk_out      per (chunk, head): the outputs
 // Decays are products of numbers in [0, 1], taken inside blocks of 8 tokens and over whole blocks, never quotients or differences of
-// logarithms: nothing overflows, a factor that underflows belongs to a term that does, and a product of n decays is off by n roundings, as in
-// the token-by-token kernel.  Inside a block of 8 tokens A is made by multiply-adds over running products; everything else is a
-// product of matrices on mma.sync m16n8k8 with every float32 operand as two TF32 numbers (hi hi + hi lo + lo hi; v is exact as one), float32 sums.
-// States, decays and sums are float32.  The order of sums differs from the token-by-token kernels', which stay for 32-bit runs, steps and short runs.
-// Infinities and NaN have no two halves (a NaN can even lose itself in the rounding): where a chunk of a head meets one, its products are
+// logarithms: nothing overflows, a factor that underflows belongs to a term that does.  Inside a block of 8 tokens A is made by multiply-adds over
+// running products; A between blocks and the outputs are products of matrices on mma.sync m16n8k16 with every float32 operand as three bfloat16
+// numbers, which hold all of it (v is exact as one), the products of the largest parts in an accumulator of their own, added up in float32 every
+// 16 terms.  The tensor core cuts its sums off, so what is most of a result where decays are fast stays with multiply-adds: a chunk's own state is
+// walked, an output's own tile of 16 tokens added term by term.  States, decays and sums are float32, products of a whole block's decays are taken in
+// 64 bits and rounded once.  The order of sums differs from the token-by-token kernels', which stay for 32-bit runs, steps and short runs.
+// Infinities and NaN have no parts (a NaN can even lose itself in the rounding): where a chunk of a head meets one, its products are
 // made by multiply-adds of the whole values instead, so that it reaches what it reaches in the token-by-token kernel.
-// The scan of one sequence of 2,048 tokens, 32 heads: 148 -> 84 us (sums 20, states 12, outputs 56 each alone), 16 heads 142 -> 54, 64 heads 249 -> 162; 16
-// sequences of 128, 32 heads 121 -> 80.  The outputs' kernel, which is most of it, uses 56 % of its issue slots and 57 % of shared memory's
-// wavefronts (two blocks of 16 warps a multiprocessor; eight warps with blocks of 16 tokens took 69 us).  Error against float64 (2-norm over 2-norm), walk / chunks: 515 tokens
-// with slow decays 8.7e-7 / 8.3e-7, 430 in two sequences with fast ones 1.4e-7 / 1.4e-7, one chunk alone 1.7e-7 / 1.9e-7.
+// Error against 64 bits (2-norm over 2-norm; w0 a decay rate, mean of three seeds), outputs and states, walk -> here: one chunk, rate 1 7.8e-8 / 3.9e-8 -> 7.4e-8 /
+// 3.6e-8, rate 0.01 1.67e-7 / 1.90e-7 -> 1.63e-7 / 1.85e-7; four sequences of 128, rate 0.1 1.06e-7 / 8.7e-8 -> 1.06e-7 / 8.4e-8; 2,048 tokens, rate 0.01 2.31e-7 / 2.25e-7 ->
+// 2.17e-7 / 2.10e-7.  With two TF32 numbers to an operand and everything on the tensor core it was 9.5e-8 / 6.4e-8 in the first of these, 2.49e-7 / 2.24e-7 in the last.
+// The scan of one sequence of 2,048 tokens, 32 heads: 146 -> 107 us (91 in that other form), 16 heads 146 -> 68, 64 heads 251 -> 206; 16 sequences of 128, 32 heads
+// 124 -> 103.
 #include "common.cuh"
 
 #define WC_L 64                 // tokens of a chunk
@@ -28,8 +31,9 @@
 #define WC_N 64                 // channels of a head
 #define WC_THREADS 512
 #define WC_STATE_THREADS 256
-#define WC_PITCH_ROW 68         // floats between rows that fragments read along (8 rows x 4 places meet 32 banks)
-#define WC_PITCH_COL 72         // and across (4 rows x 8 places)
+#define WC_PITCH_ROW 72         // floats between rows that fragments read along (4 rows x 4 pairs meet 32 banks)
+#define WC_PITCH_COL 68         // and across (every second row of 4, 8 places)
+#define WC_PITCH_PAIR 72        // and of rows of pairs (4 rows x 8 places)
 #define WC_UNIT (WC_N * WC_N + WC_N)         // scratch floats of a chunk and head: B or the state, then the product of its decays
 
 struct WkvChunkArgs {
@@ -50,36 +54,36 @@ struct WkvChunkArgs {
 };
 
 __device__ __forceinline__ void wc_mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// x as two TF32 numbers: rounded (halves away from zero), and what is left
-__device__ __forceinline__ void wc_split(float x, uint32_t& hi, uint32_t& lo) {
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = (__float_as_uint(x - __uint_as_float(hi)) + 0x1000u) & 0xffffe000u;
+// two values as three bfloat16 each, exactly: x rounded, what is left of it rounded, and the rest (x in the lower halves)
+__device__ __forceinline__ void wc_split(float x, float y, uint32_t& a, uint32_t& b, uint32_t& c) {
+    auto pack = [&](uint32_t& to) { asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(to) : "f"(y), "f"(x)); };
+    auto less = [&](uint32_t by) {
+        x -= __uint_as_float(by << 16);
+        y -= __uint_as_float(by & 0xffff0000u);
+    };
+    pack(a);
+    less(a);
+    pack(b);
+    less(b);
+    pack(c);
 }
+// two float32 numbers that are bfloat16 numbers
+__device__ __forceinline__ uint32_t wc_pair(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
 __device__ __forceinline__ float wc_decay(float z, float w0) { return expf(-expf(z + w0)); }
 // where chunk c of a sequence that starts at row0 keeps its scratch (a sequence of n rows has ceil(n / 64) chunks, so no two meet)
 __device__ __forceinline__ float* wc_unit(const WkvChunkArgs& a, int seq, int row0, int c, int head) {
     return a.scratch + ((int64_t)(row0 / WC_L + seq + c) * a.heads + head) * WC_UNIT;
 }
 
-// Sums of products stay in the tensor core for 16 terms and are added up with rounding from there on (it cuts its sums off).
-template <int NT>
-__device__ __forceinline__ void wc_add(float (&sum)[NT][4], float (&acc)[NT][4], float (&low)[NT][4]) {
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            sum[n][e] += acc[n][e] + low[n][e];
-            acc[n][e] = low[n][e] = 0.f;
-        }
-}
-
-// B and the product of decays.  A thread takes one channel of one block of tokens, then a warp 16 key channels x 16 value channels.
+#define WC_CAREFUL 4            // tokens at a chunk's end whose roundings are made up for
+// B and the product of decays.  A thread takes one channel of one block of tokens, then four key channels x two value channels, which it walks from zero
+// as the token-by-token kernel walks them: products of matrices were 12 us faster for 2,048 tokens of 32 heads, but the tensor core cuts its sums off, and
+// a state that forgets fast came out 6.1e-8 off 64 bits instead of 3.9e-8 (multiply-adds of k times its later decays: 2.1e-7 instead of 1.9e-7 for a slow one).
 __global__ void __launch_bounds__(WC_THREADS, 3) wkv_chunk_sums_kernel(WkvChunkArgs a) {
-    __shared__ __align__(16) float kd[WC_L][WC_PITCH_COL], vs[WC_L][WC_PITCH_COL];
-    __shared__ float block_decay[WC_BLOCKS][WC_N];
+    __shared__ __align__(16) float ws[WC_L][WC_N], ks[WC_L][WC_N], vs[WC_L][WC_N];
     pdl_launch_dependents();
     const int tid = threadIdx.x, c = blockIdx.x, seq = blockIdx.y, head = blockIdx.z, i = tid % WC_N, b = tid / WC_N;
     const int row0 = a.seq_first_row[seq], t0 = row0 + c * WC_L, nt = min(WC_L, a.seq_first_row[seq + 1] - t0);
@@ -96,57 +100,64 @@ __global__ void __launch_bounds__(WC_THREADS, 3) wkv_chunk_sums_kernel(WkvChunkA
         k[x] = to_f32(a.k[at]);
         v[x] = to_f32(a.v[at]);
     }
-    float all = 1.f, odd = 0.f;          // odd: NaN once a value is not finite
-#pragma unroll
-    for (int x = WC_B - 1; x >= 0; --x) {
-        const int t = b * WC_B + x;
-        vs[t][i] = t < nt ? v[x] : 0.f;
-        odd = fmaf(vs[t][i], 0.f, odd);
-        k[x] = t < nt ? k[x] * all : 0.f;                  // (with the decays of the block's later tokens)
-        all *= t < nt ? wc_decay(w[x], w0) : 1.f;
-    }
-    block_decay[b][i] = all;
-    __syncthreads();
-    float after = 1.f;
-#pragma unroll
-    for (int x = WC_BLOCKS - 1; x > 0; --x)
-        if (x > b) after *= block_decay[x][i];
+    double all = 1.;                    // (64 bits: the decays of a whole chunk in one number would be 64 roundings off otherwise)
 #pragma unroll
     for (int x = 0; x < WC_B; ++x) {
-        kd[b * WC_B + x][i] = k[x] * after;
-        odd = fmaf(k[x] * after, 0.f, odd);
+        const int t = b * WC_B + x;
+        if (t >= nt) continue;
+        const float d = wc_decay(w[x], w0);
+        ws[t][i] = d;
+        ks[t][i] = k[x];
+        vs[t][i] = v[x];
+        all *= d;
+    }
+    __syncthreads();
+    const int lane = tid & 31, warp = tid >> 5;
+    float2 sum[4] = {};
+    const int last = max(0, nt - WC_CAREFUL);
+#pragma unroll 4
+    for (int t = 0; t < last; ++t) {
+        const float4 d = *reinterpret_cast<const float4*>(&ws[t][4 * warp]), x = *reinterpret_cast<const float4*>(&ks[t][4 * warp]);
+        const float2 y = *reinterpret_cast<const float2*>(&vs[t][2 * lane]);
+        sum[0] = __ffma2_rn(make_float2(d.x, d.x), sum[0], __fmul2_rn(make_float2(x.x, x.x), y));
+        sum[1] = __ffma2_rn(make_float2(d.y, d.y), sum[1], __fmul2_rn(make_float2(x.y, x.y), y));
+        sum[2] = __ffma2_rn(make_float2(d.z, d.z), sum[2], __fmul2_rn(make_float2(x.z, x.z), y));
+        sum[3] = __ffma2_rn(make_float2(d.w, d.w), sum[3], __fmul2_rn(make_float2(x.w, x.w), y));
+    }
+    // the newest tokens with what each rounding leaves (k v is exact), so that the rounding of B itself and the one behind it are no more than a
+    // walk's (5 us of 2,048 tokens of 32 heads; without it states of 100 to 128 tokens were 4 to 5 % further off than the walk's)
+    float2 rest[4] = {};
+#pragma unroll 1
+    for (int t = last; t < nt; ++t) {
+        const float2 y = *reinterpret_cast<const float2*>(&vs[t][2 * lane]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float d1 = ws[t][4 * warp + e], x1 = ks[t][4 * warp + e];
+            const float2 d = make_float2(d1, d1), add = __fmul2_rn(make_float2(x1, x1), y), p = __fmul2_rn(d, sum[e]);
+            const float2 left = __ffma2_rn(d, sum[e], make_float2(-p.x, -p.y)), s = __fadd2_rn(p, add), b2 = __fadd2_rn(s, make_float2(-p.x, -p.y));
+            const float2 a2 = __fadd2_rn(s, make_float2(-b2.x, -b2.y));
+            const float2 off = __fadd2_rn(__fadd2_rn(p, make_float2(-a2.x, -a2.y)), __fadd2_rn(add, make_float2(-b2.x, -b2.y)));
+            rest[e] = __ffma2_rn(d, rest[e], __fadd2_rn(left, off));
+            sum[e] = s;
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 s = __fadd2_rn(sum[e], rest[e]);
+        sum[e] = make_float2(fabsf(sum[e].x) < INFINITY ? s.x : sum[e].x, fabsf(sum[e].y) < INFINITY ? s.y : sum[e].y);       // (an infinity leaves NaN)
     }
     float* unit = wc_unit(a, seq, row0, c, head);
-    if (b == 0) unit[WC_N * WC_N + i] = after * all;
-    const bool plain = __syncthreads_and(odd == 0.f);
-    const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, i0 = 16 * (warp & 3), j0 = 16 * (warp >> 2);
-    float sum[2][4] = {}, acc[2][4] = {}, low[2][4] = {};
-    if (!plain) {
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+    for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(unit + (4 * warp + e) * WC_N + 2 * lane) = sum[e];
+    __syncthreads();
+    double (*of_block)[WC_N] = reinterpret_cast<double (*)[WC_N]>(&ws[0][0]);
+    of_block[b][i] = all;
+    __syncthreads();
+    if (b == 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll 1
-                for (int s = 0; s < nt; ++s) sum[n][e] = fmaf(kd[s][i0 + g + 8 * (e >> 1)], vs[s][j0 + 8 * n + 2 * t + (e & 1)], sum[n][e]);
-    } else
-#pragma unroll
-    for (int s = 0; s < WC_L; s += 8) {
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wc_split(kd[s + t + 4 * (e >> 1)][i0 + g + 8 * (e & 1)], hi[e], lo[e]);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const uint32_t bv[2] = {__float_as_uint(vs[s + t][j0 + 8 * n + g]), __float_as_uint(vs[s + t + 4][j0 + 8 * n + g])};
-            wc_mma(acc[n], hi, bv);
-            wc_mma(low[n], lo, bv);
-        }
-        if (s % 16 == 8) wc_add(sum, acc, low);
+        for (int x = 1; x < WC_BLOCKS; ++x) all *= of_block[x][i];
+        unit[WC_N * WC_N + i] = (float)all;
     }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-            *reinterpret_cast<float2*>(unit + (i0 + g + 8 * e) * WC_N + j0 + 8 * n + 2 * t) = make_float2(sum[n][2 * e], sum[n][2 * e + 1]);
 }
 
 // The states that the chunks start from, in the place of their sums; the sequence's state goes on to its last token.  A thread takes four values.
@@ -190,6 +201,31 @@ __global__ void __launch_bounds__(WC_STATE_THREADS) wkv_chunk_states_kernel(WkvC
     }
 }
 
+// Sums of products stay in the tensor core for 16 terms and are added up with rounding from there on (it cuts its sums off); the products of
+// the largest parts have an accumulator of their own.
+template <int NT>
+__device__ __forceinline__ void wc_add(float (&sum)[NT][4], float (&acc)[NT][4], float (&low)[NT][4]) {
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            sum[n][e] = (sum[n][e] + low[n][e]) + acc[n][e];
+            acc[n][e] = low[n][e] = 0.f;
+        }
+}
+
+// a x b from both operands' three parts, the smallest products first
+__device__ __forceinline__ void wc_products(float (&acc)[4], float (&low)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[2], const uint32_t (&b1)[2], const uint32_t (&b2)[2]) {
+    wc_mma(acc, a[0], b0);
+    wc_mma(low, a[1], b2);
+    wc_mma(low, a[2], b1);
+    wc_mma(low, a[0], b2);
+    wc_mma(low, a[1], b1);
+    wc_mma(low, a[2], b0);
+    wc_mma(low, a[0], b1);
+    wc_mma(low, a[1], b0);
+}
+
 struct WkvChunkShared {
     union {
         struct {
@@ -199,7 +235,10 @@ struct WkvChunkShared {
         } in;
         struct {
             float v[WC_L][WC_PITCH_COL];
-            uint32_t s[2][WC_N][WC_PITCH_COL];     // the state's two TF32 numbers
+            union {
+                uint32_t s[3][WC_N / 2][WC_PITCH_PAIR];        // the state's three bfloat16 numbers, two key channels together
+                float whole[WC_N][WC_PITCH_PAIR];              // (as it is, where something is not finite)
+            };
         } of;
     };
     float rd[WC_L][WC_PITCH_ROW];                  // r times the decays of its block's earlier tokens
@@ -244,8 +283,9 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
         if (vrow < nt) vals = *reinterpret_cast<const uint4*>(a.v + base + (int64_t)vrow * ld + vcol);
         const float* unit = wc_unit(a, seq, row0, c, head);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) st[x] = *reinterpret_cast<const float4*>(unit + 4 * (tid + x * WC_THREADS));
+        for (int x = 0; x < 2; ++x) st[x] = *reinterpret_cast<const float4*>(unit + (tid / 16 * 2 + x) * WC_N + tid % 16 * 4);
         float all = 1.f;
+        double block = 1.;
 #pragma unroll
         for (int x = 0; x < WC_B; ++x) {
             const int t = b * WC_B + x;
@@ -257,8 +297,9 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
             sh.in.k[t][i] = __float2bfloat16_rn(k[x]);
             sh.rd[t][i] = r[x] * all;
             all *= w[x];
+            block *= w[x];
         }
-        sh.block_decay[b][i] = all;
+        sh.block_decay[b][i] = (float)block;
         float later = 1.f;
 #pragma unroll
         for (int x = WC_B - 1; x >= 0; --x) {
@@ -329,23 +370,32 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
             }
         } else
 #pragma unroll
-        for (int i = 0; i < WC_N; i += 8) {
-            float f[2][2];                                      // [place][half of the targets]: the blocks between
+        for (int i = 0; i < WC_N; i += 16) {
+            uint32_t a3[3][4], b3[3][2];
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                f[p][0] = 1.f;
-                for (int b = sb + 1; b < 2 * m; ++b) f[p][0] *= sh.block_decay[b][i + t + 4 * p];
-                f[p][1] = sb < 2 * m ? f[p][0] * sh.block_decay[2 * m][i + t + 4 * p] : 1.f;
+            for (int p = 0; p < 2; ++p) {                       // [place][half of the targets]: times the blocks between
+                const int at = i + 2 * t + 8 * p;
+                float2 f = make_float2(1.f, 1.f);
+                for (int b = sb + 1; b < 2 * m; ++b) {
+                    const float2 d = *reinterpret_cast<const float2*>(&sh.block_decay[b][at]);
+                    f.x *= d.x;
+                    f.y *= d.y;
+                }
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const float2 r = *reinterpret_cast<const float2*>(&sh.rd[16 * m + g + 8 * half][at]);
+                    wc_split(r.x * f.x, r.y * f.y, a3[0][2 * p + half], a3[1][2 * p + half], a3[2][2 * p + half]);
+                    if (half == 0 && sb < 2 * m) {
+                        const float2 d = *reinterpret_cast<const float2*>(&sh.block_decay[2 * m][at]);
+                        f.x *= d.x;
+                        f.y *= d.y;
+                    }
+                }
+                const float2 k = *reinterpret_cast<const float2*>(&sh.in.kd[sb * WC_B + g][at]);
+                wc_split(k.x, k.y, b3[0][p], b3[1][p], b3[2][p]);
             }
-            uint32_t hi[4], lo[4], bh[2], bl[2];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) wc_split(sh.rd[16 * m + g + 8 * (e & 1)][i + t + 4 * (e >> 1)] * f[e >> 1][e & 1], hi[e], lo[e]);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) wc_split(sh.in.kd[sb * WC_B + g][i + t + 4 * e], bh[e], bl[e]);
-            wc_mma(acc[0], hi, bh);
-            wc_mma(low[0], hi, bl);
-            wc_mma(low[0], lo, bh);
-            if (i % 16 == 8) wc_add(sum, acc, low);
+            wc_products(acc[0], low[0], a3, b3[0], b3[1], b3[2]);
+            wc_add(sum, acc, low);
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -360,52 +410,76 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
     plain = __syncthreads_and(odd == 0.f);
 #pragma unroll
     for (int e = 0; e < 8; e += 2) *reinterpret_cast<float2*>(&sh.of.v[vrow][vcol + e]) = make_float2(value[e], value[e + 1]);
+    const int q = tid / 16, qcol = tid % 16 * 4;           // its key channels 2 q and 2 q + 1
+    if (plain) {
+        uint32_t p[3][4];
 #pragma unroll
-    for (int x = 0; x < 2; ++x) {
-        const int at = tid + x * WC_THREADS;
-        uint32_t hi[4], lo[4];
+        for (int e = 0; e < 4; ++e) wc_split(from[e], from[4 + e], p[0][e], p[1][e], p[2][e]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            wc_split(from[4 * x + e], hi[e], lo[e]);
-            if (!plain) hi[e] = __float_as_uint(from[4 * x + e]);
-        }
-        *reinterpret_cast<uint4*>(&sh.of.s[0][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(&sh.of.s[1][at / (WC_N / 4)][at % (WC_N / 4) * 4]) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        for (int o = 0; o < 3; ++o) *reinterpret_cast<uint4*>(&sh.of.s[o][q][qcol]) = make_uint4(p[o][0], p[o][1], p[o][2], p[o][3]);
+    } else {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) *reinterpret_cast<float4*>(&sh.of.whole[2 * q + x][qcol]) = st[x];
     }
     __syncthreads();
     const int m = warp & 3, j0 = 16 * (warp >> 2);
     float sum[2][4] = {}, acc[2][4] = {}, low[2][4] = {};
-    if (plain)
-#pragma unroll
-    for (int i = 0; i < WC_N; i += 8) {
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wc_split(sh.rd[16 * m + g + 8 * (e & 1)][i + t + 4 * (e >> 1)] * sh.before[2 * m + (e & 1)][i + t + 4 * (e >> 1)], hi[e], lo[e]);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const uint32_t bh[2] = {sh.of.s[0][i + t][j0 + 8 * n + g], sh.of.s[0][i + t + 4][j0 + 8 * n + g]};
-            const uint32_t bl[2] = {sh.of.s[1][i + t][j0 + 8 * n + g], sh.of.s[1][i + t + 4][j0 + 8 * n + g]};
-            wc_mma(acc[n], hi, bh);
-            wc_mma(low[n], hi, bl);
-            wc_mma(low[n], lo, bh);
-        }
-        if (i % 16 == 8) wc_add(sum, acc, low);
-    }
     if (plain) {
-        for (int s0 = 0; s0 <= m * 16; s0 += 16) {
 #pragma unroll
-            for (int s = s0; s < s0 + 16; s += 8) {
-                uint32_t hi[4], lo[4];
+        for (int i = 0; i < WC_N; i += 16) {
+            uint32_t a3[3][4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) wc_split(sh.A[16 * m + g + 8 * (e & 1)][s + t + 4 * (e >> 1)], hi[e], lo[e]);
+            for (int e = 0; e < 4; ++e) {
+                const int at = i + 2 * t + 8 * (e >> 1);
+                const float2 r = *reinterpret_cast<const float2*>(&sh.rd[16 * m + g + 8 * (e & 1)][at]), d = *reinterpret_cast<const float2*>(&sh.before[2 * m + (e & 1)][at]);
+                wc_split(r.x * d.x, r.y * d.y, a3[0][e], a3[1][e], a3[2][e]);
+            }
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    const uint32_t bv[2] = {__float_as_uint(sh.of.v[s + t][j0 + 8 * n + g]), __float_as_uint(sh.of.v[s + t + 4][j0 + 8 * n + g])};
-                    wc_mma(acc[n], hi, bv);
-                    wc_mma(low[n], lo, bv);
-                }
+            for (int n = 0; n < 2; ++n) {
+                uint32_t b3[3][2];
+#pragma unroll
+                for (int p = 0; p < 3; ++p)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) b3[p][e] = sh.of.s[p][i / 2 + t + 4 * e][j0 + 8 * n + g];
+                wc_products(acc[n], low[n], a3, b3[0], b3[1], b3[2]);
             }
             wc_add(sum, acc, low);
+        }
+        for (int s = 0; s < m * 16; s += 16) {
+            uint32_t a3[3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 x = *reinterpret_cast<const float2*>(&sh.A[16 * m + g + 8 * (e & 1)][s + 2 * t + 8 * (e >> 1)]);
+                wc_split(x.x, x.y, a3[0][e], a3[1][e], a3[2][e]);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const int j = j0 + 8 * n + g;
+                const uint32_t bv[2] = {wc_pair(sh.of.v[s + 2 * t][j], sh.of.v[s + 2 * t + 1][j]), wc_pair(sh.of.v[s + 2 * t + 8][j], sh.of.v[s + 2 * t + 9][j])};
+                wc_mma(acc[n], a3[0], bv);
+                wc_mma(low[n], a3[2], bv);
+                wc_mma(low[n], a3[1], bv);
+            }
+            wc_add(sum, acc, low);
+        }
+        // the target's own tile of 16 tokens by multiply-adds: the newest tokens are most of an output where decays are fast
+#pragma unroll
+        for (int s = 16 * m; s < 16 * m + 16; s += 4) {
+            float a4[2][4];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) *reinterpret_cast<float4*>(a4[e]) = *reinterpret_cast<const float4*>(&sh.A[16 * m + g + 8 * e][s]);
+#pragma unroll
+            for (int x = 0; x < 4; ++x)
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    const float2 y = *reinterpret_cast<const float2*>(&sh.of.v[s + x][j0 + 8 * n + 2 * t]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float2 o = __ffma2_rn(make_float2(a4[e][x], a4[e][x]), y, make_float2(sum[n][2 * e], sum[n][2 * e + 1]));
+                        sum[n][2 * e] = o.x;
+                        sum[n][2 * e + 1] = o.y;
+                    }
+                }
         }
     } else {                // (nor may a value that is not finite meet the zeros of the tokens before it)
 #pragma unroll
@@ -415,7 +489,7 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
                 const int target = 16 * m + g + 8 * (e >> 1), j = j0 + 8 * n + 2 * t + (e & 1);
 #pragma unroll 1
                 for (int i = 0; i < WC_N; ++i)
-                    sum[n][e] = fmaf(sh.rd[target][i] * sh.before[2 * m + (e >> 1)][i], __uint_as_float(sh.of.s[0][i][j]), sum[n][e]);
+                    sum[n][e] = fmaf(sh.rd[target][i] * sh.before[2 * m + (e >> 1)][i], sh.of.whole[i][j], sum[n][e]);
 #pragma unroll 1
                 for (int s = 0; s <= target; ++s) sum[n][e] = fmaf(sh.A[target][s], sh.of.v[s][j], sum[n][e]);
             }

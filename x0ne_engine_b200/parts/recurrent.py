@@ -17,14 +17,14 @@ MIXES = ("r", "k", "v", "g", "w")
 def by_chunks(ctx, dtype, heads: int, head_dim: int, n_rows: int, state) -> bool:
     """Whether a pass's scan goes by chunks that are worked out at once: where that is ahead of the walk token by token, in us.  The walk takes
     0.072 a token of the longest sequence where every block of it has a multiprocessor (0.125 where not), and at least 0.0019 a token and head
-    over the whole pass; the chunks 12 + 0.0011 a token and head (a sequence's last chunk is half empty on average), at least 26.  Measured,
-    walk / chunks: 32 heads, one sequence of 256 / 512 / 2,048 tokens 21 / 27, 39 / 28, 149 / 85, 16 of 64 tokens 69 / 47; 16 heads 16 of 100 53 / 46;
-    64 heads one of 128 / 256 21 / 27, 35 / 28.  32-bit runs walk, so that a token's bits do not depend on where its pass began."""
+    over the whole pass; the chunks 12 + 0.0014 a token and head (and a quarter of a chunk more per sequence, whose last one is not full), at least 28.  Measured,
+    walk / chunks: 32 heads, one sequence of 256 / 512 / 2,048 tokens 23 / 29, 41 / 33, 146 / 107, 16 of 64 / 128 tokens 71 / 63, 124 / 103, 4 of 300 80 / 72; 16 heads 16 of
+    100 55 / 56, one of 2,048 146 / 68; 64 heads one of 128 / 256 / 512 23 / 29, 37 / 34, 68 / 61.  32-bit runs walk, so that a token's bits do not depend on where its pass began."""
     if dtype != torch.bfloat16 or head_dim != 64 or ctx.decode or state.stride(0) % 4 != 0 or ctx.n_seqs * ops.WKV_CHUNK > n_rows:
         return False
     per_token = 0.072 if 4 * heads * ctx.n_seqs <= ctx.sm_count else 0.125
     walk = 3 + max(per_token * ctx.max_seq_rows, 0.0019 * heads * n_rows)
-    return max(26, 12 + 0.0011 * heads * (n_rows + ops.WKV_CHUNK // 2 * ctx.n_seqs)) < 0.95 * walk
+    return max(28, 12 + 0.0014 * heads * (n_rows + ops.WKV_CHUNK // 4 * ctx.n_seqs)) < 0.95 * walk
 
 
 class MatrixStateRecurrence(Mixer):
