@@ -82,3 +82,18 @@ def test_kernels_let_their_successors_start_only_with_their_tensor_memory_in_han
 def test_rules_ask_the_device_for_its_multiprocessors(path):
     with open(path) as f:
         assert not re.search(r"\b148\b", re.sub(r"//[^\n]*", "", f.read()))
+
+
+def defined(source, name):
+    """The whole number that a source defines `name` as, through other names of the same source."""
+    with open(os.path.join(CSRC, source)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    value = re.search(rf"#define\s+{name}\s+(.+)", text).group(1)
+    return eval(re.sub(r"[A-Z][A-Z0-9_]*", lambda m: str(defined(source, m.group(0))), value))
+
+
+def test_sizes_that_python_repeats_are_the_kernels():
+    from x0ne_engine_b200.csrc import ops
+    assert ops.F32_SPLIT_K == defined("gemm_f32.cu", "F32_SPLIT_K")
+    assert (ops.WKV_CHUNK, ops.WKV_CHUNK_UNIT) == (defined("wkv_chunk.cu", "WC_L"), defined("wkv_chunk.cu", "WC_UNIT"))
+    assert ops.MOE_TC_TILE_ROWS == defined("moe_tcgen05.cu", "MT_BM")

@@ -510,7 +510,8 @@ def cmd_kernel_bench(a) -> int:
         chosen = torch.stack([torch.randperm(E, device=dev)[:top] for _ in range(rows)]).to(torch.int32).contiguous()
         i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=dev)      # noqa: E731
         tc = ops.moe_tc_takes(torch.bfloat16, pairs, hidden, ff) and (not a.gated or ff % ops.MOE_PAIR_BLOCK == 0)
-        tile = ops.MOE_TC_TILE_ROWS if tc else ops.MOE_TILE_ROWS
+        pair = tc and ops.moe_tc_in_pairs(pairs, E, (mats - 1) * ff, hidden, ff, torch.cuda.get_device_properties(dev).multi_processor_count)
+        tile = ops.MOE_TC_TILE_ROWS * (2 if pair else 1) if tc else ops.MOE_TILE_ROWS
         n_tiles = ops.moe_max_tiles(pairs, E, tile)
         offsets, listed, tiles, n_real = i32(E + 1), i32(pairs), i32(n_tiles, 3), i32(1)
         xs = torch.zeros(pairs, hidden, device=dev, dtype=torch.bfloat16)
@@ -523,8 +524,8 @@ def cmd_kernel_bench(a) -> int:
             ops.moe_group(chosen, pairs, E, offsets, listed, tiles, tile, n_real)
             if tc:
                 ops.moe_gather_rows(x, listed, offsets, E, top, xs, pairs)
-                ops.moe_product_tc(kind, xs, ups[i], listed, tiles, n_real, n_tiles, act)
-                ops.moe_product_tc(1, act, downs[i], listed, tiles, n_real, n_tiles, y)
+                ops.moe_product_tc(kind, xs, ups[i], listed, tiles, n_real, n_tiles, act, pair)
+                ops.moe_product_tc(1, act, downs[i], listed, tiles, n_real, n_tiles, y, pair)
             else:
                 ops.moe_product(kind, x, ups[i], listed, tiles, n_tiles, top, act, ops.MOE_PAIR_BLOCK if ff % ops.MOE_PAIR_BLOCK == 0 else 0)
                 ops.moe_product(1, act, downs[i], listed, tiles, n_tiles, top, y)

@@ -278,7 +278,10 @@ extern "C" int x0ne_gemm_f32_split(const float* A, const float* W, float* C, int
 
 // K from which the tensor cores take a product.  The rule may look at W alone, so that a row's bits do not depend on what is computed with
 // it.  8 / 64 rows on multiply-add units against tensor cores: K 512 7.0 / 24.6 us and 7.5 / 10.2 (N 4096), 6.4 / 17.2 and 6.3 / 6.8 (N 1024); K 1,024 10.8 /
-// 31.5 and 6.5 / 8.1 (N 1024); K 2,048 24.4 / 89 and 13.3 / 18.6 (N 4096).
+// 31.5 and 6.5 / 8.1 (N 1024); K 2,048 24.4 / 89 and 13.3 / 18.6 (N 4096); K 256 6.9 / 13.6 and 9.2 / 8.9 (N 4096), 7.4 / 10.0 and 8.7 / 8.8 (N 1024).
+// Their error against 64 bits is the smaller one for dense rows (2-norm over 2-norm, multiply-adds and tensor cores: K 256 2.9e-7 and 7.3e-8, 512 4.1e-7
+// and 7.8e-8, 2,048 8.2e-7 and 9.2e-8, 6,144 1.4e-6 and 1.2e-7; all values positive 3.3e-7 and 5.9e-8 at 512, 1.2e-6 and 6.8e-8 at 6,144), and about the same where
+// a row has a handful of terms (one value in a hundred not zero: 4.7e-8 and 4.9e-8 at 512, 8.4e-8 and 6.0e-8 at 2,048).
 #define F32_SPLIT_K 512
 
 // `batch` products of one shape: product b reads A + b sa and W + b sw and writes C + b sc.  `status`: one int in device memory, zero before the

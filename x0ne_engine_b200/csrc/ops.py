@@ -942,7 +942,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, n_rows: int, bias: Optional
                                 _stream()), "swiglu")
 
 
-F32_SPLIT_K = 512        # K from which a float32 product runs on the tensor cores (gemm_f32.cu has the reason)
+F32_SPLIT_K = 512        # K from which a float32 product runs on the tensor cores (gemm_f32.cu has the reason, and the rule: a test compares the two)
 
 
 def _f32_status(k: int, device) -> int:
@@ -1493,7 +1493,7 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor,
                                   1 if one_token else 0, _stream()), "wkv_scan")
 
 
-WKV_CHUNK, WKV_CHUNK_UNIT = 64, 64 * 64 + 64        # tokens of a chunk, scratch floats of a chunk and head
+WKV_CHUNK, WKV_CHUNK_UNIT = 64, 64 * 64 + 64        # tokens of a chunk, scratch floats of a chunk and head (wkv_chunk.cu: WC_L, WC_UNIT)
 
 
 def wkv_chunk_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor, w0: torch.Tensor, u: torch.Tensor, h: torch.Tensor,

@@ -12,9 +12,10 @@
 //   head norm     out[row, head] = o / sqrt(mean(o^2) + eps) * weight * silu(gate)
 //
 // The state of a sequence is one float32 array: heads x N x N, then `width` values of the last h.  State, decays
-// and every sum are float32; r, k, v, the gate and h come in the activation type.  A sequence's result depends
-// on its own rows and state only, and every sum runs in one fixed order, so it is the same bits however the
-// sequence's tokens are cut into passes and whatever else is in a pass.
+// and every sum are float32; r, k, v, the gate and h come in the activation type.  What these kernels make of a
+// sequence depends on its own rows and state only, and every sum runs in one fixed order, so it is the same bits however the
+// sequence's tokens are cut into passes and whatever else is in a pass.  32-bit runs have that from end to end; of bfloat16 runs long passes go by
+// chunks (wkv_chunk.cu, whose sums have another order) where a rule on the whole pass says so (`by_chunks` in parts/recurrent.py).
 #include <type_traits>
 
 #include "common.cuh"

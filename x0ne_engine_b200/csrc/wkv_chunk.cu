@@ -503,9 +503,6 @@ __global__ void __launch_bounds__(WC_THREADS, 2) wkv_chunk_out_kernel(WkvChunkAr
         }
 }
 
-X0NE_API int x0ne_wkv_chunk_tokens() { return WC_L; }
-X0NE_API int x0ne_wkv_chunk_unit() { return WC_UNIT; }
-
 // bfloat16 runs of heads of 64; at most max_seq_rows rows per sequence; scratch: (n_rows / 64 + n_seqs) x heads x WC_UNIT floats.  The rest as for
 // x0ne_wkv_scan.
 X0NE_API int x0ne_wkv_chunk_scan(const void* r, const void* k, const void* v, const float* z, const float* w0, const float* u, const void* h, float* o, float* state,

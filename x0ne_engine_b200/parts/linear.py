@@ -1,7 +1,7 @@
 """Matrix products y = x W^T for weights stored [out, in] (row-major, as checkpoints hold them).
 
 float32: this library's own kernels, whose order of sums hangs on K alone (multiply-adds, or from
-512 values of K on the tensor cores with split operands), so a row's result does not depend on the
+512 values of K on the tensor cores with every operand as three bfloat16 values that hold all of it), so a row's result does not depend on the
 batch it is in.  bfloat16: float32 accumulation with a bfloat16 or float32 result; the
 library engine delegates these products to cuBLAS (x0ne-core/runtime/src/gpu.rs:1098-1149), and
 `Linear` does the same through torch.mm unless one of this library's own kernels takes the shape.

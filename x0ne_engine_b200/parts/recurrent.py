@@ -38,7 +38,8 @@ class MatrixStateRecurrence(Mixer):
 
     What a sequence keeps is one float32 row: the heads' matrices, then the last input row (for the next token's shift).
     The decay, the state and the scan are float32 whatever the run's dtype; the projections run in the run's dtype.
-    A sequence's result depends on its own rows and state only.
+    A sequence's result depends on its own rows and state only; in a bfloat16 run the order of the scan's sums, and so the last bits, also on
+    what else is in the pass and how its tokens are cut into passes (`by_chunks`, and the routing of the projections).
 
     Parameters: hidden_size, heads, head_dim, decay_rank, eps, names.{mu (pattern with {s}), r, k, v, g, w1, w2, w0, u,
     norm, o}.
