@@ -1233,8 +1233,12 @@ def check_watched_tc_status(device) -> None:
 def clear_tc_status(device) -> None:
     """After a report: the word is zero again, here and where a copy of it has gone."""
     gemm_tc_status(device).zero_()
-    word, event = _tc_watched.get(device.index if device.index is not None else torch.cuda.current_device(), (None, None))
-    if word is not None:
+    forget_watched_tc_status()
+
+
+def forget_watched_tc_status() -> None:
+    """What has been copied from status words that are zero again is not reported a second time."""
+    for word, event in _tc_watched.values():
         event.synchronize()
         word.zero_()
 

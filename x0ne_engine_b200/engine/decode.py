@@ -215,7 +215,8 @@ class DeviceBatch:
         self._out_event[k % 2].synchronize()
         got = self._out_host[k % 2][:n + 1].tolist()
         if got[n] != 0:
-            ops.clear_tc_status(self.engine.device)
+            self.status.zero_()
+            ops.forget_watched_tc_status()
             what = "the prompts' step" if k == self._batch_first else f"decode step {k - self._batch_first}"
             raise ops.KernelError(f"{what} of this batch: {ops.describe_tc_status(got[n])}")
         return got[:n]
