@@ -174,39 +174,46 @@ class SequenceCache:
                 elif src in self.states:
                     self.states[e] = self.states[src]
         self._reads = list(reads_cache_of)
+        dev = torch.device(device)
+        self._index = None if dev.type != "cuda" else dev.index if dev.index is not None else torch.cuda.current_device()
         self._pushed: Dict[int, Optional[torch.cuda.Event]] = {}         # by stream: behind the last rows and states that went out on it
+        self._events: Dict[int, torch.cuda.Event] = {}                   # (kept: a new event for every sequence cost the host 8 us each)
 
     # ---- streams
-    def _stream(self) -> int:
-        device = torch.device(self.device)
-        return torch._C._cuda_getCurrentRawStream(device.index if device.index is not None else torch.cuda.current_device())
-
     def _note_push(self) -> None:
         """Rows or states are on their way to the device on the current stream."""
-        if torch.device(self.device).type != "cuda":
+        if self._index is None:
             return
-        stream = self._stream()
+        stream = torch._C._cuda_getCurrentRawStream(self._index)
         if stream == 0:
-            self._pushed[0] = None          # (the default stream is always there to be asked later: no event for every sequence)
+            self._pushed[0] = None          # (the default stream is always there to be asked later)
+            return
+        ev = self._events.get(stream)
+        if ev is None:
+            ev = self._events[stream] = torch.cuda.Event()
+        if torch.cuda.current_device() == self._index:
+            ev.record()
         else:
-            ev = self._pushed[stream] = torch.cuda.Event()
-            ev.record(torch.cuda.current_stream(self.device))
+            ev.record(torch.cuda.current_stream(self._index))
+        self._pushed[stream] = ev
 
     def settle(self) -> None:
         """Puts what `acquire` and `ensure` sent on other streams ahead of what the current stream launches next."""
         if not self._pushed:
             return
-        here = self._stream()
+        here = torch._C._cuda_getCurrentRawStream(self._index)
+        if len(self._pushed) == 1 and here in self._pushed:
+            return
         for stream, ev in list(self._pushed.items()):
             if stream == here:
                 continue
             if ev is None:
                 ev = self._pushed[stream] = torch.cuda.Event()
-                ev.record(torch.cuda.default_stream(self.device))
+                ev.record(torch.cuda.default_stream(self._index))
             if ev.query():
                 self._pushed.pop(stream, None)
             else:
-                torch.cuda.current_stream(self.device).wait_event(ev)
+                torch.cuda.current_stream(self._index).wait_event(ev)
 
     # ---- what parts see
     def kv_view(self, entry: int) -> PagedCacheArg:
