@@ -94,3 +94,20 @@ def test_the_word_for_waits_is_there_before_a_capture():
         assert int(word) == 1 << 20 and torch.allclose(y, x @ w.T, rtol=1e-4, atol=1e-3)          # (a replay leaves a report as it is)
     finally:
         ops._tc_status = kept
+
+
+def test_a_sequence_is_not_taken_inside_a_capture():
+    """A captured copy of the page table's row would be made from whatever the row holds when the graph is replayed."""
+    from x0ne_engine_b200.csrc import ops
+    eng = engine("bfloat16")
+    ids = prompts_for(eng.vocab_size, [20], seed=4)[0]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin()
+        with pytest.raises(ops.KernelError, match="captured"):
+            eng.new_sequence(64)
+        graph.capture_end()
+    torch.cuda.synchronize()
+    slot = eng.new_sequence(64)
+    assert bool(torch.isfinite(eng.step([slot], [ids])).all())

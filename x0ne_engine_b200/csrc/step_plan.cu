@@ -92,9 +92,13 @@ X0NE_API int x0ne_plan_pass(int n_seqs, const int32_t* slots, const int32_t* sta
 }
 
 // Host memory into device memory on the stream.  Ordinary host memory is taken over before the call returns; nothing waits for the stream.
+// Not inside a capture, whose replays would read the host memory again, whatever it holds by then.
 X0NE_API int x0ne_copy_in(void* dst, const void* src, int64_t bytes, cudaStream_t stream) {
     X0NE_REQUIRE(dst != nullptr && src != nullptr && bytes > 0, "copy_in: %lld bytes", (long long)bytes);
-    const cudaError_t e = cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyHostToDevice, stream);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(stream, &capture);
+    X0NE_REQUIRE(e == cudaSuccess && capture == cudaStreamCaptureStatusNone, "copy_in: the stream is being captured");
+    e = cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyHostToDevice, stream);
     X0NE_REQUIRE(e == cudaSuccess, "copy_in: %s", cudaGetErrorString(e));
     return 0;
 }
