@@ -26,7 +26,7 @@
 #define SP_TILE_W 128           // rows of W per block: the tensor memory's lanes
 
 template <int NX> struct SpConfig {
-    static constexpr int A_BYTES = SP_TILE_W * 128, X_BYTES = NX * 128;
+    static constexpr int A_BYTES = SP_TILE_W * 128, X_BYTES = NX * 128;      // of a slab, as it comes
     static constexpr int RAW = 4;                                    // stages of operands as they come
     static constexpr int ACC = NX == 96 ? 1 : NX == 16 ? 4 : 2;       // accumulators of a slab's large products
     static constexpr int SPLIT = NX == 64 ? 4 : NX == 16 ? 3 : 2;    // stages of split operands (W: tensor memory, x: shared memory)
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(SpConfig<NX>::THREADS, SpConfig<NX>::BLOCKS) g
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sp_dyn) + 1023) & ~(uintptr_t)1023);
     unsigned char* raw_w = base;                                        // [stage][128 rows][128 bytes], 128-byte swizzle
     unsigned char* raw_x = raw_w + RAW * Cfg::A_BYTES;                  // [stage][NX rows][128 bytes]
-    unsigned char* split_x = raw_x + RAW * Cfg::X_BYTES;                // [stage][hi, mid, lo][NX rows][128 bytes]
+    unsigned char* split_x = raw_x + RAW * Cfg::X_BYTES;                // [stage][a, b, c][NX rows][64 bytes], 64-byte swizzle
     SpShared* sh = reinterpret_cast<SpShared*>(base + Cfg::TILES);
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = CL > 1 ? (int)(blockIdx.x % CL) : 0, tile = blockIdx.x / CL;
